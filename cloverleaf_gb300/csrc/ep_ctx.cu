@@ -70,7 +70,7 @@ struct ep_ctx {
     // second branch: a batch's fix-ups beside the next batch's sampling
     cudaStream_t fix = nullptr;
     cudaStream_t fix2 = nullptr;   // the long spans' fix-ups, beside the short ones on `fix`
-    cudaEvent_t ev_red = nullptr, ev_fix = nullptr, ev_fix2 = nullptr;
+    cudaEvent_t ev_red = nullptr, ev_fix = nullptr, ev_fix2 = nullptr, ev_direct = nullptr;
     bool fix_pending = false;   // the last issued fix-ups have not been joined yet
     std::string err;
 
@@ -114,6 +114,8 @@ struct ep_ctx {
     // their slots sooner when anchors differ in work (2: forward 0.164 ->
     // 0.150 ms per batch on the 10M-node graph)
     uint32_t gather_warps = 2;
+    // warps per anchor of the staged gather (1, 2, 4); 0 = by batch size
+    uint32_t gather_split = 0;
     // warps per CTA of the sampler (1-8)
     uint32_t sample_warps = 8;
     bool tuned = false;         // autotuner has chosen chunk / fused_mode
@@ -149,6 +151,7 @@ struct ep_ctx {
         if (ev_red) cudaEventDestroy(ev_red);
         if (ev_fix) cudaEventDestroy(ev_fix);
         if (ev_fix2) cudaEventDestroy(ev_fix2);
+        if (ev_direct) cudaEventDestroy(ev_direct);
         if (fix) cudaStreamDestroy(fix);
         if (fix2) cudaStreamDestroy(fix2);
         if (side) cudaStreamDestroy(side);
@@ -255,6 +258,7 @@ extern "C" int ep_create(const ep_config* cfg, ep_ctx** out) {
         cudaEventCreateWithFlags(&c->ev_red, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_fix, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_fix2, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&c->ev_direct, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_loss, cudaEventDisableTiming) != cudaSuccess ||
@@ -285,9 +289,10 @@ extern "C" int ep_create(const ep_config* cfg, ep_ctx** out) {
     if (const char* e = getenv("EP_QUEUE_CTAS")) { const long v = atol(e); if (v == 4 || v == 5) c->queue_ctas = (uint32_t)v; }
     if (const char* e = getenv("EP_RED_CTAS")) { const long v = atol(e); if (v >= 0 && v <= 65536) c->red_ctas = (uint32_t)v; }
     if (const char* e = getenv("EP_GATHER_WARPS")) { const long v = atol(e); if (v >= 1 && v <= 8) c->gather_warps = (uint32_t)v; }
+    if (const char* e = getenv("EP_GATHER_SPLIT")) { const long v = atol(e); if (v == 1 || v == 2 || v == 4) c->gather_split = (uint32_t)v; }
     if (const char* e = getenv("EP_SAMPLE_WARPS")) { const long v = atol(e); if (v >= 1 && v <= 8) c->sample_warps = (uint32_t)v; }
     // a launch shape set by hand is used as given: no tuning
-    for (const char* k : {"EP_FUSED_MODE", "EP_REDUCE_CHUNK", "EP_GATHER_CTAS", "EP_QUEUE_CTAS", "EP_RED_CTAS", "EP_GATHER_WARPS", "EP_RING_PW",
+    for (const char* k : {"EP_FUSED_MODE", "EP_REDUCE_CHUNK", "EP_GATHER_CTAS", "EP_GATHER_SPLIT", "EP_QUEUE_CTAS", "EP_RED_CTAS", "EP_GATHER_WARPS", "EP_RING_PW",
                           "EP_RING_CW", "EP_RING_SLOTS"})
         if (getenv(k)) c->cfg.autotune = 0;
     if (const char* ch = getenv("EP_REDUCE_CHUNK")) {   // reducer items per warp (tuning)
@@ -697,6 +702,7 @@ static SampleParams sample_params(ep_ctx* c, BatchState* st, bool eval, int inje
     sp.nbr_cnt = c->nbr_cnt.as<uint32_t>();
     sp.neg = c->neg.as<uint32_t>();
     sp.occ = c->occ.as<uint32_t>();
+    sp.deferred = c->deferred.as<uint8_t>();
     return sp;
 }
 
@@ -737,6 +743,7 @@ static ForwardParams forward_params(ep_ctx* c, BatchState* st, const void* table
     fp.item_c = c->item_c.as<float>();
     fp.deferred = c->deferred.as<uint8_t>();
     fp.gather_ctas = c->gather_ctas;
+    fp.gather_split = c->gather_split;
     fp.gather_warps = c->gather_warps;
     return fp;
 }
@@ -774,6 +781,11 @@ static ReduceParams reduce_params(ep_ctx* c, BatchState* st, int out_mode, void*
     rp.queue_ctas_per_sm = c->queue_ctas;
     rp.red_ctas = c->red_ctas;
     return rp;
+}
+
+// The forward kernels in order on one stream.
+static void issue_forward(int tt, int vpl, const ForwardParams& fp, uint32_t cap, cudaStream_t s) {
+    for (int part : {FWD_GATHER, FWD_DIRECT, FWD_LOSS}) launch_forward(tt, vpl, fp, cap, s, part);
 }
 
 // Sort the emitted items and reduce them; tt selects the kernel family.
@@ -837,17 +849,25 @@ static void issue_train_batch(ep_ctx* c, cudaEvent_t* ev = nullptr, bool fork = 
             cudaStreamWaitEvent(s, c->ev_fix2, 0);
             cudaStreamWaitEvent(c->side, c->ev_fix, 0);
             cudaStreamWaitEvent(c->side, c->ev_fix2, 0);
+            cudaStreamWaitEvent(c->fix2, c->ev_fix, 0);
             c->fix_pending = false;
         }
         ForwardParams fe = forward_params(c, st, c->table.p, true, false);
-        launch_forward(c->tt, (int)c->vpl, fe, c->Bcap, c->side, FWD_EMIT);
+        launch_emit(fe, c->Bcap, c->side);
         launch_radix_sort(st, c->item_f.as<uint32_t>(), c->key_alt.as<uint32_t>(), c->item_src.as<uint32_t>(),
                           c->item_c.as<float>(), c->idx.as<uint2>(), c->idx_alt.as<uint2>(), c->hist.as<uint32_t>(),
                           c->items_cap, (int)bits_for(c->n_feat), &c->sorted_keys, &c->sorted_vals, c->side);
         cudaEventRecord(c->ev_sorted, c->side);
         ForwardParams fp = forward_params(c, st, c->table.p, false, false);
         fp.means_dead = 1;
-        launch_forward(c->tt, (int)c->vpl, fp, c->Bcap, s);
+        // the direct gathers beside the staged ones, on the long fix-ups'
+        // stream (behind the previous batch's fix-ups: they update the table)
+        cudaStreamWaitEvent(c->fix2, c->ev_fork, 0);
+        launch_forward(c->tt, (int)c->vpl, fp, c->Bcap, c->fix2, FWD_DIRECT);
+        cudaEventRecord(c->ev_direct, c->fix2);
+        launch_forward(c->tt, (int)c->vpl, fp, c->Bcap, s, FWD_GATHER);
+        cudaStreamWaitEvent(s, c->ev_direct, 0);
+        launch_forward(c->tt, (int)c->vpl, fp, c->Bcap, s, FWD_LOSS);
         cudaEventRecord(c->ev_loss, s);
         cudaStreamWaitEvent(c->side, c->ev_loss, 0);
         launch_batch_end(st, c->loss.p, c->status.as<int32_t>(), c->nbr_cnt.as<uint32_t>(), c->Bcap, c->steps_per_pass,
@@ -857,7 +877,7 @@ static void issue_train_batch(ep_ctx* c, cudaEvent_t* ev = nullptr, bool fork = 
     } else {
         ForwardParams fp = forward_params(c, st, c->table.p, true, false);
         fp.means_dead = 1;
-        launch_forward(c->tt, (int)c->vpl, fp, c->Bcap, s);
+        issue_forward(c->tt, (int)c->vpl, fp, c->Bcap, s);
         if (ev) cudaEventRecord(ev[EP_STAGE_FORWARD], s);
         launch_radix_sort(st, c->item_f.as<uint32_t>(), c->key_alt.as<uint32_t>(), c->item_src.as<uint32_t>(),
                           c->item_c.as<float>(), c->idx.as<uint2>(), c->idx_alt.as<uint2>(), c->hist.as<uint32_t>(),
@@ -1175,7 +1195,7 @@ static int run_validation(ep_ctx* c, double* mean_out) {
         SampleParams sp = sample_params(c, st, true, false);
         launch_sample(sp, c->stream);
         ForwardParams fp = forward_params(c, st, c->table.p, false, true);
-        launch_forward(c->tt, (int)c->vpl, fp, c->Bcap, c->stream);
+        issue_forward(c->tt, (int)c->vpl, fp, c->Bcap, c->stream);
         launch_batch_end(st, c->loss.p, c->status.as<int32_t>(), c->nbr_cnt.as<uint32_t>(), c->Bcap, nb, 1, 0, c->stream);
     }
     CK(cudaGetLastError(), "validation launch");
@@ -1377,7 +1397,7 @@ static int run_injected(ep_ctx* c, uint32_t B, int tt, const void* table, void* 
     fp.loss_out = loss_out;
     fp.dloss = (const float*)dloss;
     fp.dloss_f64 = tt == TT_F64;
-    launch_forward(tt, (int)c->vpl, fp, B, s);
+    issue_forward(tt, (int)c->vpl, fp, B, s);
     sort_and_reduce(c, st, tt, out_mode, adam_table, s);
     if (out_mode == OUT_DENSE && adam_table)
         launch_adam_dense(tt, (int)c->vpl, st, adam_table, c->m.as<float>(), c->v.as<float>(), c->gdense.as<float>(),

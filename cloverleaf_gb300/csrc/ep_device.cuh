@@ -170,6 +170,8 @@ struct RowIO {
     struct Raw { V v[NV]; };
     // number of raw slices that fit in about 32 registers
     static constexpr int INFLIGHT = (BYTES >= 128) ? 1 : (128 / BYTES > 8 ? 8 : 128 / BYTES);
+    // half of that, for two groups of loads in turn
+    static constexpr int GROUP = INFLIGHT >= 2 ? INFLIGHT / 2 : 1;
     static __device__ __forceinline__ Raw load_raw(const T* __restrict__ row, int lane) {
         Raw r;
         const V* src = reinterpret_cast<const V*>(row + lane * VPL);
@@ -179,6 +181,20 @@ struct RowIO {
     }
     template <typename A>
     static __device__ __forceinline__ void fma(A (&acc)[VPL], A c, const Raw& r) {
+        if constexpr (std::is_same<T, __nv_bfloat16>::value && std::is_same<A, float>::value && VPL >= 2) {
+            // a BF16 pair widens to FP32 by one shift and one mask
+            union { V v[NV]; uint32_t w[VPL / 2]; } u;
+#pragma unroll
+            for (int i = 0; i < NV; ++i) u.v[i] = r.v[i];
+            A x[VPL];
+#pragma unroll
+            for (int k = 0; k < VPL / 2; ++k) {
+                x[2 * k] = __uint_as_float(u.w[k] << 16);
+                x[2 * k + 1] = __uint_as_float(u.w[k] & 0xffff0000u);
+            }
+            axpy_slice<A, VPL>(acc, c, x);
+            return;
+        }
         union { V v[NV]; T t[VPL]; } u;
 #pragma unroll
         for (int i = 0; i < NV; ++i) u.v[i] = r.v[i];

@@ -303,6 +303,12 @@ __device__ void ares_select(const SampleParams& p, uint64_t rs, uint32_t deg, fl
     }
 }
 
+// Tables of the staged gather; an anchor beyond any of these takes the direct
+// path (k_sample decides, from the counts it has at hand).
+constexpr uint32_t NODE_CAP = 64;     // 1 + neighbours + negatives
+constexpr uint32_t OCC_CAP = 512;     // feature occurrences of one anchor
+constexpr uint32_t ROLE_CAP = 34;     // R + 2
+
 // ---------------------------------------------------------------------------
 // k_sample: one warp per anchor.
 // ---------------------------------------------------------------------------
@@ -577,19 +583,23 @@ __global__ void __launch_bounds__(256) k_sample(SampleParams p) {
     const uint32_t cnt = p.nbr_cnt[a];
     uint64_t occ = 0;
     float unused;
-    if (lane == 0) occ += fd_kept(c.fd, v, salt, 0, (uint32_t)(p.fptr[v + 1] - p.fptr[v]), unused);
+    bool far = false;      // a feature range past 32-bit indices
+    auto count = [&](uint32_t u, uint32_t q) {
+        const uint64_t fs = p.fptr[u], fe = p.fptr[u + 1];
+        far = far || fe > 0xffffffffull;
+        occ += fd_kept(c.fd, v, salt, q, (uint32_t)(fe - fs), unused);
+    };
+    if (lane == 0) count(v, 0);
     const uint32_t* nb = p.nbr + (uint64_t)a * c.Kcap;
-    for (uint32_t q = lane; q < cnt; q += 32) {
-        const uint32_t u = nb[q];
-        occ += fd_kept(c.fd, v, salt, 1 + q, (uint32_t)(p.fptr[u + 1] - p.fptr[u]), unused);
-    }
+    for (uint32_t q = lane; q < cnt; q += 32) count(nb[q], 1 + q);
     const uint32_t* ng = p.neg + (uint64_t)a * c.R;
-    for (uint32_t q = lane; q < c.R; q += 32) {
-        const uint32_t u = ng[q];
-        occ += fd_kept(c.fd, v, salt, 1 + cnt + q, (uint32_t)(p.fptr[u + 1] - p.fptr[u]), unused);
-    }
+    for (uint32_t q = lane; q < c.R; q += 32) count(ng[q], 1 + cnt + q);
     occ = warp_sum<unsigned long long>((unsigned long long)occ);
-    if (lane == 0) p.occ[a] = (uint32_t)min(occ, (uint64_t)0xffffffffu);
+    far = __any_sync(FULL, far);
+    if (lane == 0) {
+        p.occ[a] = (uint32_t)min(occ, (uint64_t)0xffffffffu);
+        p.deferred[a] = far || occ > OCC_CAP || (uint64_t)cnt + c.R >= NODE_CAP || c.R + 2 > ROLE_CAP;
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -799,119 +809,200 @@ __device__ A gather_role_fd(const ForwardParams& p, const T* __restrict__ table,
 }
 
 // ---------------------------------------------------------------------------
-// Staged gather (the common case): per-warp shared-memory tables of the
-// anchor's role nodes and of all their feature occurrences, so that the row
-// pointers of all roles are loaded in one round, all feature ids in one more,
-// and each role's rows are then read eight at a time from the table.
+// Staged gather (the common case): shared-memory tables of the anchor's role
+// nodes and of all their feature occurrences, so that the row pointers of all
+// roles are loaded in one round, all feature ids in one more, and each role's
+// rows are then streamed from the table.  A group of W warps works on one
+// anchor: W = 1 when the batch has warps enough to fill the chip, more for
+// small batches, whose time is one anchor's chain of loads.
 // ---------------------------------------------------------------------------
-constexpr uint32_t NODE_CAP = 64;     // 1 + neighbours + negatives
-constexpr uint32_t OCC_CAP = 512;     // feature occurrences of one anchor
-constexpr uint32_t ROLE_CAP = 34;     // R + 2
 constexpr int FWD_WARPS = 8;
 
-struct WarpTables {
+struct GatherTables {
+    uint2 occ[OCC_CAP];               // feature id and count weight (bits) of each occurrence
     uint32_t node_fs[NODE_CAP];       // first feature index (fptr) of the node
     uint32_t node_n[NODE_CAP];        // feature count of the node (before dropout)
-    uint32_t node_incl[NODE_CAP];     // inclusive prefix of feature counts
+    uint32_t node_incl[NODE_CAP];     // inclusive prefix of kept feature counts
     float node_c[NODE_CAP];           // count weight of the node's occurrences
     uint32_t role_ob[ROLE_CAP + 1];   // first occurrence of each role
     float role_n[ROLE_CAP];           // sum of count weights of each role
-    uint32_t occ_f[OCC_CAP];
-    float occ_c[OCC_CAP];
 };
 
 __device__ __forceinline__ uint32_t node_role(uint32_t q, uint32_t cnt) {
     return q == 0 ? 0u : (q <= cnt ? 1u : 2u + (q - 1u - cnt));
 }
 
-// Phases A and B.  Returns false (warp-uniform) when the anchor does not fit
-// the tables; nothing has been emitted then.
-template <typename A>
-__device__ bool stage_anchor(const ForwardParams& p, WarpTables& W, uint32_t a, uint32_t v, uint32_t cnt,
-                             uint64_t pos, bool emit, uint32_t sbase, uint32_t salt, int lane) {
+// Barrier of the W warps of one anchor (the CTA when W > 1).
+template <int W>
+__device__ __forceinline__ void group_sync() {
+    if constexpr (W == 1) __syncwarp();
+    else __syncthreads();
+}
+
+// Phase A (one warp): the anchor's nodes.  The row pointers of up to 64 nodes
+// are loaded together, two per lane.
+__device__ __forceinline__ void stage_nodes(const ForwardParams& p, GatherTables& S, uint32_t a, uint32_t v, uint32_t cnt,
+                                            uint32_t salt, int lane) {
     const uint32_t R = p.R;
     const uint32_t n_nodes = 1 + cnt + R;
-    if (n_nodes > NODE_CAP || R + 2 > ROLE_CAP) return false;
     const uint32_t* nb = p.nbr + (uint64_t)a * p.Kcap;
     const float* nw = p.nbr_w + (uint64_t)a * p.Kcap;
     const uint32_t* ng = p.neg + (uint64_t)a * R;
-    uint32_t carry = 0;
-    float n1 = 0.f;                  // role 1 weight total (lane-partial)
-    bool big = false;
-    for (uint32_t q0 = 0; q0 < n_nodes; q0 += 32) {
-        const uint32_t q = q0 + lane;
-        uint32_t fn = 0;
+    constexpr int NS = NODE_CAP / 32;
+    uint64_t fs[NS], fe[NS];
+    float c[NS];
+#pragma unroll
+    for (int s = 0; s < NS; ++s) {
+        const uint32_t q = (uint32_t)(32 * s + lane);
+        fs[s] = fe[s] = 0;
+        c[s] = 1.f;
         if (q < n_nodes) {
             uint32_t u;
-            float c;
-            if (q == 0) { u = v; c = 1.f; }
-            else if (q <= cnt) { u = nb[q - 1]; c = nw[q - 1]; }
-            else { u = ng[q - 1 - cnt]; c = 1.f; }
-            const uint64_t fs = p.fptr[u];
-            const uint32_t nall = (uint32_t)(p.fptr[u + 1] - fs);
+            if (q == 0) u = v;
+            else if (q <= cnt) { u = nb[q - 1]; c[s] = nw[q - 1]; }
+            else u = ng[q - 1 - cnt];
+            fs[s] = p.fptr[u];
+            fe[s] = p.fptr[u + 1];
+        }
+    }
+    uint32_t carry = 0;
+    float n1 = 0.f;                  // role 1 weight total (lane-partial)
+#pragma unroll
+    for (int s = 0; s < NS; ++s) {
+        if ((uint32_t)(32 * s) >= n_nodes) break;
+        const uint32_t q = (uint32_t)(32 * s + lane);
+        uint32_t fn = 0;
+        if (q < n_nodes) {
+            const uint32_t nall = (uint32_t)(fe[s] - fs[s]);
             float scal;
             fn = fd_kept(p.fd, v, salt, q, nall, scal);
-            c += scal;
-            big = big || (fs + nall) > 0xffffffffull;
-            W.node_fs[q] = (uint32_t)fs;
-            W.node_n[q] = nall;
-            W.node_c[q] = c;
+            const float cq = c[s] + scal;
+            S.node_fs[q] = (uint32_t)fs[s];
+            S.node_n[q] = nall;
+            S.node_c[q] = cq;
             const uint32_t r = node_role(q, cnt);
-            const float wsum = c * (float)fn;
+            const float wsum = cq * (float)fn;
             if (r == 1) n1 += wsum;
-            else W.role_n[r] = wsum;
+            else S.role_n[r] = wsum;
         }
         const uint32_t incl = warp_incl_scan(fn, lane) + carry;
-        if (q < n_nodes) W.node_incl[q] = incl;
+        if (q < n_nodes) S.node_incl[q] = incl;
         carry = __shfl_sync(FULL, incl, 31);
     }
-    if (__any_sync(FULL, big)) return false;
-    const uint32_t total = carry;
-    if (total > OCC_CAP) return false;
     n1 = warp_sum<float>(n1);
     __syncwarp();
     if (lane == 0) {
-        W.role_n[1] = n1;
-        W.role_ob[0] = 0;
-        W.role_ob[1] = W.node_incl[0];
-        W.role_ob[2] = W.node_incl[cnt];
-        for (uint32_t i = 1; i <= R; ++i) W.role_ob[2 + i] = W.node_incl[cnt + i];
+        S.role_n[1] = n1;
+        S.role_ob[0] = 0;
     }
+    // role r >= 2 starts after the nodes of the roles before it
+    for (uint32_t i = lane; i <= R; i += 32) S.role_ob[2 + i] = S.node_incl[cnt + i];
+    if (lane == 0) S.role_ob[1] = S.node_incl[0];
+}
+
+// Phases A and B by the W warps of an anchor that fits the tables (`tid`
+// counts within the group).
+template <int W>
+__device__ void stage_anchor(const ForwardParams& p, GatherTables& S, uint32_t a, uint32_t v, uint32_t cnt,
+                             uint64_t pos, bool emit, uint32_t sbase, uint32_t salt, int tid) {
+    const uint32_t n_nodes = 1 + cnt + p.R;
+    const int lane = tid & 31, w = tid >> 5;
+    if (W == 1 || w == 0) stage_nodes(p, S, a, v, cnt, salt, lane);
+    group_sync<W>();
     if (p.fd.kind != S_ALL) {
-        // phase B with feature dropout: node by node, the kept positions in
-        // position order (the same keys k_sample counted)
-        __syncwarp();
-        uint32_t o = 0;
-        for (uint32_t q = 0; q < n_nodes; ++q) {
-            const uint32_t nall = W.node_n[q], fs = W.node_fs[q];
-            const float c = W.node_c[q];
-            const uint32_t src = sbase + node_role(q, cnt);
-            const FdNode nd = fd_node(p.fd, v, salt, q, nall, lane);
-            for (uint32_t j0 = 0; j0 < nall; j0 += 32) {
-                const unsigned m = fd_mask(p.fd, nd, v, salt, q, nall, j0, lane);
-                if ((m >> lane) & 1u) {
-                    const uint32_t oo = o + __popc(m & ((1u << lane) - 1u));
-                    const uint32_t f = p.fids[(uint64_t)fs + j0 + lane];
-                    W.occ_f[oo] = f;
-                    W.occ_c[oo] = c;
+        // phase B with feature dropout (the same keys k_sample counted): 32
+        // positions per step, as many whole nodes as fit; a position's rank
+        // among its node's keys comes from shuffles over the node's lanes.
+        // Steps alternate over the warps; a node's output slots are known
+        // from node_incl.  A node of more than 32 features takes a step (and
+        // the per-node walk) for itself.
+        int turn = 0;
+        for (uint32_t q0 = 0; q0 < n_nodes;) {
+            const uint32_t qn = q0 + lane;
+            const uint32_t len = qn < n_nodes ? S.node_n[qn] : 33u;
+            const uint32_t incl = warp_incl_scan(len, lane);
+            uint32_t m = (uint32_t)__popc(__ballot_sync(FULL, qn < n_nodes && incl <= 32u));
+            const bool mine = W == 1 || (turn++ % W) == w;
+            if (m == 0) {
+                if (mine) {
+                    const uint32_t nall = S.node_n[q0], fs = S.node_fs[q0];
+                    uint32_t o = q0 ? S.node_incl[q0 - 1] : 0u;
+                    const FdNode nd = fd_node(p.fd, v, salt, q0, nall, lane);
+                    for (uint32_t j0 = 0; j0 < nall; j0 += 32) {
+                        const unsigned km = fd_mask(p.fd, nd, v, salt, q0, nall, j0, lane);
+                        if ((km >> lane) & 1u) {
+                            const uint32_t oo = o + __popc(km & ((1u << lane) - 1u));
+                            const uint32_t f = p.fids[(uint64_t)fs + j0 + lane];
+                            S.occ[oo] = make_uint2(f, __float_as_uint(S.node_c[q0]));
+                            if (emit) {
+                                p.item_f[pos + oo] = f;
+                                p.item_src[pos + oo] = sbase + node_role(q0, cnt);
+                                p.item_c[pos + oo] = S.node_c[q0];
+                            }
+                        }
+                        o += __popc(km);
+                    }
+                }
+                ++q0;
+                continue;
+            }
+            if (mine) {
+                const uint32_t total = __shfl_sync(FULL, incl, (int)m - 1);
+                // owner: the first node of the step whose inclusive prefix exceeds the lane
+                uint32_t k = 0;
+#pragma unroll
+                for (int st = 16; st >= 1; st >>= 1) {
+                    const uint32_t iv = __shfl_sync(FULL, incl, (int)(k + st - 1) & 31);
+                    if (k + st <= m && iv <= (uint32_t)lane) k += st;
+                }
+                const bool act = (uint32_t)lane < total;
+                const uint32_t kk = act ? k : 0u;
+                const uint32_t end = __shfl_sync(FULL, incl, (int)kk);
+                const uint32_t n = __shfl_sync(FULL, len, (int)kk);
+                const uint32_t beg = end - n, q = q0 + kk, j = (uint32_t)lane - beg;
+                const uint32_t key = act ? fd_key(p.fd, v, salt, q, j) : 0xffffffffu;
+                uint32_t rank = 0;
+                const uint32_t most = __reduce_max_sync(FULL, act ? n : 0u);
+                for (uint32_t t = 0; t < most; ++t) {
+                    const uint32_t kt = __shfl_sync(FULL, key, (int)(beg + t) & 31);
+                    rank += t < n && (kt < key || (kt == key && t < j));
+                }
+                bool sel;
+                if (p.fd.kind == S_FIXED) {
+                    sel = act && rank < min(p.fd.k, n);
+                } else {
+                    const unsigned own = (n >= 32u ? FULL : ((1u << n) - 1u)) << (beg & 31u);
+                    const bool pass = act && key < p.fd.thr;
+                    const unsigned pm = __ballot_sync(FULL, pass);
+                    sel = act && ((pm & own) ? pass : rank == 0u);
+                }
+                const unsigned sm = __ballot_sync(FULL, sel);
+                if (sel) {
+                    const unsigned below = ((1u << lane) - 1u) & ~((1u << beg) - 1u);   // beg <= lane < 32
+                    const uint32_t oo = (q ? S.node_incl[q - 1] : 0u) + __popc(sm & below);
+                    const uint32_t f = p.fids[(uint64_t)S.node_fs[q] + j];
+                    const float c = S.node_c[q];
+                    S.occ[oo] = make_uint2(f, __float_as_uint(c));
                     if (emit) {
                         p.item_f[pos + oo] = f;
-                        p.item_src[pos + oo] = src;
+                        p.item_src[pos + oo] = sbase + node_role(q, cnt);
                         p.item_c[pos + oo] = c;
                     }
                 }
-                o += __popc(m);
             }
+            q0 += m;
         }
-        __syncwarp();
-        return true;
+        group_sync<W>();
+        return;
     }
+    const uint32_t total = S.node_incl[n_nodes - 1];
     // phase B: one feature id per lane, four batches of loads in flight
-    for (uint32_t o0 = 0; o0 < total; o0 += 128) {
+    constexpr uint32_t STEP = 32 * W;
+    for (uint32_t o0 = 0; o0 < total; o0 += 4 * STEP) {
         uint32_t fid[4], q_of[4];
 #pragma unroll
         for (int b = 0; b < 4; ++b) {
-            const uint32_t o = o0 + b * 32 + lane;
+            const uint32_t o = o0 + b * STEP + tid;
             fid[b] = 0;
             q_of[b] = 0;
             if (o < total) {
@@ -919,20 +1010,19 @@ __device__ bool stage_anchor(const ForwardParams& p, WarpTables& W, uint32_t a, 
                 uint32_t lo = 0, hi = n_nodes - 1;
                 while (lo < hi) {
                     const uint32_t mid = (lo + hi) >> 1;
-                    if (W.node_incl[mid] > o) hi = mid; else lo = mid + 1;
+                    if (S.node_incl[mid] > o) hi = mid; else lo = mid + 1;
                 }
-                const uint32_t excl = lo ? W.node_incl[lo - 1] : 0u;
+                const uint32_t excl = lo ? S.node_incl[lo - 1] : 0u;
                 q_of[b] = lo;
-                fid[b] = p.fids[(uint64_t)W.node_fs[lo] + (o - excl)];
+                fid[b] = p.fids[(uint64_t)S.node_fs[lo] + (o - excl)];
             }
         }
 #pragma unroll
         for (int b = 0; b < 4; ++b) {
-            const uint32_t o = o0 + b * 32 + lane;
+            const uint32_t o = o0 + b * STEP + tid;
             if (o < total) {
-                const float c = W.node_c[q_of[b]];
-                W.occ_f[o] = fid[b];
-                W.occ_c[o] = c;
+                const float c = S.node_c[q_of[b]];
+                S.occ[o] = make_uint2(fid[b], __float_as_uint(c));
                 if (emit) {
                     p.item_f[pos + o] = fid[b];
                     p.item_src[pos + o] = sbase + node_role(q_of[b], cnt);
@@ -941,30 +1031,35 @@ __device__ bool stage_anchor(const ForwardParams& p, WarpTables& W, uint32_t a, 
             }
         }
     }
-    __syncwarp();
-    return true;
+    group_sync<W>();
 }
 
-// Phase C: every role's rows in occurrence order (role-major), U rows in
-// flight across role boundaries.  As each role closes, its mean
-// sum(c * row) / sum(c) is written to the role's direction row and its weight
-// total sum(c) to scale; the loss kernel reads both back.
+// Phase C (one warp): the rows of roles [r0, r1) in occurrence order
+// (role-major), two groups of G rows in flight across role boundaries.  As
+// each role closes, its mean sum(c * row) / sum(c) is written to the role's
+// direction row and its weight total sum(c) to scale; the loss kernel reads
+// both back.  Lanes past the row (dims < 32 x VPL) read its last slice and
+// store nothing, so that the loop has no lane-dependent branch.
 template <typename T, typename A, int VPL>
 __device__ __forceinline__ void roles_from_table(const ForwardParams& p, const T* __restrict__ table,
-                                                 const WarpTables& W, uint32_t NR, uint64_t sbase, int lane,
-                                                 bool lane_on) {
+                                                 const GatherTables& S, uint32_t r0, uint32_t r1, uint64_t sbase,
+                                                 int lane) {
     using IO = RowIO<T, VPL>;
-    constexpr int U = IO::INFLIGHT;
+    constexpr int G = IO::GROUP;
     const uint32_t dpad = p.dpad;
+    const bool lane_on = (uint32_t)(lane * VPL) < dpad;
+    const int lane_ld = lane_on ? lane : (int)(dpad / VPL) - 1;
     A* dir = (A*)p.dir;
     A* scale = (A*)p.scale;
-    const uint32_t total = W.role_ob[NR];
+    uint32_t r = r0;
+    if (r >= r1) return;
+    const uint32_t total = S.role_ob[r1];
+    uint32_t rend = S.role_ob[r + 1];
     A acc[VPL];
 #pragma unroll
     for (int k = 0; k < VPL; ++k) acc[k] = 0;
-    uint32_t r = 0, rend = W.role_ob[1];
     auto close_role = [&]() {
-        const A n = (A)W.role_n[r];
+        const A n = (A)S.role_n[r];
         if (lane_on) {
             const A rn = (A)1 / n;
             A m[VPL];
@@ -976,25 +1071,45 @@ __device__ __forceinline__ void roles_from_table(const ForwardParams& p, const T
 #pragma unroll
         for (int k = 0; k < VPL; ++k) acc[k] = 0;
         ++r;
-        if (r < NR) rend = W.role_ob[r + 1];
+        if (r < r1) rend = S.role_ob[r + 1];
     };
-    for (uint32_t j = 0; j < total; j += U) {
-        typename IO::Raw rows[U];
-        if (lane_on) {
+    auto fetch = [&](typename IO::Raw (&x)[G], uint32_t j) {
+        if (j + G <= total) {
 #pragma unroll
-            for (int u = 0; u < U; ++u)
-                if (j + u < total) rows[u] = IO::load_raw(table + (uint64_t)W.occ_f[j + u] * dpad, lane);
+            for (int u = 0; u < G; ++u) x[u] = IO::load_raw(table + (uint64_t)S.occ[j + u].x * dpad, lane_ld);
+        } else {
+#pragma unroll
+            for (int u = 0; u < G; ++u)
+                if (j + u < total) x[u] = IO::load_raw(table + (uint64_t)S.occ[j + u].x * dpad, lane_ld);
+        }
+    };
+    auto take = [&](const typename IO::Raw (&x)[G], uint32_t j) {
+        if (j + G <= rend) {                 // all of one role
+#pragma unroll
+            for (int u = 0; u < G; ++u) IO::template fma<A>(acc, (A)__uint_as_float(S.occ[j + u].y), x[u]);
+            return;
         }
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const uint32_t jj = j + u;
-            if (jj < total) {
-                while (jj >= rend) close_role();
-                if (lane_on) IO::template fma<A>(acc, (A)W.occ_c[jj], rows[u]);
+        for (int u = 0; u < G; ++u) {
+            if (j + u < total) {
+                while (j + u >= rend) close_role();
+                IO::template fma<A>(acc, (A)__uint_as_float(S.occ[j + u].y), x[u]);
             }
         }
+    };
+    uint32_t j = S.role_ob[r0];
+    typename IO::Raw x[G], y[G];
+    fetch(x, j);
+    while (j < total) {
+        fetch(y, j + G);
+        take(x, j);
+        j += G;
+        if (j >= total) break;
+        fetch(x, j + G);
+        take(y, j);
+        j += G;
     }
-    while (r < NR) close_role();
+    while (r < r1) close_role();
 }
 
 template <typename A, int VPL>
@@ -1030,45 +1145,76 @@ __device__ __forceinline__ bool warp_all_finite(const A (&x)[VPL]) {
     return __all_sync(FULL, ok);
 }
 
-// k_fwd_gather: one warp per anchor; the mean of every role of the anchor
+// The gather of anchor a (phases A-C) by its W warps: the mean of every role
 // (h(v), ~h(v), h(u_1..R)) into its direction row, the role's weight total
-// into scale, and the anchor's gradient items.  STAGED = true: the common path
-// through the per-warp tables; anchors that do not fit are flagged in
-// p.deferred and skipped.  STAGED = false: the direct path, run afterwards for
-// the flagged anchors only (every anchor when p.deferred is null).  Both
-// produce identical items, means and totals.
-// The staged gather of anchor a (phases A-C) by one warp; anchors that do not
-// fit the tables are flagged for the direct path.
-template <typename T, typename A, int VPL>
-__device__ __forceinline__ void gather_staged(const ForwardParams& p, WarpTables& W, uint32_t a, int lane) {
+// into scale, and the anchor's gradient items.  Anchors that do not fit the
+// tables (flagged by k_sample) are left to k_fwd_direct.  The W warps take consecutive ranges of roles of about equal length;
+// every role is summed by one warp in occurrence order, so the results do not
+// depend on W.
+template <typename T, typename A, int VPL, int W>
+__device__ __forceinline__ void gather_staged(const ForwardParams& p, GatherTables& S, uint32_t a, int tid) {
+    if (p.deferred[a]) return;       // uniform over the group
     const uint32_t NR = p.R + 2;
-    const bool lane_on = (uint32_t)(lane * VPL) < p.dpad;
     const uint32_t v = p.anchors[a];
     const bool emit = p.emit && p.st->n_items > 0;
     const uint64_t pos = emit ? p.occ_off[a] : 0;
     const uint64_t sbase = (uint64_t)a * NR;
     const uint32_t cnt = p.nbr_cnt[a];
     const uint32_t salt = p.eval ? 0xffffffffu : (uint32_t)p.st->step;   // as k_sample
-    const bool staged = stage_anchor<A>(p, W, a, v, cnt, pos, emit, (uint32_t)sbase, salt, lane);
-    if (lane == 0) p.deferred[a] = staged ? 0 : 1;
-    if (staged) roles_from_table<T, A, VPL>(p, (const T*)p.table, W, NR, sbase, lane, lane_on);
-    __syncwarp();
+    stage_anchor<W>(p, S, a, v, cnt, pos, emit, (uint32_t)sbase, salt, tid);
+    uint32_t r0 = 0, r1 = NR;
+    if constexpr (W > 1) {
+        // warp w starts at the first role at or past w / W of the occurrences
+        const uint32_t w = (uint32_t)tid >> 5, lane = (uint32_t)tid & 31u, total = S.role_ob[NR];
+        auto first = [&](uint32_t ww) {
+            uint32_t below = 0;
+            for (uint32_t b = 0; b < NR; b += 32) {
+                const uint32_t i = b + lane;
+                below += (uint32_t)__popc(__ballot_sync(FULL, i < NR && S.role_ob[i] * W < ww * total));
+            }
+            return below;
+        };
+        r0 = first(w);
+        r1 = w + 1 == W ? NR : first(w + 1);
+    }
+    roles_from_table<T, A, VPL>(p, (const T*)p.table, S, r0, r1, sbase, tid & 31);
+    group_sync<W>();
 }
 
-template <typename T, typename A, int VPL, bool STAGED>
-__global__ void __launch_bounds__(256, STAGED ? (VPL <= 8 ? 4 : 3) : 1) k_fwd_gather(ForwardParams p) {
+// k_fwd_gather: W warps per anchor.  W = 1: CTAs of a few warps, each with
+// its own anchor and tables.  W > 1: a CTA per anchor.  Bound by the latency
+// of its dependent loads (node, row pointer, feature id, row) and by issue
+// slots: 75 instructions per row before the streaming loop below lost its
+// per-row checks.  Measured per batch: 8,192 anchors x 256 BF16 (756k rows)
+// 96 -> 68 us, 32,768 anchors (5.6M rows) 507 -> 350 us, 1,024 anchors x 128
+// FP32 at 4 warps each 52 -> 23 us.
+template <typename T, typename A, int VPL, int W>
+__global__ void __launch_bounds__(W == 1 ? 256 : 32 * W, W == 1 ? (VPL <= 8 ? 4 : 3) : (VPL <= 8 ? 32 / W : 1))
+    k_fwd_gather(const __grid_constant__ ForwardParams p) {
+    pdl_wait();
+    pdl_trigger();
+    extern __shared__ __align__(16) unsigned char fwd_smem[];
+    GatherTables* S = reinterpret_cast<GatherTables*>(fwd_smem);
+    const uint32_t n = p.st->n_anchors;
+    if constexpr (W == 1) {
+        const uint32_t a = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+        if (a < n) gather_staged<T, A, VPL, 1>(p, S[threadIdx.x >> 5], a, threadIdx.x & 31);
+    } else {
+        if (blockIdx.x < n) gather_staged<T, A, VPL, W>(p, S[0], blockIdx.x, threadIdx.x);
+    }
+}
+
+// k_fwd_direct: every role's nodes walked in global memory, for the anchors
+// that do not fit the staged gather's tables (p.deferred, set by k_sample).
+// One warp per anchor; identical items, means and totals.  In replayed graphs
+// it runs beside the staged gather.
+template <typename T, typename A, int VPL>
+__global__ void __launch_bounds__(256) k_fwd_direct(const __grid_constant__ ForwardParams p) {
     pdl_wait();
     pdl_trigger();
     const int lane = threadIdx.x & 31;
-    const uint32_t n = p.st->n_anchors;
-    if constexpr (STAGED) {
-        extern __shared__ __align__(16) unsigned char fwd_smem[];
-        const uint32_t a = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-        if (a < n) gather_staged<T, A, VPL>(p, reinterpret_cast<WarpTables*>(fwd_smem)[threadIdx.x >> 5], a, lane);
-        return;
-    }
     const uint32_t a = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (a >= n) return;
+    if (a >= p.st->n_anchors || !p.deferred[a]) return;
     const uint32_t R = p.R, NR = R + 2, dpad = p.dpad;
     const bool lane_on = (uint32_t)(lane * VPL) < dpad;
     const T* __restrict__ table = (const T*)p.table;
@@ -1078,29 +1224,26 @@ __global__ void __launch_bounds__(256, STAGED ? (VPL <= 8 ? 4 : 3) : 1) k_fwd_ga
     const uint64_t sbase = (uint64_t)a * NR;
     const uint32_t cnt = p.nbr_cnt[a];
     const uint32_t salt = p.eval ? 0xffffffffu : (uint32_t)p.st->step;   // as k_sample
-    {
-        if (p.deferred && !p.deferred[a]) return;
-        A* dir = (A*)p.dir;
-        A* scale = (A*)p.scale;
-        for (uint32_t r = 0; r < NR; ++r) {
-            const uint32_t* nodes = r == 0 ? &v : (r == 1 ? p.nbr + (uint64_t)a * p.Kcap : p.neg + (uint64_t)a * R + (r - 2));
-            const float* w = r == 1 ? p.nbr_w + (uint64_t)a * p.Kcap : nullptr;
-            const uint32_t count = r == 1 ? cnt : 1u;
-            const uint32_t slot0 = r == 0 ? 0u : (r == 1 ? 1u : 1u + cnt + (r - 2));
-            A acc[VPL];
-            const A nr = p.fd.kind == S_ALL
-                             ? gather_role<T, A, VPL>(p, table, nodes, w, count, (uint32_t)(sbase + r), pos, emit, acc,
-                                                      lane, lane_on)
-                             : gather_role_fd<T, A, VPL>(p, table, nodes, w, count, slot0, v, salt,
-                                                         (uint32_t)(sbase + r), pos, emit, acc, lane, lane_on);
-            if (lane_on) {
-                const A rn = (A)1 / nr;
+    A* dir = (A*)p.dir;
+    A* scale = (A*)p.scale;
+    for (uint32_t r = 0; r < NR; ++r) {
+        const uint32_t* nodes = r == 0 ? &v : (r == 1 ? p.nbr + (uint64_t)a * p.Kcap : p.neg + (uint64_t)a * R + (r - 2));
+        const float* w = r == 1 ? p.nbr_w + (uint64_t)a * p.Kcap : nullptr;
+        const uint32_t count = r == 1 ? cnt : 1u;
+        const uint32_t slot0 = r == 0 ? 0u : (r == 1 ? 1u : 1u + cnt + (r - 2));
+        A acc[VPL];
+        const A nr = p.fd.kind == S_ALL
+                         ? gather_role<T, A, VPL>(p, table, nodes, w, count, (uint32_t)(sbase + r), pos, emit, acc, lane,
+                                                  lane_on)
+                         : gather_role_fd<T, A, VPL>(p, table, nodes, w, count, slot0, v, salt, (uint32_t)(sbase + r), pos,
+                                                     emit, acc, lane, lane_on);
+        if (lane_on) {
+            const A rn = (A)1 / nr;
 #pragma unroll
-                for (int k = 0; k < VPL; ++k) acc[k] *= rn;
-                store_row<A, VPL, A>(dir + (sbase + r) * dpad, lane, acc);
-            }
-            if (lane == 0) scale[sbase + r] = nr;
+            for (int k = 0; k < VPL; ++k) acc[k] *= rn;
+            store_row<A, VPL, A>(dir + (sbase + r) * dpad, lane, acc);
         }
+        if (lane == 0) scale[sbase + r] = nr;
     }
 }
 
@@ -1112,11 +1255,11 @@ __global__ void __launch_bounds__(256, STAGED ? (VPL <= 8 ? 4 : 3) : 1) k_fwd_ga
 // register budget of the loop (the one-shot kernel is at its 64-register
 // limit at 4).
 template <typename T, typename A, int VPL, int MINB>
-__global__ void __launch_bounds__(256, MINB) k_fwd_gather_queue(ForwardParams p) {
+__global__ void __launch_bounds__(256, MINB) k_fwd_gather_queue(const __grid_constant__ ForwardParams p) {
     pdl_wait();
     pdl_trigger();
     extern __shared__ __align__(16) unsigned char fwd_smem[];
-    WarpTables& W = reinterpret_cast<WarpTables*>(fwd_smem)[threadIdx.x >> 5];
+    GatherTables& S = reinterpret_cast<GatherTables*>(fwd_smem)[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
     const uint32_t n = p.st->n_anchors;
     for (;;) {
@@ -1124,7 +1267,7 @@ __global__ void __launch_bounds__(256, MINB) k_fwd_gather_queue(ForwardParams p)
         if (lane == 0) a = atomicAdd(&p.st->fwd_next, 1u);
         a = __shfl_sync(FULL, a, 0);
         if (a >= n) break;
-        gather_staged<T, A, VPL>(p, W, a, lane);
+        gather_staged<T, A, VPL, 1>(p, S, a, lane);
     }
 }
 
@@ -1134,8 +1277,7 @@ __global__ void __launch_bounds__(256, MINB) k_fwd_gather_queue(ForwardParams p)
 // path's role walk with no lane reading rows.  In replayed graphs it runs
 // ahead of the radix sort on a second stream, so that the sort overlaps the
 // gathers, which then run with emission off.
-template <typename T, typename A, int VPL>
-__global__ void __launch_bounds__(256) k_fwd_emit(ForwardParams p) {
+__global__ void __launch_bounds__(256) k_fwd_emit(const __grid_constant__ ForwardParams p) {
     pdl_wait();
     pdl_trigger();
     const int lane = threadIdx.x & 31;
@@ -1149,19 +1291,22 @@ __global__ void __launch_bounds__(256) k_fwd_emit(ForwardParams p) {
     const uint32_t cnt = p.nbr_cnt[a];
     const uint32_t salt = p.eval ? 0xffffffffu : (uint32_t)p.st->step;   // as k_sample
     extern __shared__ __align__(16) unsigned char fwd_smem[];
-    WarpTables& W = reinterpret_cast<WarpTables*>(fwd_smem)[threadIdx.x >> 5];
-    if (stage_anchor<A>(p, W, a, v, cnt, pos, true, (uint32_t)sbase, salt, lane)) return;
+    GatherTables& S = reinterpret_cast<GatherTables*>(fwd_smem)[threadIdx.x >> 5];
+    if (!p.deferred[a]) {
+        stage_anchor<1>(p, S, a, v, cnt, pos, true, (uint32_t)sbase, salt, lane);
+        return;
+    }
     for (uint32_t r = 0; r < NR; ++r) {
         const uint32_t* nodes = r == 0 ? &v : (r == 1 ? p.nbr + (uint64_t)a * p.Kcap : p.neg + (uint64_t)a * R + (r - 2));
         const float* w = r == 1 ? p.nbr_w + (uint64_t)a * p.Kcap : nullptr;
         const uint32_t count = r == 1 ? cnt : 1u;
         const uint32_t slot0 = r == 0 ? 0u : (r == 1 ? 1u : 1u + cnt + (r - 2));
-        A acc[VPL];
+        float acc[1];
         if (p.fd.kind == S_ALL)
-            gather_role<T, A, VPL>(p, nullptr, nodes, w, count, (uint32_t)(sbase + r), pos, true, acc, lane, false);
+            gather_role<float, float, 1>(p, nullptr, nodes, w, count, (uint32_t)(sbase + r), pos, true, acc, lane, false);
         else
-            gather_role_fd<T, A, VPL>(p, nullptr, nodes, w, count, slot0, v, salt, (uint32_t)(sbase + r), pos, true, acc,
-                                      lane, false);
+            gather_role_fd<float, float, 1>(p, nullptr, nodes, w, count, slot0, v, salt, (uint32_t)(sbase + r), pos, true,
+                                            acc, lane, false);
     }
 }
 
@@ -1703,13 +1848,32 @@ void launch_scan_occ(BatchState* st, uint32_t* occ, uint32_t cap, uint64_t items
     launch_chain(k_scan_occ, 1, 1024, 0, s, st, occ, items_cap);
 }
 
+// Warps per anchor of the staged gather, by the batch's anchors.  One warp
+// each fills the chip's 152 x 32 gather slots from about 5,000 anchors on;
+// below that, the time is one anchor's chain, which more warps shorten until
+// they wait for each other.  Forward stage in us at 1 / 2 / 4 / 8 warps: 225
+// anchors (sbm10k, 64 FP32) 25.1 / 21.4 / 20.9 / 20.5; 1,024 (cl1m, 128 FP32)
+// 47.6 / 38.0 / 37.5 / 42.2; 8,192 (cl10m, 256 BF16) 110 / 118 / - / -.
+static uint32_t gather_split(const ForwardParams& p, uint32_t cap) {
+    if (p.gather_split) return p.gather_split;
+    return cap <= 2048 ? 4 : (cap <= 4096 ? 2 : 1);
+}
+
 template <typename T, typename A, int VPL>
 static void fwd_launch(const ForwardParams& p, uint32_t cap, cudaStream_t s, int part) {
+    if (part == FWD_LOSS) {
+        launch_chain(k_fwd_loss<T, A, VPL>, (cap + 3) / 4, 128, 0, s, p);
+        return;
+    }
+    if (part == FWD_DIRECT) {
+        launch_chain(k_fwd_direct<T, A, VPL>, (cap + 7) / 8, 256, 0, s, p);
+        return;
+    }
     const uint32_t blocks = (cap + FWD_WARPS - 1) / FWD_WARPS;
-    const size_t smem = sizeof(WarpTables) * FWD_WARPS;
+    const size_t smem = sizeof(GatherTables) * FWD_WARPS;
     static bool attr = false;   // opt in to > 48 KB of dynamic shared memory once
     if (!attr) {
-        cudaFuncSetAttribute(k_fwd_gather<T, A, VPL, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaFuncSetAttribute(k_fwd_gather<T, A, VPL, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         cudaFuncSetAttribute(k_fwd_gather_queue<T, A, VPL, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         cudaFuncSetAttribute(k_fwd_gather_queue<T, A, VPL, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         attr = true;
@@ -1718,21 +1882,15 @@ static void fwd_launch(const ForwardParams& p, uint32_t cap, cudaStream_t s, int
     // smaller CTAs free their slots sooner when anchors differ in work
     const uint32_t gw = p.gather_warps >= 1 && p.gather_warps <= (uint32_t)FWD_WARPS ? p.gather_warps : FWD_WARPS;
     const uint32_t gblocks = (cap + gw - 1) / gw;
-    const size_t gsmem = sizeof(WarpTables) * gw;
-    if (part == FWD_EMIT) {
-        launch_chain(k_fwd_emit<T, A, VPL>, gblocks, 32 * gw, gsmem, s, p);
-        return;
-    }
-    if (part != FWD_LOSS) {
-        if (p.gather_ctas > 2 * 152)
-            launch_chain(k_fwd_gather_queue<T, A, VPL, 3>, std::min(p.gather_ctas, blocks), 32 * FWD_WARPS, smem, s, p);
-        else if (p.gather_ctas)
-            launch_chain(k_fwd_gather_queue<T, A, VPL, 2>, std::min(p.gather_ctas, blocks), 32 * FWD_WARPS, smem, s, p);
-        else
-            launch_chain(k_fwd_gather<T, A, VPL, true>, gblocks, 32 * gw, gsmem, s, p);
-        launch_chain(k_fwd_gather<T, A, VPL, false>, blocks, 32 * FWD_WARPS, 0, s, p);
-    }
-    if (part != FWD_GATHER) launch_chain(k_fwd_loss<T, A, VPL>, (cap + 3) / 4, 128, 0, s, p);
+    const size_t gsmem = sizeof(GatherTables) * gw, one = sizeof(GatherTables);
+    const uint32_t split = gather_split(p, cap);
+    if (p.gather_ctas > 2 * 152)
+        launch_chain(k_fwd_gather_queue<T, A, VPL, 3>, std::min(p.gather_ctas, blocks), 32 * FWD_WARPS, smem, s, p);
+    else if (p.gather_ctas)
+        launch_chain(k_fwd_gather_queue<T, A, VPL, 2>, std::min(p.gather_ctas, blocks), 32 * FWD_WARPS, smem, s, p);
+    else if (split == 4) launch_chain(k_fwd_gather<T, A, VPL, 4>, cap, 128, one, s, p);
+    else if (split == 2) launch_chain(k_fwd_gather<T, A, VPL, 2>, cap, 64, one, s, p);
+    else launch_chain(k_fwd_gather<T, A, VPL, 1>, gblocks, 32 * gw, gsmem, s, p);
 }
 
 template <typename T, typename A>
@@ -1750,6 +1908,11 @@ void launch_forward(int tt, int vpl, const ForwardParams& p, uint32_t cap, cudaS
     if (tt == TT_F32) fwd_dispatch<float, float>(vpl, p, cap, s, part);
     else if (tt == TT_BF16) fwd_dispatch<__nv_bfloat16, float>(vpl, p, cap, s, part);
     else fwd_dispatch<double, double>(vpl, p, cap, s, part);
+}
+
+void launch_emit(const ForwardParams& p, uint32_t cap, cudaStream_t s) {
+    const uint32_t gw = p.gather_warps >= 1 && p.gather_warps <= (uint32_t)FWD_WARPS ? p.gather_warps : FWD_WARPS;
+    launch_chain(k_fwd_emit, (cap + gw - 1) / gw, 32 * gw, sizeof(GatherTables) * gw, s, p);
 }
 
 void launch_batch_end(BatchState* st, const void* loss, const int32_t* status, const uint32_t* nbr_cnt,

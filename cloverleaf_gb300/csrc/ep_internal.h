@@ -7,9 +7,10 @@
 //   k_batch_begin  -> BatchState (batch range, lr, Adam bias corrections)
 //   k_sample       -> anchors, sampled neighbours, negatives, occurrence counts
 //   k_scan_occ     -> exclusive item offsets per anchor
-//   k_forward      -> role means, loss, per-role gradient directions and
-//                     scales, one item (feature, role-src, count) per feature
-//                     occurrence, written at deterministic offsets
+//   k_fwd_gather   -> role means and one item (feature, role-src, count) per
+//                     feature occurrence, written at deterministic offsets
+//                     (k_fwd_direct for anchors too big for its tables)
+//   k_fwd_loss     -> loss, per-role gradient directions and scales
 //   radix sort     -> items stably ordered by feature id
 //   k_reduce       -> per-feature gradient = sum over kept items, with the
 //                     first-occurrence rule; fused Adam (FUSED) or a dense
@@ -129,6 +130,7 @@ struct SampleParams {
     uint32_t* nbr_cnt;
     uint32_t* neg;
     uint32_t* occ;          // per-anchor item counts
+    uint8_t* deferred;      // [n_anchors]: 1 = the anchor does not fit the staged gather's tables
 };
 
 struct ForwardParams {
@@ -154,8 +156,9 @@ struct ForwardParams {
     int dloss_f64;
     int emit;                 // 0: forward only (validation)
     uint64_t items_cap;
-    uint8_t* deferred;        // [n_anchors]: 1 = anchor left to the direct path
+    uint8_t* deferred;        // [n_anchors]: 1 = anchor left to k_fwd_direct (set by k_sample)
     uint32_t gather_warps;    // warps per CTA of the one-warp-per-anchor gather and item emission (1-8; 0 = 8)
+    uint32_t gather_split;    // warps per anchor of the staged gather (1, 2, 4; 0 = by batch size)
     uint32_t gather_ctas;     // staged gather: 0 = a warp per anchor; else this many persistent CTAs
                               // whose warps take anchors from BatchState::fwd_next
     // outputs
@@ -214,10 +217,12 @@ void launch_batch_begin(BatchState* st, uint32_t n_order, uint32_t batch_cap,
 void launch_sample(const SampleParams& p, cudaStream_t s);
 void launch_scan_occ(BatchState* st, uint32_t* occ, uint32_t cap, uint64_t items_cap,
                      cudaStream_t s);
-// part: FWD_ALL, the gathers alone (they emit the items when ForwardParams
-// says so), the loss alone, or the item emission alone (k_fwd_emit)
-enum ForwardPart : int { FWD_ALL = 0, FWD_GATHER = 1, FWD_LOSS = 2, FWD_EMIT = 3 };
-void launch_forward(int tt, int vpl, const ForwardParams& p, uint32_t cap, cudaStream_t s, int part = FWD_ALL);
+// part: the staged gather, the direct gather of the anchors that do not fit
+// its tables (independent of it), or the loss (after both)
+enum ForwardPart : int { FWD_GATHER = 0, FWD_DIRECT = 1, FWD_LOSS = 2 };
+void launch_forward(int tt, int vpl, const ForwardParams& p, uint32_t cap, cudaStream_t s, int part);
+// the item emission alone (k_fwd_emit)
+void launch_emit(const ForwardParams& p, uint32_t cap, cudaStream_t s);
 void launch_radix_sort(BatchState* st, uint32_t* keys, uint32_t* keys_alt, const uint32_t* item_src,
                        const float* item_c, uint2* vals, uint2* vals_alt, uint32_t* hist, uint64_t cap,
                        int key_bits, uint32_t** sorted_keys, uint2** sorted_vals, cudaStream_t s);

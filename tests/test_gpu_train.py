@@ -351,3 +351,30 @@ def test_level_one_tuning_keeps_results_identical():
         ctx.train_batches(110)
         tables.append(ctx.get_table(w["n_feat"], w["ep"]["dims"]))
     assert np.array_equal(tables[0], tables[1])
+
+
+@pytest.mark.parametrize("max_features", [None, 3.0, 0.4])
+def test_gather_split_gives_the_same_table(monkeypatch, max_features):
+    # 1, 2 or 4 warps per anchor; nodes of 1 to 40 features (dropout packs
+    # whole nodes of up to 32 into a step), some anchors past the tables
+    from tests._cases import random_problem
+    prob = random_problem(98, n=2000, n_feat=5000, dims=52, deg=(1, 30), feats=(1, 40))
+    tables = []
+    for split in ("1", "2", "4"):
+        monkeypatch.setenv("EP_GATHER_SPLIT", split)
+        for form, graphs in ((_native.FORM_FUSED_BF16, 1), (_native.FORM_FUSED_BF16, 0)):
+            cfg = _native.default_config()
+            cfg.use_graphs, cfg.form = graphs, form
+            cfg.dims, cfg.negatives, cfg.loss, cfg.gamma = 52, 7, _native.LOSS_STARSPACE, 0.5
+            cfg.batch_size, cfg.passes, cfg.valid_pct = 300, 1, 0.0
+            cfg.max_nodes_kind, cfg.max_nodes = _native.SAMPLE_FIXED, 20.0
+            if max_features is not None:
+                cfg.max_features = max_features
+                cfg.max_features_kind = _native.SAMPLE_PROB if max_features < 1 else _native.SAMPLE_FIXED
+            ctx = _native.Context(cfg)
+            ctx.upload_graph(prob["rows"], prob["cols"], None)
+            ctx.upload_features(prob["fptr"], prob["fids"], prob["n_feat"])
+            ctx.set_table(None)
+            assert ctx.train_batches(9)["kept_anchors"] > 0
+            tables.append(ctx.get_table(prob["n_feat"], 52))
+    assert all(np.array_equal(tables[0], t) for t in tables[1:])
