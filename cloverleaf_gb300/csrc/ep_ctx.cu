@@ -94,6 +94,8 @@ struct ep_ctx {
     DevBuf check;   // CSR validation result / bound histogram scratch
     uint32_t long_cap = 0;   // owner chunks per parity in long_list
     uint64_t items_cap = 0;
+    uint64_t typ_items = 0;   // items the batches in flight are expected to emit (launch shapes only)
+    uint64_t train_items = 0; // the same of a training batch
     uint32_t buf_B = 0, buf_K = 0, buf_es = 0;
     uint32_t chunk = 128;
     // FUSED form's Adam placement: 0 = by the reducing warp as each feature
@@ -110,6 +112,8 @@ struct ep_ctx {
     // persistent reducer grid (CTAs whose warps take chunks from a work
     // counter); 0 = one warp per chunk
     uint32_t red_ctas = 0;
+    // warps per reducer chunk (1, 2, 4); 0 = by the batch's chunk count
+    uint32_t red_split = 0;
     // warps per CTA of the one-warp-per-anchor gather (1-8): small CTAs free
     // their slots sooner when anchors differ in work (2: forward 0.164 ->
     // 0.150 ms per batch on the 10M-node graph)
@@ -288,11 +292,12 @@ extern "C" int ep_create(const ep_config* cfg, ep_ctx** out) {
     if (const char* e = getenv("EP_GATHER_CTAS")) { const long v = atol(e); if (v >= 0 && v <= 65536) c->gather_ctas = (uint32_t)v; }
     if (const char* e = getenv("EP_QUEUE_CTAS")) { const long v = atol(e); if (v == 4 || v == 5) c->queue_ctas = (uint32_t)v; }
     if (const char* e = getenv("EP_RED_CTAS")) { const long v = atol(e); if (v >= 0 && v <= 65536) c->red_ctas = (uint32_t)v; }
+    if (const char* e = getenv("EP_RED_SPLIT")) { const long v = atol(e); if (v == 1 || v == 2 || v == 4) c->red_split = (uint32_t)v; }
     if (const char* e = getenv("EP_GATHER_WARPS")) { const long v = atol(e); if (v >= 1 && v <= 8) c->gather_warps = (uint32_t)v; }
     if (const char* e = getenv("EP_GATHER_SPLIT")) { const long v = atol(e); if (v == 1 || v == 2 || v == 4) c->gather_split = (uint32_t)v; }
     if (const char* e = getenv("EP_SAMPLE_WARPS")) { const long v = atol(e); if (v >= 1 && v <= 8) c->sample_warps = (uint32_t)v; }
     // a launch shape set by hand is used as given: no tuning
-    for (const char* k : {"EP_FUSED_MODE", "EP_REDUCE_CHUNK", "EP_GATHER_CTAS", "EP_GATHER_SPLIT", "EP_QUEUE_CTAS", "EP_RED_CTAS", "EP_GATHER_WARPS", "EP_RING_PW",
+    for (const char* k : {"EP_FUSED_MODE", "EP_REDUCE_CHUNK", "EP_GATHER_CTAS", "EP_GATHER_SPLIT", "EP_RED_SPLIT", "EP_QUEUE_CTAS", "EP_RED_CTAS", "EP_GATHER_WARPS", "EP_RING_PW",
                           "EP_RING_CW", "EP_RING_SLOTS"})
         if (getenv(k)) c->cfg.autotune = 0;
     if (const char* ch = getenv("EP_REDUCE_CHUNK")) {   // reducer items per warp (tuning)
@@ -569,18 +574,22 @@ __global__ void k_bound_hist(const uint32_t* __restrict__ b, uint32_t n, uint32_
     }
 }
 
+constexpr uint32_t BOUND_BINS = 65536;
+constexpr size_t BOUND_SCRATCH = (size_t)BOUND_BINS * 12 + 16;   // sums, counts, largest bound, *typical of k_node_bound
+
 static int top_sum_bound(ep_ctx* c, uint32_t n, uint32_t top, uint64_t* out) {
-    constexpr uint32_t BINS = 65536;
-    if (!c->check.ensure((size_t)BINS * 12 + 16)) return c->fail(EP_ERR_OOM, "scratch allocation failed");
+    constexpr uint32_t BINS = BOUND_BINS;
     unsigned long long* sum = c->check.as<unsigned long long>();
     uint32_t* cnt = (uint32_t*)(sum + BINS);
     uint32_t* dmx = cnt + BINS;
     const uint32_t* b = c->bound.as<uint32_t>();
-    CK(cudaMemsetAsync(c->check.p, 0, (size_t)BINS * 12 + 16, c->stream), "bounds");
     k_bound_max<<<152 * 4, 256, 0, c->stream>>>(b, n, dmx);
-    uint32_t mx = 0;
-    CK(cudaMemcpyAsync(&mx, dmx, 4, cudaMemcpyDeviceToHost, c->stream), "bounds");
+    struct { uint32_t mx, pad; unsigned long long typical; } h = {};
+    CK(cudaMemcpyAsync(&h, dmx, 16, cudaMemcpyDeviceToHost, c->stream), "bounds");
     CK(cudaStreamSynchronize(c->stream), "bounds");
+    const uint32_t mx = h.mx;
+    // a typical batch: the nodes' mean, and the negatives at the mean feature count
+    c->train_items = (uint64_t)((double)top / n * ((double)h.typical + (double)c->R * (double)c->n_fids));
     uint32_t bits = 0;
     while (bits < 32 && (mx >> bits)) ++bits;
     const uint32_t shift = bits > 16 ? bits - 16 : 0;
@@ -626,9 +635,12 @@ static int prepare_train(ep_ctx* c) {
     if (c->cfg.loss == EP_LOSS_PPR) K = c->R;     // one slot per walk
     // item bound: sum of the B largest per-anchor bounds
     if (!c->bound.ensure((size_t)n * 4)) return c->fail(EP_ERR_OOM, "bound allocation failed");
+    if (!c->check.ensure(BOUND_SCRATCH)) return c->fail(EP_ERR_OOM, "scratch allocation failed");
+    CK(cudaMemsetAsync(c->check.p, 0, BOUND_SCRATCH, c->stream), "bounds");
     launch_node_bound(c->row.as<uint64_t>(), c->cols.as<uint32_t>(), c->fptr.as<uint64_t>(), n, c->cfg.max_nodes_kind,
                       (uint32_t)c->cfg.max_nodes, c->R, c->max_feat, c->cfg.loss == EP_LOSS_PPR,
-                      c->bound.as<uint32_t>(), c->stream);
+                      c->bound.as<uint32_t>(),
+                      (unsigned long long*)(c->check.as<char>() + (size_t)BOUND_BINS * 12 + 8), c->stream);
     uint64_t items = 0;
     int rcb = top_sum_bound(c, n, std::min<uint32_t>(B, n), &items);
     if (rcb) return rcb;
@@ -780,6 +792,8 @@ static ReduceParams reduce_params(ep_ctx* c, BatchState* st, int out_mode, void*
     rp.ring_slots = c->ring_slots;
     rp.queue_ctas_per_sm = c->queue_ctas;
     rp.red_ctas = c->red_ctas;
+    rp.red_split = c->red_split;
+    rp.typ_items = c->typ_items;
     return rp;
 }
 
@@ -886,6 +900,7 @@ static void issue_train_batch(ep_ctx* c, cudaEvent_t* ev = nullptr, bool fork = 
     }
     const bool plain = c->cfg.form == EP_FORM_PLAIN_FP32 || c->fused_mode == 1;
     if (plain) cudaMemsetAsync(c->n_touched.p, 0, 4, s);
+    c->typ_items = c->train_items;
     ReduceParams rp = reduce_params(c, st, plain ? OUT_DENSE : fused_out_mode(c), c->table.p);
     launch_reduce(c->tt, (int)c->vpl, rp, c->items_cap, s);
     if (ev) cudaEventRecord(ev[EP_STAGE_REDUCE], s);
@@ -1354,6 +1369,7 @@ static int stage_samples(ep_ctx* c, const ep_batch_samples* sm, uint32_t es, cud
     for (uint64_t j = 0; j < (uint64_t)B * c->R; ++j)
         if (sm->negatives[j] >= c->n_nodes) return c->fail(EP_ERR_INVALID_ARG, "negative id out of range");
     const uint64_t items = (uint64_t)B * c->max_feat * (1ull + c->R + K);
+    c->typ_items = (uint64_t)((double)c->n_fids / (double)c->n_nodes * ((double)B * (1. + c->R) + nn));
     int rc = ensure_bufs(c, B, K, items, es, true);
     if (rc) return rc;
     const uint32_t Ks = c->buf_K;

@@ -1783,24 +1783,40 @@ __global__ void k_table_out4(const T* __restrict__ dev, float4* __restrict__ out
 // k_split: train / validation ids as the first n_train / remaining positions
 //   of a seeded permutation of all nodes (mod.rs:118-122).
 // ---------------------------------------------------------------------------
+// *typical adds up, over all nodes, the items an anchor's positive part is
+// expected to emit under uniform sampling (features of its sampled neighbours,
+// and its own); the launch shapes are chosen by it.
 __global__ void k_node_bound(const uint64_t* row_ptr, const uint32_t* cols, const uint64_t* fptr, uint32_t n,
-                             int nodes_kind, uint32_t K, uint32_t R, uint32_t max_feat, int ppr, uint32_t* bound) {
+                             int nodes_kind, uint32_t K, uint32_t R, uint32_t max_feat, int ppr, uint32_t* bound,
+                             unsigned long long* typical) {
     const uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= n) return;
-    const uint64_t rs = row_ptr[v], re = row_ptr[v + 1];
-    const uint64_t deg = re - rs;
-    uint64_t nb = 0;
-    if (ppr) {
-        nb = (uint64_t)R * max_feat;          // R walk end nodes
-    } else if (nodes_kind == S_FIXED && deg > K) {
-        uint64_t mx = 0;
-        for (uint64_t j = rs; j < re; ++j) { const uint32_t u = cols[j]; mx = max(mx, fptr[u + 1] - fptr[u]); }
-        nb = (uint64_t)K * mx;
-    } else {
-        for (uint64_t j = rs; j < re; ++j) { const uint32_t u = cols[j]; nb += fptr[u + 1] - fptr[u]; }
+    unsigned long long typ = 0;
+    if (v < n) {
+        const uint64_t rs = row_ptr[v], re = row_ptr[v + 1];
+        const uint64_t deg = re - rs;
+        uint64_t nb = 0, sum = 0, mx = 0;
+        for (uint64_t j = rs; j < re && !ppr; ++j) {
+            const uint32_t u = cols[j];
+            const uint64_t fn = fptr[u + 1] - fptr[u];
+            sum += fn;
+            mx = max(mx, fn);
+        }
+        typ = fptr[v + 1] - fptr[v];
+        if (ppr) {
+            nb = (uint64_t)R * max_feat;          // R walk end nodes
+            typ += nb / 2;
+        } else if (nodes_kind == S_FIXED && deg > K) {
+            nb = (uint64_t)K * mx;
+            typ += sum * K / deg;
+        } else {
+            nb = sum;
+            typ += sum;
+        }
+        const uint64_t b = (fptr[v + 1] - fptr[v]) + (uint64_t)R * max_feat + nb;
+        bound[v] = (uint32_t)min(b, (uint64_t)0xffffffffu);
     }
-    const uint64_t b = (fptr[v + 1] - fptr[v]) + (uint64_t)R * max_feat + nb;
-    bound[v] = (uint32_t)min(b, (uint64_t)0xffffffffu);
+    typ = warp_sum<unsigned long long>(typ);
+    if ((threadIdx.x & 31) == 0 && typ) atomicAdd(typical, typ);
 }
 
 __global__ void k_split(uint32_t* train, uint32_t n_train, uint32_t* valid, uint32_t n, uint64_t seed,
@@ -1817,8 +1833,8 @@ __global__ void k_split(uint32_t* train, uint32_t n_train, uint32_t* valid, uint
 
 void launch_node_bound(const uint64_t* row_ptr, const uint32_t* cols, const uint64_t* fptr, uint32_t n,
                        int nodes_kind, uint32_t K, uint32_t R, uint32_t max_feat, int ppr, uint32_t* bound,
-                       cudaStream_t s) {
-    k_node_bound<<<(n + 255) / 256, 256, 0, s>>>(row_ptr, cols, fptr, n, nodes_kind, K, R, max_feat, ppr, bound);
+                       unsigned long long* typical, cudaStream_t s) {
+    k_node_bound<<<(n + 255) / 256, 256, 0, s>>>(row_ptr, cols, fptr, n, nodes_kind, K, R, max_feat, ppr, bound, typical);
 }
 
 void launch_split(uint32_t* train, uint32_t n_train, uint32_t* valid, uint32_t n, uint64_t seed, uint32_t half,

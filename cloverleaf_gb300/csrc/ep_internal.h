@@ -208,6 +208,9 @@ struct ReduceParams {
     // 0: one warp per chunk (static stride); else a persistent grid of this
     // many CTAs whose warps take chunks from BatchState::red_next
     uint32_t red_ctas;
+    // warps per chunk (1, 2, 4; 0 = by the batch's chunk count)
+    uint32_t red_split;
+    uint64_t typ_items;     // items a batch is expected to emit (launch shape only)
 };
 
 // ---- launchers (defined in the kernel translation units) -----------------
@@ -247,7 +250,7 @@ void launch_convert_table(int tt_dst, void* dst, const float* src, uint64_t n_fe
                           uint32_t dims, uint32_t dpad, int to_device_layout, cudaStream_t s);
 void launch_node_bound(const uint64_t* row_ptr, const uint32_t* cols, const uint64_t* fptr, uint32_t n,
                        int nodes_kind, uint32_t K, uint32_t R, uint32_t max_feat, int ppr, uint32_t* bound,
-                       cudaStream_t s);
+                       unsigned long long* typical, cudaStream_t s);
 void launch_split(uint32_t* train, uint32_t n_train, uint32_t* valid, uint32_t n, uint64_t seed,
                   uint32_t half, uint32_t* err, cudaStream_t s);
 void launch_pack_rows(size_t es, const void* dense, const uint32_t* rows, const uint32_t* n_rows,

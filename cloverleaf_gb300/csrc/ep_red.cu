@@ -38,10 +38,13 @@ constexpr uint32_t NONE = 0xffffffffu;
 // (its partial sum is in carry_head); THROUGH = that feature also continues
 // past the chunk; OWNER = the chunk's last feature starts here and continues
 // (partial in carry_tail); *_KEPT = the partial contains at least one kept item.
-enum : uint32_t { CF_HEAD = 1u, CF_THROUGH = 2u, CF_OWNER = 4u, CF_HEAD_KEPT = 8u, CF_TAIL_KEPT = 16u };
+// The chunk's first feature sets the low half of the word, its last the high
+// half, so that two warps of a split chunk can store them apart.
+enum : uint32_t { CF_HEAD = 1u, CF_THROUGH = 2u, CF_HEAD_KEPT = 8u, CF_OWNER = 4u << 16, CF_TAIL_KEPT = 16u << 16 };
 constexpr int RED_THREADS = 256;
 constexpr int FIX_THREADS = 128;
 constexpr uint32_t RED_MAX_CTAS = 152 * 8;
+constexpr uint32_t RED_SPLIT_CHUNKS = 3648;   // batches of up to this many chunks take several warps per chunk
 
 uint32_t reduce_chunks(uint64_t cap, uint32_t chunk) { return (uint32_t)((cap + chunk - 1) / chunk); }
 
@@ -619,10 +622,31 @@ __device__ __forceinline__ bool span_is_long(const ReduceParams& p, uint32_t c, 
     return probe < M && p.skey[probe] == f;
 }
 
-template <typename T, typename A, int VPL, int MODE>
-__device__ __forceinline__ void reduce_body(const ReduceParams& p);
+// Warps per chunk.  A chunk's features are independent sums, so its warps
+// take consecutive ranges of features, each feature still summed by one warp
+// in item order.  Small batches leave the chip idle at a warp per chunk, and
+// their time is one chunk's chain: reduce stage in us at 1 / 2 / 4 warps, 29
+// chunks (100 FP32) 24.3 / 18.7 / 15.1; 531 (100 BF16, queued Adam) 55.6 /
+// 33.8 / 23.8; 1,270 (128 FP32) 43.6 / 28.8 / 27.0.  From about 3,600 chunks
+// on, two warps gain nothing (6,500 chunks: 135.2 / 135.1).
+__device__ __forceinline__ uint32_t chunk_split(const ReduceParams& p) {
+    const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
+    const uint32_t nchunks = (p.st->n_items + p.chunk - 1) / p.chunk;
+    uint32_t w = p.red_split;
+    if (!w) w = nchunks <= 1824u ? 4u : (nchunks <= RED_SPLIT_CHUNKS ? 2u : 1u);
+    while (w > 1 && nchunks * w > warps) w >>= 1;
+    return w;
+}
 
-// k_reduce: one warp per chunk of C sorted items, in windows of RW items.
+template <typename T, typename A, int VPL, int MODE, bool SPLIT>
+__device__ __forceinline__ void reduce_body(const ReduceParams& p, uint32_t split);
+
+// k_reduce: one warp (or, in small batches, two or four) per chunk of C sorted
+// items, in windows of RW items.  Chunks are taken from the end of the sorted
+// order: the rare features, whose chunks hold many finished rows (a chunk of
+// 128 features takes several times as long as one inside a hot feature), come
+// last there when ids are given in the order features are met, and would be
+// the grid's tail.
 // Phase 1 takes the window 32 items (one per lane) at a time: the
 // first-occurrence rule is evaluated for all 32 at once with ballots (group
 // starts: new feature or new anchor; valid roles; for every item the first
@@ -638,7 +662,21 @@ template <typename T, typename A, int VPL, int MODE>
 __global__ void __launch_bounds__(MODE == OUT_RING ? RING_MAX_WARPS * 32 : (MODE == OUT_QUEUE ? QUEUE_THREADS : RED_THREADS),
                                   MODE == OUT_RING ? 1 : (VPL >= 16 ? 1 : (MODE == OUT_DENSE ? 3 : (MODE == OUT_QUEUE ? 4 : 2))))
     k_reduce(ReduceParams p) {
-    reduce_body<T, A, VPL, MODE>(p);
+    pdl_wait();
+    pdl_trigger();
+    reduce_body<T, A, VPL, MODE, false>(p, 1);
+}
+
+// The same for batches of few chunks: a chunk's warps counted by chunk_split.
+// A kernel of its own, since the split's bookkeeping costs the large batches
+// registers (256 FP32: 84 us a batch without it, 95 with it).
+template <typename T, typename A, int VPL, int MODE>
+__global__ void __launch_bounds__(MODE == OUT_QUEUE ? QUEUE_THREADS : RED_THREADS,
+                                  VPL >= 16 ? 1 : (MODE == OUT_QUEUE ? 4 : (VPL <= 4 ? 3 : 2)))
+    k_reduce_split(ReduceParams p) {
+    pdl_wait();
+    pdl_trigger();
+    reduce_body<T, A, VPL, MODE, true>(p, chunk_split(p));
 }
 
 // The per-warp queue reducer at five CTAs per SM instead of four: registers
@@ -646,13 +684,13 @@ __global__ void __launch_bounds__(MODE == OUT_RING ? RING_MAX_WARPS * 32 : (MODE
 // warps.  Same arithmetic in the same order.
 template <typename T, typename A, int VPL>
 __global__ void __launch_bounds__(QUEUE_THREADS, 5) k_reduce_q5(ReduceParams p) {
-    reduce_body<T, A, VPL, OUT_QUEUE>(p);
-}
-
-template <typename T, typename A, int VPL, int MODE>
-__device__ __forceinline__ void reduce_body(const ReduceParams& p) {
     pdl_wait();
     pdl_trigger();
+    reduce_body<T, A, VPL, OUT_QUEUE, false>(p, 1);
+}
+
+template <typename T, typename A, int VPL, int MODE, bool SPLIT>
+__device__ __forceinline__ void reduce_body(const ReduceParams& p, uint32_t split) {
     using D = typename DirOf<T, A>::type;
     using IO = RowIO<D, VPL>;
     // rows in flight: about 24-32 registers of raw data in the rows-only mode,
@@ -707,11 +745,15 @@ __device__ __forceinline__ void reduce_body(const ReduceParams& p) {
     }
     const unsigned lt_mask = (1u << lane) - 1u;
     // OUT_RING: warps [0, ring_pw) reduce, the others run Adam
-    const uint32_t gw = MODE == OUT_RING ? blockIdx.x * p.ring_pw + warp : (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const uint32_t nw = MODE == OUT_RING ? gridDim.x * p.ring_pw : (gridDim.x * blockDim.x) >> 5;
     const uint32_t M = p.st->n_items;
     const uint32_t C = p.chunk;
     const uint32_t nchunks = (M + C - 1) / C;
+    // warps per chunk (a power of two; consecutive warps of a CTA) and this
+    // warp's place among them
+    const uint32_t all_warps = MODE == OUT_RING ? gridDim.x * p.ring_pw : (gridDim.x * blockDim.x) >> 5;
+    const uint32_t gwarp = MODE == OUT_RING ? blockIdx.x * p.ring_pw + warp : (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const uint32_t gw = SPLIT ? gwarp / split : gwarp, part = SPLIT ? gwarp % split : 0u;
+    const uint32_t nw = SPLIT ? all_warps / split : all_warps;
     const uint32_t NR = p.NR;
     const bool lane_on = (uint32_t)(lane * VPL) < p.dpad;
     // lanes past the row (dims < 32 x VPL) read its last slice and accumulate
@@ -739,7 +781,8 @@ __device__ __forceinline__ void reduce_body(const ReduceParams& p) {
         if (lane == 0) t = atomicAdd(&p.st->red_next, 1u);
         return __shfl_sync(FULL, t, 0);
     };
-    for (uint32_t c = take ? next_chunk() : gw; c < nchunks; c = take ? next_chunk() : c + nw) {
+    for (uint32_t t = take ? next_chunk() : gw; t < nchunks; t = take ? next_chunk() : t + nw) {
+        const uint32_t c = nchunks - 1 - t;
         const uint32_t i0 = c * C, i1 = min(i0 + C, M);
         uint32_t cur_f = p.skey[i0];
         const bool head_partial = i0 > 0 && p.skey[i0 - 1] == cur_f;
@@ -778,6 +821,7 @@ __device__ __forceinline__ void reduce_body(const ReduceParams& p) {
         for (int k = 0; k < VPL; ++k) acc[k] = 0;
         bool started_here = !head_partial;
         bool any_kept = false;
+        bool tail = true;                 // this warp ends with the chunk's last feature
         uint32_t flags = 0;
         if constexpr (MODE == OUT_ADAM) prefetch_segment_state<T>(p, i0, i1, lane);
 
@@ -862,7 +906,7 @@ __device__ __forceinline__ void reduce_body(const ReduceParams& p) {
                 if (lane == 0) { pf = prev_f; pa = prev_anchor; ps = prev_src; }
                 const bool seg_start = act && f != pf;
                 const bool grp_start = act && (seg_start || anchor != pa);
-                if (act) g_cnt += (seg_start || s != ps);
+                if (act && part == 0) g_cnt += (seg_start || s != ps);
                 const unsigned GS = __ballot_sync(FULL, grp_start);
                 const unsigned V = __ballot_sync(FULL, act && v);
                 bool keep;
@@ -907,17 +951,49 @@ __device__ __forceinline__ void reduce_body(const ReduceParams& p) {
             }
             __syncwarp();
             // phase 2: the kept items in order, NF direction rows in flight;
-            // features close where the next one's first kept item comes
-            uint32_t j = 0;
-            uint32_t next_b = ns ? segs[0].y : 0xffffffffu;
-            for (uint32_t k = 0; k < nk; k += NF) {
+            // features close where the next one's first kept item comes.  A
+            // split chunk (one window): this warp's features are the open one
+            // (part 0) and segments [j, je), cut where items plus the weight
+            // of a finished row pass part / split of the whole.
+            uint32_t j = 0, k = 0;
+            uint32_t je = ns, kend = nk;
+            if constexpr (SPLIT) {
+                constexpr uint32_t ROW = MODE == OUT_DENSE ? 2u : 6u;   // a finished row's work in items
+                const uint32_t all = nk + ROW * ns;
+                auto cut = [&](uint32_t w) {
+                    uint32_t n = 0;
+                    for (uint32_t b = 0; b < ns; b += 32) {
+                        const uint32_t i = b + lane;
+                        n += (uint32_t)__popc(__ballot_sync(FULL, i < ns && (segs[i].y + ROW * i) * split < w * all));
+                    }
+                    return n;
+                };
+                if (part) j = cut(part);
+                if (part + 1 < split) je = cut(part + 1);
+                if (je < ns) kend = segs[je].y;
+                tail = je == ns;
+                if (part) {
+                    if (j >= je) {          // no feature starts in this part
+                        tail = false;
+                        kend = 0;
+                        je = 0;
+                    } else {
+                        cur_f = segs[j].x;
+                        k = segs[j].y;
+                        started_here = true;
+                        ++j;
+                    }
+                }
+            }
+            uint32_t next_b = j < je ? segs[j].y : 0xffffffffu;
+            for (; k < kend; k += NF) {
                 uint32_t src[NF];
                 A wv[NF];
 #pragma unroll
                 for (int u = 0; u < NF; ++u) {
                     src[u] = 0;
                     wv[u] = 0;
-                    if (k + u < nk) {
+                    if (k + u < kend) {
                         const RedEntry<A> e = ents[k + u];
                         src[u] = e.src;
                         wv[u] = e.w;
@@ -926,8 +1002,8 @@ __device__ __forceinline__ void reduce_body(const ReduceParams& p) {
                 typename IO::Raw r[NF];
 #pragma unroll
                 for (int u = 0; u < NF; ++u)
-                    if (k + u < nk) r[u] = IO::load_raw(dir + (uint64_t)src[u] * p.dpad, lane_ld);
-                if (k + NF <= nk && k + NF <= next_b) {   // no feature starts among these NF
+                    if (k + u < kend) r[u] = IO::load_raw(dir + (uint64_t)src[u] * p.dpad, lane_ld);
+                if (k + NF <= kend && k + NF <= next_b) {   // no feature starts among these NF
 #pragma unroll
                     for (int u = 0; u < NF; ++u) IO::template fma<A>(acc, wv[u], r[u]);
                     any_kept = true;
@@ -935,11 +1011,11 @@ __device__ __forceinline__ void reduce_body(const ReduceParams& p) {
                 }
 #pragma unroll
                 for (int u = 0; u < NF; ++u) {
-                    if (k + u < nk) {
+                    if (k + u < kend) {
                         while (k + u >= next_b) {
                             close_open(segs[j].x);
                             ++j;
-                            next_b = j < ns ? segs[j].y : 0xffffffffu;
+                            next_b = j < je ? segs[j].y : 0xffffffffu;
                         }
                         IO::template fma<A>(acc, wv[u], r[u]);
                         any_kept = true;
@@ -947,28 +1023,39 @@ __device__ __forceinline__ void reduce_body(const ReduceParams& p) {
                 }
             }
             // features of the window with no kept item after their start
-            for (; j < ns; ++j) close_open(segs[j].x);
+            for (; j < je; ++j) close_open(segs[j].x);
+            if (SPLIT && !tail && (part == 0 || je)) close_open(NONE);     // the next part's feature follows
             __syncwarp();
         }
-        const bool cont = i1 < M && p.skey[i1] == cur_f;
-        if (started_here && !cont) {
-            if (any_kept) {
-                finish_row<T, A, VPL, MODE>(p, cur_f, acc, lane, lane_on, as, fin, n_fin, &q, rh, ring_slots);
-                ++u_cnt;
-            }
-        } else if (!started_here) {
-            if (lane_on) store_row<A, VPL, A>((A*)p.carry_head + (uint64_t)c * p.dpad, lane, acc);
-            flags |= CF_HEAD | (cont ? CF_THROUGH : 0u) | (any_kept ? CF_HEAD_KEPT : 0u);
-        } else {
-            if (lane_on) store_row<A, VPL, A>((A*)p.carry_tail + (uint64_t)c * p.dpad, lane, acc);
-            if (lane == 0) p.carry_f[c] = cur_f;
-            flags |= CF_OWNER | (any_kept ? CF_TAIL_KEPT : 0u);
-            if (lane == 0 && span_is_long(p, c, cur_f, M, C)) {
-                const uint32_t par = as.step & 1u;
-                p.long_list[(size_t)par * p.long_cap + atomicAdd(&p.st->n_long[par], 1u)] = c;
+        if (tail) {
+            const bool cont = i1 < M && p.skey[i1] == cur_f;
+            if (started_here && !cont) {
+                if (any_kept) {
+                    finish_row<T, A, VPL, MODE>(p, cur_f, acc, lane, lane_on, as, fin, n_fin, &q, rh, ring_slots);
+                    ++u_cnt;
+                }
+            } else if (!started_here) {
+                if (lane_on) store_row<A, VPL, A>((A*)p.carry_head + (uint64_t)c * p.dpad, lane, acc);
+                flags |= CF_HEAD | (cont ? CF_THROUGH : 0u) | (any_kept ? CF_HEAD_KEPT : 0u);
+            } else {
+                if (lane_on) store_row<A, VPL, A>((A*)p.carry_tail + (uint64_t)c * p.dpad, lane, acc);
+                if (lane == 0) p.carry_f[c] = cur_f;
+                flags |= CF_OWNER | (any_kept ? CF_TAIL_KEPT : 0u);
+                if (lane == 0 && span_is_long(p, c, cur_f, M, C)) {
+                    const uint32_t par = as.step & 1u;
+                    p.long_list[(size_t)par * p.long_cap + atomicAdd(&p.st->n_long[par], 1u)] = c;
+                }
             }
         }
-        if (lane == 0) p.carry_flags[c] = flags;
+        if (lane == 0) {
+            if constexpr (SPLIT) {
+                uint16_t* half = reinterpret_cast<uint16_t*>(p.carry_flags + c);
+                if (part == 0) half[0] = (uint16_t)flags;
+                if (tail) half[1] = (uint16_t)(flags >> 16);
+            } else {
+                p.carry_flags[c] = flags;
+            }
+        }
     }
     if constexpr (MODE == OUT_DENSE) fin_flush(p, fin, n_fin, lane);
     if constexpr (MODE == OUT_QUEUE) queue_flush<T, VPL>(p, q, lane, lane_on, as);
@@ -1260,6 +1347,18 @@ static void red_launch(const ReduceParams& p, uint64_t cap, cudaStream_t s, int 
     const uint32_t nch = reduce_chunks(cap, p.chunk);
     const uint32_t warps = nch ? nch : 1;
     if (which == 0) {
+        // few chunks expected: several warps each, with room for four
+        const bool split = p.red_split > 1 || (!p.red_split && reduce_chunks(p.typ_items, p.chunk) <= RED_SPLIT_CHUNKS);
+        if (split && !p.red_ctas && p.chunk <= RW && (p.out_mode == OUT_DENSE || p.out_mode == OUT_QUEUE)) {
+            const uint32_t w4 = (uint32_t)std::min<uint64_t>(4ull * warps, 8ull * RED_MAX_CTAS);
+            if (p.out_mode == OUT_DENSE)
+                launch_chain(k_reduce_split<T, A, VPL, OUT_DENSE>, (w4 + 7) / 8, RED_THREADS,
+                             (size_t)(RED_THREADS / 32) * list_bytes<A>(), s, p);
+            else
+                launch_chain(k_reduce_split<T, A, VPL, OUT_QUEUE>, (w4 + 3) / 4, QUEUE_THREADS, queue_smem<T, A>(p.dpad), s,
+                             p);
+            return;
+        }
         uint32_t ctas = (warps + RED_THREADS / 32 - 1) / (RED_THREADS / 32);
         if (ctas > RED_MAX_CTAS) ctas = RED_MAX_CTAS;
         if (p.red_ctas) ctas = std::min<uint32_t>(ctas, p.red_ctas);
@@ -1318,6 +1417,9 @@ static cudaError_t fixl_setup() {
         e = cudaFuncSetAttribute(k_fixup_long<T, A, VPL, OUT_ADAM>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(k_reduce<T, A, VPL, OUT_QUEUE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)queue_smem<T, A>(VPL * 32));
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_reduce_split<T, A, VPL, OUT_QUEUE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)queue_smem<T, A>(VPL * 32));
     if constexpr (VPL <= 8) {
         if (e == cudaSuccess)

@@ -378,3 +378,28 @@ def test_gather_split_gives_the_same_table(monkeypatch, max_features):
             assert ctx.train_batches(9)["kept_anchors"] > 0
             tables.append(ctx.get_table(prob["n_feat"], 52))
     assert all(np.array_equal(tables[0], t) for t in tables[1:])
+
+
+@pytest.mark.parametrize("form", [_native.FORM_FUSED_BF16, _native.FORM_PLAIN_FP32])
+@pytest.mark.parametrize("n_feat", [3, 40, 4000])
+def test_reducer_split_gives_the_same_table(monkeypatch, form, n_feat):
+    # 1, 2 or 4 warps per reducer chunk: chunks inside one hot feature (3
+    # features), of a few features, and of one feature per item; the last
+    # chunk ragged
+    from tests._cases import random_problem
+    prob = random_problem(99, n=1500, n_feat=n_feat, dims=36, deg=(1, 9), feats=(1, 5))
+    tables = []
+    for split in ("1", "2", "4"):
+        monkeypatch.setenv("EP_RED_SPLIT", split)
+        cfg = _native.default_config()
+        cfg.form, cfg.dims, cfg.negatives, cfg.loss, cfg.gamma = form, 36, 4, _native.LOSS_STARSPACE, 0.5
+        cfg.batch_size, cfg.passes, cfg.valid_pct = 150, 1, 0.0
+        ctx = _native.Context(cfg)
+        ctx.upload_graph(prob["rows"], prob["cols"], None)
+        ctx.upload_features(prob["fptr"], prob["fids"], prob["n_feat"])
+        ctx.set_table(None)
+        st = ctx.train_batches(7)
+        assert st["kept_anchors"] > 0
+        tables.append((ctx.get_table(prob["n_feat"], 36), st["unique_rows"], st["gathered_rows"]))
+    for t, u, g in tables[1:]:
+        assert np.array_equal(tables[0][0], t) and (u, g) == tables[0][1:]
