@@ -2,9 +2,9 @@
 //
 // Owns the device copies of the graph CSR, the feature CSR, the feature table
 // and Adam moments, plus per-batch scratch, and sequences the per-batch
-// kernels (see ep_internal.h) on the context's stream.  In the FUSED form one
-// batch is captured once as a CUDA graph and replayed for every batch of every
-// pass; the kernels read their batch index, step and learning rate from a
+// kernels (see ep_internal.h) on the context's stream.  With use_graphs a few
+// batches are captured once as a CUDA graph and replayed for every batch of
+// every pass; the kernels read their batch index, step and learning rate from a
 // device-resident BatchState that the last kernel of the batch advances.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -128,6 +128,7 @@ struct ep_ctx {
     cudaGraphExec_t gexec_run = nullptr;   // graph_batches consecutive batches
     std::map<uint32_t, cudaGraphExec_t> gexec_rem;   // 2 .. graph_batches - 1 consecutive batches (a run's remainder)
     uint32_t graph_batches = 16;
+    bool graph_batches_set = false;   // by the environment
     uint32_t* sorted_keys = nullptr;
     uint2* sorted_vals = nullptr;
     BatchState* h_st = nullptr;   // pinned mirror
@@ -280,7 +281,7 @@ extern "C" int ep_create(const ep_config* cfg, ep_ctx** out) {
     c->NR = c->R + 2;
     if (const char* gb = getenv("EP_GRAPH_BATCHES")) {   // batches per replayed graph (tuning)
         const long v = atol(gb);
-        if (v >= 1 && v <= 1024) c->graph_batches = (uint32_t)v;
+        if (v >= 1 && v <= 1024) { c->graph_batches = (uint32_t)v; c->graph_batches_set = true; }
     }
     if (const char* fm = getenv("EP_FUSED_MODE")) {   // (tuning)
         const int v = atoi(fm);
@@ -448,6 +449,7 @@ extern "C" int ep_set_table(ep_ctx* c, const float* init) {
     cudaSetDevice(c->device);
     const size_t es = c->tt == TT_BF16 ? 2 : 4;
     const size_t rows = (size_t)c->n_feat * c->dpad;
+    const void *was_t = c->table.p, *was_m = c->m.p, *was_v = c->v.p;
     if (!c->table.ensure(rows * es) || !c->m.ensure(rows * 4) || !c->v.ensure(rows * 4))
         return c->fail(EP_ERR_OOM, "table allocation failed (%zu rows)", (size_t)c->n_feat);
     if (init) {
@@ -460,7 +462,8 @@ extern "C" int ep_set_table(ep_ctx* c, const float* init) {
     }
     CK(cudaGetLastError(), "table init");
     c->table_ok = true;
-    c->drop_graph();
+    // captured batches hold the buffers' addresses, nothing of their contents
+    if (c->table.p != was_t || c->m.p != was_m || c->v.p != was_v) c->drop_graph();
     return reset_state(c);
 }
 
@@ -611,6 +614,21 @@ static int top_sum_bound(ep_ctx* c, uint32_t n, uint32_t top, uint64_t* out) {
     return EP_OK;
 }
 
+// Batches per replayed graph.  A batch costs about 90 us of host time to
+// record, instantiate, upload and destroy (2.7 ms for 30 batches of 20
+// kernels), and every replay about 20 us at its boundary, where a batch's
+// fix-ups are joined instead of running beside the next batch's sampling.  A
+// pass replays steps / g graphs of g batches and one of the remainder.
+static uint32_t pick_graph_batches(uint32_t steps, uint32_t passes) {
+    uint32_t best = 1;
+    double least = 1e300;
+    for (uint32_t g = 1; g <= 16 && g <= std::max<uint32_t>(steps, 1); ++g) {
+        const double cost = 90. * (g + steps % g) + 20. * ((double)steps / g) * std::max<uint32_t>(passes, 1);
+        if (cost < least) { least = cost; best = g; }
+    }
+    return best;
+}
+
 static int prepare_train(ep_ctx* c) {
     if (!c->graph_ok || !c->feats_ok) return c->fail(EP_ERR_STATE, "upload the graph and the features first");
     if (!c->table_ok) return c->fail(EP_ERR_STATE, "set the table first");
@@ -655,6 +673,7 @@ static int prepare_train(ep_ctx* c) {
     if (rc) return rc;
     c->Bcap = B;
     c->Kcap = c->buf_K;
+    if (!c->graph_batches_set) c->graph_batches = pick_graph_batches(c->steps_per_pass, c->cfg.passes);
     c->prepared = true;
     return EP_OK;
 }
@@ -845,6 +864,7 @@ static uint32_t kernels_per_batch(const ep_ctx* c, bool fork) {
 static void issue_train_batch(ep_ctx* c, cudaEvent_t* ev = nullptr, bool fork = false, bool last = true) {
     BatchState* st = c->st.as<BatchState>();
     cudaStream_t s = c->stream;
+    const bool plain = c->cfg.form == EP_FORM_PLAIN_FP32 || c->fused_mode == 1;
     launch_batch_begin(st, c->n_train, c->Bcap, c->steps_per_pass, c->total_steps, c->warmup, c->cfg.alpha, 0,
                        c->cfg.noise, noise_decay(c), s);
     SampleParams sp = sample_params(c, st, false, false);
@@ -857,6 +877,7 @@ static void issue_train_batch(ep_ctx* c, cudaEvent_t* ev = nullptr, bool fork = 
         // which run with emission off and read neither; then k_batch_end
         cudaEventRecord(c->ev_fork, s);
         cudaStreamWaitEvent(c->side, c->ev_fork, 0);
+        if (plain) cudaMemsetAsync(c->n_touched.p, 0, 4, c->side);   // the last batch's Adam kernel has read it
         launch_scan_occ(st, c->occ.as<uint32_t>(), c->Bcap, c->items_cap, c->side);
         if (c->fix_pending) {   // the previous batch's fix-ups: the table, and the sorted items they read
             cudaStreamWaitEvent(s, c->ev_fix, 0);
@@ -898,8 +919,7 @@ static void issue_train_batch(ep_ctx* c, cudaEvent_t* ev = nullptr, bool fork = 
                           c->items_cap, (int)bits_for(c->n_feat), &c->sorted_keys, &c->sorted_vals, s);
         if (ev) cudaEventRecord(ev[EP_STAGE_SORT], s);
     }
-    const bool plain = c->cfg.form == EP_FORM_PLAIN_FP32 || c->fused_mode == 1;
-    if (plain) cudaMemsetAsync(c->n_touched.p, 0, 4, s);
+    if (plain && !fork) cudaMemsetAsync(c->n_touched.p, 0, 4, s);
     c->typ_items = c->train_items;
     ReduceParams rp = reduce_params(c, st, plain ? OUT_DENSE : fused_out_mode(c), c->table.p);
     launch_reduce(c->tt, (int)c->vpl, rp, c->items_cap, s);
@@ -1117,7 +1137,7 @@ static int capture_batches(ep_ctx* c, uint32_t batches, cudaGraphExec_t* out) {
 // Builds, ahead of a run of n batches, the graphs that run will replay, so
 // that the one-time capture and instantiation stay outside its timing.
 static int prepare_graphs(ep_ctx* c, uint32_t n) {
-    if (!(c->cfg.use_graphs && c->cfg.form == EP_FORM_FUSED_BF16) || n == 0) return EP_OK;
+    if (!c->cfg.use_graphs || n == 0) return EP_OK;
     if (c->cfg.autotune && !tune_from_cache(c)) {
         std::vector<TuneChoice> s1;
         uint32_t need = 0;
@@ -1142,7 +1162,7 @@ static int launch_train_run(ep_ctx* c, uint32_t n) {
         int rc = autotune(c, n);
         if (rc) return rc;
     }
-    const bool use_graph = c->cfg.use_graphs && c->cfg.form == EP_FORM_FUSED_BF16;
+    const bool use_graph = c->cfg.use_graphs;
     const uint32_t k = c->graph_batches;
     while (n) {
         if (use_graph && k > 1 && n >= k) {
@@ -1178,7 +1198,7 @@ static int launch_train_run(ep_ctx* c, uint32_t n) {
 }
 
 static int launch_train_batch(ep_ctx* c) {
-    const bool use_graph = c->cfg.use_graphs && c->cfg.form == EP_FORM_FUSED_BF16;
+    const bool use_graph = c->cfg.use_graphs;
     if (use_graph) {
         if (!c->gexec) {
             int rc = capture_batches(c, 1, &c->gexec);

@@ -59,7 +59,8 @@ enum { EP_LW_NONE = 0, EP_LW_LOG = 1, EP_LW_EXP = 2 };
 /* Implementation form.  PLAIN_FP32: FP32 table, one kernel per stage, the
  * batch gradient materialised before a separate Adam kernel.  FUSED_BF16:
  * BF16 table (stochastic rounding) with FP32 accumulation and FP32 Adam
- * moments, gradient reduction fused with Adam, replayed as a CUDA graph. */
+ * moments, gradient reduction fused with Adam.  Both replay CUDA graphs of a
+ * few batches (use_graphs). */
 enum { EP_FORM_PLAIN_FP32 = 0, EP_FORM_FUSED_BF16 = 1 };
 /* Gradient extraction.  REFERENCE: a feature's per-anchor gradient comes from
  * the first role (h(v), ~h(v), h(u_1..R)) in which it has a finite gradient
@@ -92,7 +93,7 @@ typedef struct ep_config {
     int32_t form;                /* EP_FORM_* */
     int32_t grad_mode;           /* EP_GRAD_* */
     int32_t device;              /* CUDA device ordinal */
-    int32_t use_graphs;          /* replay each batch as a CUDA graph */
+    int32_t use_graphs;          /* replay the batches as CUDA graphs */
     int32_t autotune;            /* pick launch shapes by timing candidates on the
                                     first training batches (see ep_get_launch_shape):
                                     0 off; 1 (default) only shapes that leave results
