@@ -199,26 +199,35 @@ __device__ __forceinline__ float ares_key(const SampleParams& p, uint64_t rs, ui
     return wi > 0.f ? __logf(u) / wi : -INFINITY;
 }
 
-// r <= 32: lane t < r holds one member of the running set; 32 candidates at a
-// time enter while they beat the set's smallest key.
-__device__ void ares_small(const SampleParams& p, uint64_t rs, uint32_t deg, float sw, uint32_t r, uint32_t v,
-                           uint32_t salt, uint32_t* out, float* outw, int lane) {
-    float skey = -INFINITY;
-    uint32_t spos = 0xffffffffu;
-    if ((uint32_t)lane < r) { spos = (uint32_t)lane; skey = ares_key(p, rs, lane, deg, sw, v, salt); }
-    for (uint32_t base = r; base < deg; base += 32) {
-        const uint32_t i = base + lane;
-        float ck = i < deg ? ares_key(p, rs, i, deg, sw, v, salt) : -INFINITY;
-        for (uint32_t guard = 0; guard <= 32; ++guard) {
-            // the set's smallest key and the lane holding it
-            float mk = (uint32_t)lane < r ? skey : INFINITY;
-            int ml = lane;
+// The running set for r <= 32: lane t < r holds one member.
+struct AresSet {
+    float key, mk;      // this lane's member; the set's smallest key ...
+    uint32_t pos;
+    int ml;             // ... and the lane holding it
+
+    __device__ __forceinline__ void smallest(uint32_t r, int lane) {
+        mk = (uint32_t)lane < r ? key : INFINITY;
+        ml = lane;
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                const float ok2 = __shfl_xor_sync(FULL, mk, o);
-                const int ol = __shfl_xor_sync(FULL, ml, o);
-                if (ok2 < mk || (ok2 == mk && ol < ml)) { mk = ok2; ml = ol; }
-            }
+        for (int o = 16; o > 0; o >>= 1) {
+            const float ok2 = __shfl_xor_sync(FULL, mk, o);
+            const int ol = __shfl_xor_sync(FULL, ml, o);
+            if (ok2 < mk || (ok2 == mk && ol < ml)) { mk = ok2; ml = ol; }
+        }
+    }
+    // the first r positions
+    __device__ __forceinline__ void start(const SampleParams& p, uint64_t rs, uint32_t deg, float sw, uint32_t r,
+                                          uint32_t v, uint32_t salt, int lane) {
+        key = -INFINITY;
+        pos = 0xffffffffu;
+        if ((uint32_t)lane < r) { pos = (uint32_t)lane; key = ares_key(p, rs, lane, deg, sw, v, salt); }
+        smallest(r, lane);
+    }
+    // 32 candidates (position i, key ck of each lane): they enter while they
+    // beat the set's smallest key, best first.  The smallest key is searched
+    // again only after a member was replaced.
+    __device__ __forceinline__ void offer(float ck, uint32_t i, uint32_t r, int lane) {
+        for (uint32_t guard = 0; guard <= 32; ++guard) {
             const bool better = ck > mk;
             if (!__ballot_sync(FULL, better)) break;
             // the best candidate replaces the smallest member
@@ -231,11 +240,79 @@ __device__ void ares_small(const SampleParams& p, uint64_t rs, uint32_t deg, flo
                 if (ok2 > bk || (ok2 == bk && ol < bl)) { bk = ok2; bl = ol; }
             }
             const uint32_t bpos = __shfl_sync(FULL, i, bl);
-            if (lane == ml) { skey = bk; spos = bpos; }
+            if (lane == ml) { key = bk; pos = bpos; }
             if (lane == bl) ck = -INFINITY;
+            smallest(r, lane);
         }
     }
-    if ((uint32_t)lane < r) { out[lane] = p.cols[rs + spos]; outw[lane] = __uint_as_float(spos); }
+    __device__ __forceinline__ void finish(const SampleParams& p, uint64_t rs, uint32_t r, uint32_t* out, float* outw,
+                                           int lane) const {
+        if ((uint32_t)lane < r) { out[lane] = p.cols[rs + pos]; outw[lane] = __uint_as_float(pos); }
+    }
+};
+
+// r <= 32, one warp: the keys of four blocks of 32 candidates are computed
+// together, with their loads in flight at once.
+__device__ void ares_small(const SampleParams& p, uint64_t rs, uint32_t deg, float sw, uint32_t r, uint32_t v,
+                           uint32_t salt, uint32_t* out, float* outw, int lane) {
+    AresSet set;
+    set.start(p, rs, deg, sw, r, v, salt, lane);
+    constexpr int NB = 4;
+    for (uint32_t base = r; base < deg; base += 32 * NB) {
+        float key[NB];
+#pragma unroll
+        for (int b = 0; b < NB; ++b) {
+            const uint32_t i = base + 32 * b + lane;
+            key[b] = i < deg ? ares_key(p, rs, i, deg, sw, v, salt) : -INFINITY;
+        }
+#pragma unroll
+        for (int b = 0; b < NB; ++b) set.offer(key[b], base + 32 * b + lane, r, lane);
+    }
+    set.finish(p, rs, r, out, outw, lane);
+}
+
+// Fixed(K <= 32) anchors of more than HUB_DEG edges: the warps of the CTA
+// compute the keys together, HUB_KEYS per warp and round into shared memory,
+// and the anchor's warp offers them in position order, so that the result is
+// ares_small's.  One hub per batch otherwise sets the sampler's time: 1,000
+// anchors of a 60,000-node power-law graph with 2 hard negatives, 101 us a
+// batch at the start, 65 us with ares_small's cheaper blocks and the row scan
+// of the hard negatives, 49 us with the hubs shared (what is left is the
+// walks' chain of loads).
+constexpr uint32_t HUB_DEG = 512, HUB_KEYS = 256;
+
+struct HubAnchor {
+    uint64_t rs;
+    uint32_t v, deg;    // deg 0: none
+};
+
+__device__ void ares_hubs(const SampleParams& p, const HubAnchor* hubs, uint32_t salt, float* keys, int lane) {
+    const uint32_t w = threadIdx.x >> 5, nw = blockDim.x >> 5, r = p.cfg.K;
+    for (uint32_t h = 0; h < nw; ++h) {
+        const HubAnchor hub = hubs[h];
+        if (!hub.deg) continue;                    // uniform over the CTA
+        const float sw = (float)hub.deg / (float)r;
+        AresSet set;
+        if (w == h) set.start(p, hub.rs, hub.deg, sw, r, hub.v, salt, lane);
+        const uint32_t slab = nw * HUB_KEYS;
+        for (uint32_t base = r; base < hub.deg; base += slab) {
+#pragma unroll 4
+            for (uint32_t b = 0; b < HUB_KEYS; b += 32) {
+                const uint32_t j = w * HUB_KEYS + b + lane, i = base + j;
+                keys[j] = i < hub.deg ? ares_key(p, hub.rs, i, hub.deg, sw, hub.v, salt) : -INFINITY;
+            }
+            __syncthreads();
+            if (w == h) {
+                const uint32_t m = min(slab, hub.deg - base);
+                for (uint32_t b = 0; b < m; b += 32) set.offer(keys[b + lane], base + b + lane, r, lane);
+            }
+            __syncthreads();
+        }
+        if (w == h) {
+            const uint32_t a = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+            set.finish(p, hub.rs, r, p.nbr + (uint64_t)a * p.cfg.Kcap, p.nbr_w + (uint64_t)a * p.cfg.Kcap, lane);
+        }
+    }
 }
 
 // Order-preserving image of a float key as an unsigned integer.
@@ -313,21 +390,19 @@ constexpr uint32_t ROLE_CAP = 34;     // R + 2
 // k_sample: one warp per anchor.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) k_sample(SampleParams p) {
-    __shared__ uint32_t s_hist[8][256];   // per warp: ares_select's histogram
+    __shared__ uint32_t s_hist[8][256];   // per warp: ares_select's histogram; ares_hubs' keys
+    __shared__ HubAnchor s_hub[8];
     pdl_wait();
     pdl_trigger();
     const int lane = threadIdx.x & 31;
     const uint32_t a = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     BatchState* st = p.st;
     const uint32_t n = st->n_anchors;
-    if (a >= n) return;
     const SampleCfg& c = p.cfg;
     const uint32_t salt = p.eval ? 0xffffffffu : (uint32_t)st->step;
-    uint32_t v;
-    if (p.injected == 1) {
-        v = p.anchors[a];
-    } else {
-        if (p.injected == 2) {
+    uint32_t v = 0;
+    if (a < n) {
+        if (p.injected) {
             v = p.anchors[a];
         } else {
             const uint32_t pos = st->b0 + a;
@@ -341,7 +416,26 @@ __global__ void __launch_bounds__(256) k_sample(SampleParams p) {
             v = p.order[idx];
             if (lane == 0) p.anchors[a] = v;
         }
-
+    }
+    // hubs by the whole CTA (a condition of the launch, not of the warp)
+    bool hub = false;
+    if (p.injected != 1 && !c.ppr && c.nodes_kind == S_FIXED && c.weighted_sampling && c.weighted_avg && p.wcdf &&
+        c.K >= 1 && c.K <= 32 && c.K <= c.Kcap) {
+        if (lane == 0) {
+            HubAnchor h{0, v, 0};
+            if (a < n) {
+                h.rs = p.row_ptr[v];
+                const uint64_t deg = p.row_ptr[v + 1] - h.rs;
+                h.deg = deg > HUB_DEG ? (uint32_t)deg : 0u;
+            }
+            s_hub[threadIdx.x >> 5] = h;
+        }
+        __syncthreads();
+        hub = s_hub[threadIdx.x >> 5].deg != 0;
+        ares_hubs(p, s_hub, salt, reinterpret_cast<float*>(&s_hist[0][0]), lane);
+    }
+    if (a >= n) return;
+    if (p.injected != 1) {
         // --- neighbours (reconstruct_node_embedding, model.rs:342-386) ---
         const uint64_t rs = p.row_ptr[v];
         const uint32_t deg = (uint32_t)(p.row_ptr[v + 1] - rs);
@@ -398,7 +492,8 @@ __global__ void __launch_bounds__(256) k_sample(SampleParams p) {
             if (r == deg) {
                 take_all = 1;
             } else if (c.weighted_sampling && c.weighted_avg && p.wcdf) {
-                if (r <= 32) ares_small(p, rs, deg, sw, r, v, salt, out, outw, lane);
+                if (hub) {}                    // sampled above
+                else if (r <= 32) ares_small(p, rs, deg, sw, r, v, salt, out, outw, lane);
                 else ares_select(p, rs, deg, sw, r, v, salt, out, outw, s_hist[(threadIdx.x >> 5) & 7], lane);
                 cnt = r;
             } else if (r <= 32) {
@@ -547,17 +642,24 @@ __global__ void __launch_bounds__(256) k_sample(SampleParams p) {
                     }
                     ok = node != v;
                 }
-                // not one of the anchor's neighbours: the warp scans the row,
-                // each lane tests its own end node
-                bool hit = false;
-                for (uint64_t b = rs; b < ae; b += 32) {
-                    const uint32_t x = b + lane < ae ? p.cols[b + lane] : 0u;
-                    const uint32_t m = (uint32_t)min((uint64_t)32, ae - b);
-                    for (uint32_t s2 = 0; s2 < m; ++s2) {
-                        const uint32_t y = __shfl_sync(FULL, x, s2);   // every lane takes part
-                        hit = hit || y == node;
+                // not one of the anchor's neighbours: the lanes scan the row,
+                // 256 ids in flight, each against every walk's end node (few),
+                // marking the walks whose node they meet
+                const uint32_t nw = min(32u, walks - w0);
+                uint32_t met = 0;
+                for (uint64_t b = rs; b < ae; b += 256) {
+                    uint32_t x[8];
+#pragma unroll
+                    for (int k2 = 0; k2 < 8; ++k2) x[k2] = b + 32 * k2 + lane < ae ? p.cols[b + 32 * k2 + lane] : 0xffffffffu;
+                    for (uint32_t s2 = 0; s2 < nw; ++s2) {
+                        const uint32_t y = __shfl_sync(FULL, node, (int)s2);
+                        bool eq = false;
+#pragma unroll
+                        for (int k2 = 0; k2 < 8; ++k2) eq = eq || x[k2] == y;
+                        met |= (uint32_t)eq << s2;
                     }
                 }
+                const bool hit = (__reduce_or_sync(FULL, met) >> lane) & 1u;
                 ok = ok && !hit;
                 // keep the first occurrence among valid end nodes, in walk order
                 bool dup = false;

@@ -307,3 +307,35 @@ def test_weighted_sampling_many_neighbours(kind, val):
     freq = counts / (8 * A)
     assert np.abs(freq - want).max() < 0.06, np.abs(freq - want).max()
     assert freq[-1] > freq[0] + 0.3          # heavy neighbours far more often
+
+
+def test_weighted_sampling_of_hubs_does_not_depend_on_the_cta(monkeypatch):
+    # anchors of more than 512 edges are sampled by all warps of a CTA, in
+    # slabs of 256 keys per warp: the same neighbours, in the same slots, for
+    # CTAs of 1, 3 and 8 warps; degrees around the slabs' edges
+    rng = np.random.default_rng(12)
+    deg = np.array([5, 12, 13, 511, 512, 513, 12 + 256, 12 + 257, 12 + 768, 12 + 2048, 12 + 2049, 3000, 7001] * 3)
+    n = len(deg)
+    rows = np.zeros(n + 1, np.uint64)
+    rows[1:] = np.cumsum(deg)
+    cols = rng.integers(0, n, int(rows[-1])).astype(np.uint32)
+    cdf = _native.cdf_convert(rows, rng.uniform(1, 5, len(cols)).astype(np.float32))
+    fptr = np.arange(n + 1, dtype=np.uint64)
+    got = []
+    for warps in ("1", "3", "8"):
+        monkeypatch.setenv("EP_SAMPLE_WARPS", warps)
+        cfg = _native.default_config()
+        cfg.dims, cfg.negatives, cfg.batch_size, cfg.valid_pct = 16, 2, n, 0.0
+        cfg.max_nodes_kind, cfg.max_nodes = _native.SAMPLE_FIXED, 12.0
+        cfg.weighted_neighbor_sampling = cfg.weighted_neighbor_averaging = 1
+        ctx = _native.Context(cfg)
+        ctx.upload_graph(rows, cols, cdf)
+        ctx.upload_features(fptr, np.arange(n, dtype=np.uint32), n)
+        ctx.set_table(None)
+        cnt, nbr, w, _ = ctx.sample(np.arange(n, dtype=np.uint32), 3, 12)
+        assert np.array_equal(cnt, np.minimum(deg, 12))
+        for v in range(n):
+            assert np.isin(nbr[v, :cnt[v]], cols[int(rows[v]):int(rows[v + 1])]).all()
+        got.append((nbr, w))
+    for nbr, w in got[1:]:
+        assert np.array_equal(got[0][0], nbr) and np.array_equal(got[0][1], w)
