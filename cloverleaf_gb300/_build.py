@@ -28,7 +28,7 @@ DATAGEN_SOURCES = ("ep_datagen.cpp",)
 
 CU_SOURCES = ("ep_fwd.cu", "ep_sort.cu", "ep_red.cu", "ep_ctx.cu", "ep_knn.cu")
 CPP_SOURCES = ("ep_host.cpp",)
-HEADERS = ("ep_internal.h", "ep_device.cuh", "ep_launch.cuh")
+HEADERS = ("ep_internal.h", "ep_device.cuh", "ep_launch.cuh", "ep_hostmem.h")
 
 ARCH = "-gencode=arch=compute_103a,code=sm_103a"
 NVCC_FLAGS = ["-O3", "-std=c++17", ARCH, "-lineinfo", "-Xcompiler", "-fPIC", "-I" + INCLUDE]

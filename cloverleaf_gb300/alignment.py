@@ -28,9 +28,11 @@ class NeighborhoodAligner:
         n = graph.nodes()
         if embeddings.len() < n:
             raise ValueError(f"embeddings hold {embeddings.len()} rows for a graph of {n} nodes")
+        rows = _native.align(graph.rows, graph.cols, graph.weights, embeddings.table[:n], self.alpha, self.max_neighbors)
+        if embeddings.len() == n:
+            return rows
         out = np.zeros_like(embeddings.table)    # rows past the graph's nodes stay zero (lib.rs:3119-3124)
-        out[:n] = _native.align(graph.rows, graph.cols, graph.weights, embeddings.table[:n], self.alpha,
-                                self.max_neighbors)
+        out[:n] = rows
         return out
 
     def align(self, embeddings: NodeEmbeddings, graph: Graph) -> NodeEmbeddings:

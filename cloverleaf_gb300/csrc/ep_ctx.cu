@@ -21,6 +21,7 @@
 #include <vector>
 
 #include "../../include/ep_gb300.h"
+#include "ep_hostmem.h"
 #include "ep_internal.h"
 
 using namespace ep;
@@ -474,7 +475,8 @@ extern "C" int ep_get_table(ep_ctx* c, float* out) {
     // page-locked caller memory: the kernel writes the FP32 rows into it
     // directly (no staging buffer to allocate, no separate copy)
     cudaPointerAttributes pa{};
-    if (cudaPointerGetAttributes(&pa, out) == cudaSuccess && pa.type == cudaMemoryTypeHost && pa.devicePointer &&
+    const bool known = cudaPointerGetAttributes(&pa, out) == cudaSuccess;
+    if (known && pa.type == cudaMemoryTypeHost && pa.devicePointer &&
         launch_table_out(c->tt, c->table.p, static_cast<float*>(pa.devicePointer), c->n_feat, c->dims, c->dpad,
                          c->stream)) {
         CK(cudaGetLastError(), "table download");
@@ -483,10 +485,17 @@ extern "C" int ep_get_table(ep_ctx* c, float* out) {
     }
     cudaGetLastError();   // pageable memory: the attribute query may leave an error behind
     const size_t dense = (size_t)c->n_feat * c->dims * 4;
+    // the array's pages are made resident while the rows are converted (not
+    // those of device memory: the copy to it fails)
+    ResultPages pages(out, known && pa.type == cudaMemoryTypeDevice ? 0 : dense);
     if (!c->xfer.ensure(dense)) return c->fail(EP_ERR_OOM, "staging allocation failed");
     launch_convert_table(c->tt, c->table.p, c->xfer.as<float>(), c->n_feat, c->dims, c->dpad, 0, c->stream);
     CK(cudaGetLastError(), "table download");
-    CK(cudaMemcpyAsync(out, c->xfer.p, dense, cudaMemcpyDeviceToHost, c->stream), "download table");
+    for (size_t at = 0; at < dense; at += ResultPages::SLAB) {
+        pages.wait(at / ResultPages::SLAB);
+        CK(cudaMemcpyAsync((char*)out + at, c->xfer.as<char>() + at, std::min(dense - at, ResultPages::SLAB),
+                           cudaMemcpyDeviceToHost, c->stream), "download table");
+    }
     CK(cudaStreamSynchronize(c->stream), "download table");
     return EP_OK;
 }

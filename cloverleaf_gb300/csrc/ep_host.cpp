@@ -22,7 +22,10 @@
 #include <omp.h>
 #endif
 
+#include <unistd.h>
+
 #include "../../include/ep_gb300.h"
+#include "ep_hostmem.h"
 
 // ---------------------------------------------------------------------------
 // graph.rs restatement on the boundary
@@ -603,3 +606,84 @@ extern "C" int64_t ep_format_edges(const ep_vocab* v, const char* anon_type, uin
     for (const auto& x : part) { memcpy(out + o, x.data(), x.size()); o += x.size(); }
     return (int64_t)total;
 }
+
+// ---------------------------------------------------------------------------
+// Host memory (ep_hostmem.h)
+// ---------------------------------------------------------------------------
+namespace ep {
+
+namespace {
+constexpr size_t PAGE_PIECE = 1u << 20;      // bytes a thread takes at a time (divides a slab)
+constexpr size_t SMALL_PIECE = 1u << 16;
+}
+
+ResultPages::ResultPages(void* p, size_t bytes)
+    : p_(static_cast<char*>(p)), bytes_(bytes), page_((size_t)sysconf(_SC_PAGESIZE)) {
+    pieces_ = (bytes + PAGE_PIECE - 1) / PAGE_PIECE;
+    if (bytes < THREADED) {
+        later_ = true;
+        return;
+    }
+    const unsigned cores = std::max(1u, std::thread::hardware_concurrency());
+    const size_t want = std::min<size_t>({8, cores, pieces_});
+    try {
+        left_.reset(new std::atomic<uint32_t>[slabs()]);
+        for (size_t i = 0; i < slabs(); ++i)
+            left_[i] = (uint32_t)std::min(SLAB / PAGE_PIECE, pieces_ - i * (SLAB / PAGE_PIECE));
+        threads_.reserve(want);
+        for (size_t t = 0; t < want; ++t) threads_.emplace_back([this] { work(); });
+    } catch (...) {
+        // fewer threads, or none: wait() takes the pieces that are left
+    }
+}
+
+ResultPages::~ResultPages() {
+    next_ = pieces_;      // whatever is not taken yet is not needed any more
+    for (auto& t : threads_) t.join();
+}
+
+void ResultPages::touch(size_t from, size_t to) {
+    if (from >= to) return;
+    volatile char* c = p_;
+    if (from == 0) c[0] = 0;
+    const uintptr_t base = (uintptr_t)p_;
+    for (uintptr_t a = (base + from + page_ - 1) / page_ * page_; a < base + to; a += page_) c[a - base] = 0;
+}
+
+void ResultPages::work() {
+    for (size_t i = next_++; i < pieces_; i = next_++) {
+        touch(i * PAGE_PIECE, std::min(bytes_, (i + 1) * PAGE_PIECE));
+        left_[i / (SLAB / PAGE_PIECE)].fetch_sub(1, std::memory_order_release);
+    }
+}
+
+void ResultPages::wait(size_t i) {
+    if (later_) {
+        later_ = false;
+        // the whole OpenMP team or none of it: a smaller one would make the
+        // runtime end the others' threads and start them again later (0.6 ms)
+        const int64_t n = (int64_t)((bytes_ + SMALL_PIECE - 1) / SMALL_PIECE);
+#pragma omp parallel for if (n > 128) schedule(static)
+        for (int64_t k = 0; k < n; ++k) touch((size_t)k * SMALL_PIECE, std::min(bytes_, ((size_t)k + 1) * SMALL_PIECE));
+        return;
+    }
+    if (!left_ || i >= slabs()) return;
+    if (threads_.empty()) work();
+    while (left_[i].load(std::memory_order_acquire)) std::this_thread::yield();
+}
+
+bool all_below(const uint32_t* ids, uint64_t n, uint64_t bound) {
+    uint32_t most = 0;
+#pragma omp simd reduction(max : most)
+    for (uint64_t i = 0; i < n; ++i) most = ids[i] > most ? ids[i] : most;
+    return !n || most < bound;
+}
+
+bool monotone(const uint64_t* off, uint64_t n) {
+    int bad = 0;
+#pragma omp parallel for if (n > (1u << 18)) schedule(static) reduction(| : bad)
+    for (int64_t i = 0; i < (int64_t)n; ++i) bad |= off[i + 1] < off[i];
+    return !bad;
+}
+
+}  // namespace ep

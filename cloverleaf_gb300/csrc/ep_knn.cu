@@ -5,7 +5,7 @@
 //                      with AvgAggregator / WeightedAggregator
 //                      (src/algos/aggregator.rs:17-120): warp per node.
 //   ep_align           NeighborhoodAligner.align (src/algos/alignment.rs,
-//                      src/lib.rs:3040-3110): warp per node.
+//                      src/lib.rs:3040-3110): warp per node, hubs by slices.
 //   ep_knn_cosine      NodeEmbeddings.nearest_neighbor for many queries at
 //                      once (src/embeddings.rs:149-173, cosine distance):
 //                      rows normalised to BF16, then a tcgen05 GEMM (FP32
@@ -23,6 +23,7 @@
 
 #include "../../include/ep_gb300.h"
 #include "ep_device.cuh"
+#include "ep_hostmem.h"
 
 namespace ep {
 namespace {
@@ -52,78 +53,304 @@ struct DevMem {
     cudaError_t alloc(size_t n) { return cudaMalloc(&p, n ? n : 16); }
 };
 
-// ---------------------------------------------------------------------------
-// Node embeddings: out[v] = sum_f w_f E[f] / sum_f w_f over v's features in
-// CSR order, f32 as the reference (w_f * e rounded, then added; the weights
-// summed in f32); nodes without features stay zero.  Up to 16 elements per
-// lane (dims <= 512).
-// ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) k_embed(uint64_t n, const uint64_t* __restrict__ fptr,
-                                               const uint32_t* __restrict__ fids, const float* __restrict__ fw,
-                                               uint32_t d, const float* __restrict__ table, float* __restrict__ out) {
-    const int lane = threadIdx.x & 31;
-    const uint64_t v = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (v >= n) return;
-    float acc[16];
-#pragma unroll
-    for (int i = 0; i < 16; ++i) acc[i] = 0.f;
-    float wsum = 0.f;
-    const uint64_t b = fptr[v], e = fptr[v + 1];
-    for (uint64_t j = b; j < e; ++j) {
-        const uint32_t f = fids[j];
-        const float w = fw ? fw[f] : 1.f;
-        wsum += w;
-        const float* row = table + (uint64_t)f * d;
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-            const uint32_t k = (uint32_t)lane + 32u * i;
-            if (k < d) acc[i] = __fadd_rn(acc[i], fw ? __fmul_rn(w, row[k]) : row[k]);
-        }
+// One device allocation cut into 256-byte-aligned pieces: a call allocates
+// and frees once (each cudaMalloc / cudaFree pair of some MB costs 50-200 us).
+struct Arena {
+    DevMem mem;
+    size_t used = 0;
+    size_t reserve(size_t n) { const size_t at = used; used += (n + 255) & ~(size_t)255; return at; }
+    template <typename X> X* at(size_t o) const { return reinterpret_cast<X*>(static_cast<char*>(mem.p) + o); }
+};
+
+// Counts whether any id is out of range.
+__global__ void __launch_bounds__(256) k_check_ids(const uint32_t* __restrict__ ids, uint64_t n, uint64_t bound,
+                                                   uint32_t* __restrict__ bad) {
+    const uint64_t step = (uint64_t)gridDim.x * blockDim.x;
+    bool out = false;
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += step) out = out || ids[i] >= bound;
+    if (out) *bad = 1u;
+}
+
+// Copies the ids to the device and reports whether all are below bound; the
+// kernels that follow index with the copy.  Few ids are checked by the host,
+// in less time than the answer takes to come back (35 us).
+constexpr uint64_t HOST_IDS = 1u << 17;
+cudaError_t upload_ids(uint32_t* dst, const uint32_t* src, uint64_t n, uint64_t bound, uint32_t* d_bad, cudaStream_t s,
+                       bool* ok) {
+    *ok = true;
+    if (!n) return cudaSuccess;
+    if (n <= HOST_IDS) {
+        *ok = all_below(src, n, bound);
+        return *ok ? cudaMemcpyAsync(dst, src, n * 4, cudaMemcpyHostToDevice, s) : cudaSuccess;
     }
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-        const uint32_t k = (uint32_t)lane + 32u * i;
-        if (k < d) out[v * d + k] = e > b ? acc[i] / wsum : 0.f;
+    cudaError_t e = cudaMemsetAsync(d_bad, 0, 4, s);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(dst, src, n * 4, cudaMemcpyHostToDevice, s);
+    if (e != cudaSuccess) return e;
+    k_check_ids<<<(unsigned)std::min<uint64_t>((n + 255) / 256, 152 * 8), 256, 0, s>>>(dst, n, bound, d_bad);
+    uint32_t bad = 0;
+    e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&bad, d_bad, 4, cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    *ok = !bad;
+    return e;
+}
+
+cudaError_t upload(void* dst, const void* src, size_t bytes, cudaStream_t s) {
+    return bytes ? cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s) : cudaSuccess;
+}
+
+// Bytes of a result array whose pages the host may touch: none of memory that
+// is the device's (the copy to it fails, as it should).
+size_t host_bytes(const void* out, size_t bytes) {
+    cudaPointerAttributes pa{};
+    const bool dev = cudaPointerGetAttributes(&pa, out) == cudaSuccess && pa.type == cudaMemoryTypeDevice;
+    cudaGetLastError();
+    return dev ? 0 : bytes;
+}
+
+// A result into the caller's array, each slab once its pages are resident.
+cudaError_t download(char* out, const void* d_out, size_t bytes, ResultPages& pages, cudaStream_t s) {
+    cudaError_t e = cudaSuccess;
+    for (size_t at = 0; at < bytes && e == cudaSuccess; at += ResultPages::SLAB) {
+        pages.wait(at / ResultPages::SLAB);
+        e = cudaMemcpyAsync(out + at, static_cast<const char*>(d_out) + at, std::min(bytes - at, ResultPages::SLAB),
+                            cudaMemcpyDeviceToHost, s);
     }
+    return e == cudaSuccess ? cudaStreamSynchronize(s) : e;
 }
 
 // ---------------------------------------------------------------------------
-// Neighbourhood alignment (NeighborhoodAligner.align, src/algos/alignment.rs:
-// 25-75): out[v] = (1 - a) * sum_j p_j E[u_j] + a * E[v] over the first
-// min(deg, kmax) edges in CSR order, p_j the edge probability recovered from
-// the CDF weights (w_0, w_j - w_{j-1}), a = alpha, or min(1, 1 / ln(deg + 1))
-// when alpha < 0.  f32 as the reference: every product rounded, then added,
-// per element in edge order.  Warp per node, up to 16 elements per lane.
+// Weighted sums of rows, one warp per node (k_rows):
+//   ROWS_MEAN / ROWS_WEIGHTED (node embeddings): out[v] = sum_f w_f E[f] /
+//     sum_f w_f over v's features in CSR order, f32 as the reference (w_f * e
+//     rounded, then added; the weights summed in f32); nodes without features
+//     get zeros.
+//   ROWS_ALIGN (NeighborhoodAligner.align, src/algos/alignment.rs:25-75):
+//     out[v] = (1 - a) * sum_j p_j E[u_j] + a * E[v] over the first
+//     min(deg, kmax) edges in CSR order, p_j the edge probability recovered
+//     from the CDF weights (w_0, w_j - w_{j-1}), a = alpha, or min(1, 1 /
+//     ln(deg + 1)) when alpha < 0; every product rounded, then added, per
+//     element in edge order.
+// A lane owns NV groups of 4 consecutive elements (V4; dims a multiple of 4
+// and a 16-byte-aligned result) or NV elements 32 apart.  Ids and
+// coefficients come 32 at a time across the lanes; U rows are in flight.
+// Bound by the row reads from L2 (ROWS_ALIGN, 200,000 nodes, 4M edges x 128:
+// 2 GB).
+// Rows of more than HUB_ROWS edges, whose sums are one long chain, are left
+// to the first HUB_CTAS CTAs of the grid: a CTA per hub and slice of 32
+// elements, whose warps load and weigh HUB_TILE rows at a time into shared
+// memory while one warp adds up the tile before, in edge order.  (4.1 ms
+// before, all of it the 10,000-edge hub's chain with one row in flight.)
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) k_align(uint64_t n, const uint64_t* __restrict__ rp,
-                                               const uint32_t* __restrict__ cols, const float* __restrict__ cdf,
-                                               uint32_t d, const float* __restrict__ E, float alpha, uint64_t kmax,
-                                               float* __restrict__ out) {
+enum RowsMode : int { ROWS_MEAN = 0, ROWS_WEIGHTED = 1, ROWS_ALIGN = 2 };
+constexpr uint32_t HUB_ROWS = 256;
+constexpr unsigned HUB_CTAS = 152;
+constexpr uint32_t HUB_TILE = 128;
+
+struct RowsParams {
+    uint64_t n;                  // nodes
+    const uint64_t* ptr;         // CSR offsets
+    const uint32_t* ids;         // feature ids / neighbours
+    const float* w;              // feature weights / CDF weights
+    uint32_t d;
+    const float* table;
+    float alpha;
+    uint64_t kmax;
+    const uint32_t* hubs;        // nodes of more than HUB_ROWS edges
+    const uint32_t* n_hubs;
+    float* out;
+};
+
+__device__ __forceinline__ float align_keep(const RowsParams& p, uint64_t deg) {
+    return p.alpha >= 0.f ? p.alpha : fminf(__fdiv_rn(1.f, logf(__fadd_rn((float)deg, 1.f))), 1.f);
+}
+
+__device__ __forceinline__ float edge_p(const RowsParams& p, uint64_t b, uint64_t j) {
+    return j ? __fsub_rn(p.w[b + j], p.w[b + j - 1]) : p.w[b];
+}
+
+__device__ void hub_rows(const RowsParams& p) {
+    __shared__ float tile[2][HUB_TILE][32];
+    constexpr uint32_t PW = HUB_TILE / 8;                // rows of a tile per warp
     const int lane = threadIdx.x & 31;
-    const uint64_t v = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (v >= n) return;
-    float acc[16];
+    const uint32_t w = threadIdx.x >> 5;
+    const uint32_t slices = (p.d + 31) / 32;
+    const uint64_t n = (uint64_t)*p.n_hubs * slices;
+    for (uint64_t it = blockIdx.x; it < n; it += HUB_CTAS) {
+        const uint64_t v = p.hubs[it / slices];
+        const uint32_t k = (uint32_t)(it % slices) * 32u + lane;
+        const uint32_t kl = k < p.d ? k : p.d - 1;       // lanes past the row read its last element
+        const uint64_t b = p.ptr[v], deg = p.ptr[v + 1] - b;
+        const uint64_t m = deg < p.kmax ? deg : p.kmax;
+        float x[PW], pj = 0.f;
+        // this warp's rows of the tile at edge t0, into registers
+        auto load = [&](uint64_t t0) {
+            const uint64_t j = t0 + w * PW + lane;
+            uint32_t id = 0;
+            pj = 0.f;
+            if ((uint32_t)lane < PW && j < m) {
+                id = p.ids[b + j];
+                pj = edge_p(p, b, j);
+            }
 #pragma unroll
-    for (int i = 0; i < 16; ++i) acc[i] = 0.f;
-    const uint64_t b = rp[v], deg = rp[v + 1] - b;
-    const uint64_t m = deg < kmax ? deg : kmax;
-    for (uint64_t j = 0; j < m; ++j) {
-        const float p = j ? __fsub_rn(cdf[b + j], cdf[b + j - 1]) : cdf[b];
-        const float* row = E + (uint64_t)cols[b + j] * d;
+            for (uint32_t t = 0; t < PW; ++t) {
+                const uint32_t u = __shfl_sync(FULL, id, (int)t);
+                if (t0 + w * PW + t < m) x[t] = p.table[(uint64_t)u * p.d + kl];
+            }
+        };
+        auto store = [&](uint64_t t0, uint32_t buf) {
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {
-            const uint32_t k = (uint32_t)lane + 32u * i;
-            if (k < d) acc[i] = __fadd_rn(acc[i], __fmul_rn(p, row[k]));
+            for (uint32_t t = 0; t < PW; ++t) {
+                const float q = __shfl_sync(FULL, pj, (int)t);
+                if (t0 + w * PW + t < m) tile[buf][w * PW + t][lane] = __fmul_rn(q, x[t]);
+            }
+        };
+        float acc = 0.f;
+        uint32_t buf = 0;
+        load(0);
+        store(0, 0);
+        __syncthreads();
+        for (uint64_t t0 = 0; t0 < m; t0 += HUB_TILE, buf ^= 1u) {
+            const bool more = t0 + HUB_TILE < m;
+            if (more) load(t0 + HUB_TILE);               // in flight while the tile is summed
+            if (w == 0) {
+                const uint32_t cnt = (uint32_t)min((uint64_t)HUB_TILE, m - t0);
+                if (cnt == HUB_TILE) {
+#pragma unroll 16
+                    for (uint32_t t = 0; t < HUB_TILE; ++t) acc = __fadd_rn(acc, tile[buf][t][lane]);
+                } else {
+                    for (uint32_t t = 0; t < cnt; ++t) acc = __fadd_rn(acc, tile[buf][t][lane]);
+                }
+            }
+            if (more) store(t0 + HUB_TILE, buf ^ 1u);
+            __syncthreads();
+        }
+        const float a = align_keep(p, deg), c = __fsub_rn(1.f, a);
+        if (w == 0 && k < p.d) p.out[v * p.d + k] = __fadd_rn(__fmul_rn(acc, c), __fmul_rn(p.table[v * p.d + k], a));
+    }
+}
+
+template <int NV, bool V4, int MODE>
+__global__ void __launch_bounds__(256) k_rows(const RowsParams p) {
+    unsigned block = blockIdx.x;
+    if constexpr (MODE == ROWS_ALIGN) {
+        if (block < HUB_CTAS) {
+            hub_rows(p);
+            return;
+        }
+        block -= HUB_CTAS;
+    }
+    constexpr int E = V4 ? 4 : 1;
+    constexpr int U = NV * E >= 16 ? 2 : (NV * E >= 8 ? 4 : 8);     // rows in flight
+    const int lane = threadIdx.x & 31;
+    const uint64_t v = ((uint64_t)block * blockDim.x + threadIdx.x) >> 5;
+    if (v >= p.n) return;
+    const uint32_t d = p.d;
+    const uint64_t b = p.ptr[v], deg = p.ptr[v + 1] - b;
+    if (MODE == ROWS_ALIGN && deg > HUB_ROWS) return;
+    const uint64_t m = MODE == ROWS_ALIGN && p.kmax < deg ? p.kmax : deg;
+    float acc[NV][E];
+#pragma unroll
+    for (int i = 0; i < NV; ++i)
+#pragma unroll
+        for (int e = 0; e < E; ++e) acc[i][e] = 0.f;
+    uint32_t at[NV];
+    bool on[NV];
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+        at[i] = (uint32_t)(lane + 32 * i) * E;
+        on[i] = at[i] < d;
+        if (!on[i]) at[i] = 0;         // read, and not stored
+    }
+    auto load = [&](uint64_t row, float (&x)[NV][E]) {
+        const float* r = p.table + row * d;
+#pragma unroll
+        for (int i = 0; i < NV; ++i) {
+            if constexpr (V4) {
+                const float4 q = *reinterpret_cast<const float4*>(r + at[i]);
+                x[i][0] = q.x; x[i][1] = q.y; x[i][2] = q.z; x[i][3] = q.w;
+            } else {
+                x[i][0] = r[at[i]];
+            }
+        }
+    };
+    float wsum = 0.f;
+    for (uint64_t j0 = 0; j0 < m; j0 += 32) {
+        const uint32_t cnt = (uint32_t)min((uint64_t)32, m - j0);
+        uint32_t id = 0;
+        float cf = 1.f;
+        if ((uint32_t)lane < cnt) {
+            id = p.ids[b + j0 + lane];
+            if (MODE == ROWS_WEIGHTED) cf = p.w[id];
+            if (MODE == ROWS_ALIGN) cf = edge_p(p, b, j0 + lane);
+        }
+        for (uint32_t t0 = 0; t0 < cnt; t0 += U) {
+            float x[U][NV][E];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const uint32_t row = __shfl_sync(FULL, id, (int)(t0 + u) & 31);
+                if (t0 + u < cnt) load(row, x[u]);
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const float c = __shfl_sync(FULL, cf, (int)(t0 + u) & 31);
+                if (t0 + u < cnt) {
+                    if (MODE != ROWS_ALIGN) wsum += c;
+#pragma unroll
+                    for (int i = 0; i < NV; ++i)
+#pragma unroll
+                        for (int e = 0; e < E; ++e)
+                            acc[i][e] = __fadd_rn(acc[i][e], MODE == ROWS_MEAN ? x[u][i][e] : __fmul_rn(c, x[u][i][e]));
+                }
+            }
         }
     }
-    const float a = alpha >= 0.f ? alpha : fminf(__fdiv_rn(1.f, logf(__fadd_rn((float)deg, 1.f))), 1.f);
-    const float c = __fsub_rn(1.f, a);
-    const float* own = E + v * d;
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-        const uint32_t k = (uint32_t)lane + 32u * i;
-        if (k < d) out[v * d + k] = __fadd_rn(__fmul_rn(acc[i], c), __fmul_rn(own[k], a));
+    float own[NV][E];
+    float a = 0.f, c = 0.f;
+    if constexpr (MODE == ROWS_ALIGN) {
+        a = align_keep(p, deg);
+        c = __fsub_rn(1.f, a);
+        load(v, own);
     }
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+        float o[E];
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+            if constexpr (MODE == ROWS_ALIGN) o[e] = __fadd_rn(__fmul_rn(acc[i][e], c), __fmul_rn(own[i][e], a));
+            else o[e] = m ? acc[i][e] / wsum : 0.f;
+        }
+        if (on[i]) {
+            float* to = p.out + v * d + at[i];
+            if constexpr (V4) *reinterpret_cast<float4*>(to) = make_float4(o[0], o[1], o[2], o[3]);
+            else *to = o[0];
+        }
+    }
+}
+
+// The nodes of more than HUB_ROWS edges, in any order.
+__global__ void __launch_bounds__(256) k_find_hubs(uint64_t n, const uint64_t* __restrict__ ptr, uint32_t* __restrict__ hubs,
+                                                   uint32_t* __restrict__ n_hubs) {
+    for (uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (uint64_t)gridDim.x * blockDim.x)
+        if (ptr[v + 1] - ptr[v] > HUB_ROWS) hubs[atomicAdd(n_hubs, 1u)] = (uint32_t)v;
+}
+
+template <int MODE>
+cudaError_t launch_rows(const RowsParams& p, cudaStream_t s) {
+    const unsigned blocks = (unsigned)((p.n + 7) / 8) + (MODE == ROWS_ALIGN ? HUB_CTAS : 0u);
+    const uint32_t d = p.d;
+    if (d % 4 == 0) {            // rows of 16-byte multiples (table and result are arena pieces)
+        if (d <= 128) k_rows<1, true, MODE><<<blocks, 256, 0, s>>>(p);
+        else if (d <= 256) k_rows<2, true, MODE><<<blocks, 256, 0, s>>>(p);
+        else k_rows<4, true, MODE><<<blocks, 256, 0, s>>>(p);
+    } else {
+        if (d <= 32) k_rows<1, false, MODE><<<blocks, 256, 0, s>>>(p);
+        else if (d <= 64) k_rows<2, false, MODE><<<blocks, 256, 0, s>>>(p);
+        else if (d <= 128) k_rows<4, false, MODE><<<blocks, 256, 0, s>>>(p);
+        else if (d <= 256) k_rows<8, false, MODE><<<blocks, 256, 0, s>>>(p);
+        else k_rows<16, false, MODE><<<blocks, 256, 0, s>>>(p);
+    }
+    return cudaGetLastError();
 }
 
 // Rows scaled to unit L2 norm (zero rows stay zero), rounded to BF16 and
@@ -614,33 +841,38 @@ extern "C" int ep_embed_features(int device, uint64_t n_nodes, const uint64_t* f
                                  float* out) {
     if (!fptr || !out || (n_nodes && !table && n_feat) || dims == 0 || dims > 512)
         return knn_fail(EP_ERR_INVALID_ARG, "invalid arguments (dims must be in [1, 512])");
+    if (!monotone(fptr, n_nodes)) return knn_fail(EP_ERR_INVALID_ARG, "fptr is not monotone");
     const uint64_t nf = fptr[n_nodes];
-    for (uint64_t v = 0; v < n_nodes; ++v)
-        if (fptr[v + 1] < fptr[v]) return knn_fail(EP_ERR_INVALID_ARG, "fptr is not monotone");
-    for (uint64_t j = 0; j < nf; ++j)
+    for (uint64_t j = 0; !n_nodes && j < nf; ++j)      // no node reads them, but they are the caller's
         if (fids[j] >= n_feat) return knn_fail(EP_ERR_INVALID_ARG, "feature id out of range");
     KCK(cudaSetDevice(device), "select device");
     if (!n_nodes) return EP_OK;
     cudaStream_t s;
     KCK(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking), "stream");
     struct SG { cudaStream_t s; ~SG() { cudaStreamDestroy(s); } } sg{s};
-    DevMem dptr, dids, dw, dtab, dout;
-    KCK(dptr.alloc((n_nodes + 1) * 8), "alloc");
-    KCK(dids.alloc(nf * 4), "alloc");
-    KCK(dtab.alloc((size_t)n_feat * dims * 4), "alloc");
-    KCK(dout.alloc((size_t)n_nodes * dims * 4), "alloc");
-    if (fweight) KCK(dw.alloc((size_t)n_feat * 4), "alloc");
-    KCK(cudaMemcpyAsync(dptr.p, fptr, (n_nodes + 1) * 8, cudaMemcpyHostToDevice, s), "upload");
-    if (nf) KCK(cudaMemcpyAsync(dids.p, fids, nf * 4, cudaMemcpyHostToDevice, s), "upload");
-    if (n_feat) KCK(cudaMemcpyAsync(dtab.p, table, (size_t)n_feat * dims * 4, cudaMemcpyHostToDevice, s), "upload");
-    if (fweight) KCK(cudaMemcpyAsync(dw.p, fweight, (size_t)n_feat * 4, cudaMemcpyHostToDevice, s), "upload");
-    const uint64_t blocks = (n_nodes * 32 + 255) / 256;
-    k_embed<<<(unsigned)blocks, 256, 0, s>>>(n_nodes, (const uint64_t*)dptr.p, (const uint32_t*)dids.p,
-                                             fweight ? (const float*)dw.p : nullptr, dims, (const float*)dtab.p,
-                                             (float*)dout.p);
-    KCK(cudaGetLastError(), "embed launch");
-    KCK(cudaMemcpyAsync(out, dout.p, (size_t)n_nodes * dims * 4, cudaMemcpyDeviceToHost, s), "download");
-    KCK(cudaStreamSynchronize(s), "embed");
+    Arena ar;
+    const size_t out_bytes = (size_t)n_nodes * dims * 4;
+    const size_t o_bad = ar.reserve(4), o_ptr = ar.reserve((n_nodes + 1) * 8), o_ids = ar.reserve(nf * 4),
+                 o_tab = ar.reserve((size_t)n_feat * dims * 4), o_w = ar.reserve(fweight ? (size_t)n_feat * 4 : 0),
+                 o_out = ar.reserve(out_bytes);
+    KCK(ar.mem.alloc(ar.used), "alloc");
+    bool ok = true;
+    KCK(upload_ids(ar.at<uint32_t>(o_ids), fids, nf, n_feat, ar.at<uint32_t>(o_bad), s, &ok), "upload");
+    if (!ok) return knn_fail(EP_ERR_INVALID_ARG, "feature id out of range");
+    ResultPages pages(out, host_bytes(out, out_bytes));
+    KCK(upload(ar.at<void>(o_ptr), fptr, (n_nodes + 1) * 8, s), "upload");
+    KCK(upload(ar.at<void>(o_tab), table, (size_t)n_feat * dims * 4, s), "upload");
+    if (fweight) KCK(upload(ar.at<void>(o_w), fweight, (size_t)n_feat * 4, s), "upload");
+    RowsParams p{};
+    p.n = n_nodes;
+    p.ptr = ar.at<uint64_t>(o_ptr);
+    p.ids = ar.at<uint32_t>(o_ids);
+    p.w = ar.at<float>(o_w);
+    p.d = dims;
+    p.table = ar.at<float>(o_tab);
+    p.out = ar.at<float>(o_out);
+    KCK((fweight ? launch_rows<ROWS_WEIGHTED>(p, s) : launch_rows<ROWS_MEAN>(p, s)), "embed launch");
+    KCK(download((char*)out, p.out, out_bytes, pages, s), "embed");
     return EP_OK;
 }
 
@@ -652,39 +884,49 @@ extern "C" int ep_align(int device, uint64_t n_nodes, const uint64_t* row_ptr, c
     if (alpha > 1.f || alpha != alpha) return knn_fail(EP_ERR_INVALID_ARG, "alpha must be <= 1 (negative: adaptive)");
     const uint64_t ne = row_ptr[n_nodes];
     if (ne && (!cols || !w_cdf)) return knn_fail(EP_ERR_INVALID_ARG, "null edge arrays");
-    for (uint64_t v = 0; v < n_nodes; ++v)
-        if (row_ptr[v + 1] < row_ptr[v]) return knn_fail(EP_ERR_INVALID_ARG, "row_ptr is not monotone");
-    for (uint64_t j = 0; j < ne; ++j)
-        if (cols[j] >= n_nodes) return knn_fail(EP_ERR_INVALID_ARG, "column id out of range");
+    if (!monotone(row_ptr, n_nodes)) return knn_fail(EP_ERR_INVALID_ARG, "row_ptr is not monotone");
+    if (!n_nodes && ne) return knn_fail(EP_ERR_INVALID_ARG, "column id out of range");
     KCK(cudaSetDevice(device), "select device");
     if (!n_nodes) return EP_OK;
     cudaStream_t s;
     KCK(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking), "stream");
     struct SG { cudaStream_t s; ~SG() { cudaStreamDestroy(s); } } sg{s};
-    DevMem drp, dcols, dcdf, demb, dout;
-    KCK(drp.alloc((n_nodes + 1) * 8), "alloc");
-    KCK(dcols.alloc(ne * 4), "alloc");
-    KCK(dcdf.alloc(ne * 4), "alloc");
-    KCK(demb.alloc((size_t)n_nodes * dims * 4), "alloc");
-    KCK(dout.alloc((size_t)n_nodes * dims * 4), "alloc");
-    KCK(cudaMemcpyAsync(drp.p, row_ptr, (n_nodes + 1) * 8, cudaMemcpyHostToDevice, s), "upload");
-    if (ne) {
-        KCK(cudaMemcpyAsync(dcols.p, cols, ne * 4, cudaMemcpyHostToDevice, s), "upload");
-        KCK(cudaMemcpyAsync(dcdf.p, w_cdf, ne * 4, cudaMemcpyHostToDevice, s), "upload");
-    }
-    KCK(cudaMemcpyAsync(demb.p, emb, (size_t)n_nodes * dims * 4, cudaMemcpyHostToDevice, s), "upload");
+    Arena ar;
+    const size_t out_bytes = (size_t)n_nodes * dims * 4;
+    const size_t o_bad = ar.reserve(4), o_nh = ar.reserve(4), o_rp = ar.reserve((n_nodes + 1) * 8), o_cols = ar.reserve(ne * 4),
+                 o_cdf = ar.reserve(ne * 4), o_emb = ar.reserve(out_bytes),
+                 o_hubs = ar.reserve((ne / (HUB_ROWS + 1) + 1) * 4), o_out = ar.reserve(out_bytes);
+    KCK(ar.mem.alloc(ar.used), "alloc");
+    bool ok = true;
+    KCK(upload_ids(ar.at<uint32_t>(o_cols), cols, ne, n_nodes, ar.at<uint32_t>(o_bad), s, &ok), "upload");
+    if (!ok) return knn_fail(EP_ERR_INVALID_ARG, "column id out of range");
+    ResultPages pages(out, host_bytes(out, out_bytes));
+    KCK(upload(ar.at<void>(o_rp), row_ptr, (n_nodes + 1) * 8, s), "upload");
+    KCK(upload(ar.at<void>(o_cdf), w_cdf, ne * 4, s), "upload");
+    KCK(upload(ar.at<void>(o_emb), emb, out_bytes, s), "upload");
+    RowsParams p{};
+    p.n = n_nodes;
+    p.ptr = ar.at<uint64_t>(o_rp);
+    p.ids = ar.at<uint32_t>(o_cols);
+    p.w = ar.at<float>(o_cdf);
+    p.d = dims;
+    p.table = ar.at<float>(o_emb);
+    p.alpha = alpha;
+    p.kmax = max_neighbors ? max_neighbors : ~0ull;
+    p.hubs = ar.at<uint32_t>(o_hubs);
+    p.n_hubs = ar.at<uint32_t>(o_nh);
+    p.out = ar.at<float>(o_out);
     cudaEvent_t e0, e1;
     KCK(cudaEventCreate(&e0), "events");
     KCK(cudaEventCreate(&e1), "events");
     struct EG { cudaEvent_t a, b; ~EG() { cudaEventDestroy(a); cudaEventDestroy(b); } } eg{e0, e1};
+    KCK(cudaMemsetAsync(ar.at<void>(o_nh), 0, 4, s), "clear");
     cudaEventRecord(e0, s);
-    k_align<<<(unsigned)((n_nodes * 32 + 255) / 256), 256, 0, s>>>(
-        n_nodes, (const uint64_t*)drp.p, (const uint32_t*)dcols.p, (const float*)dcdf.p, dims,
-        (const float*)demb.p, alpha, max_neighbors ? max_neighbors : ~0ull, (float*)dout.p);
+    k_find_hubs<<<(unsigned)std::min<uint64_t>((n_nodes + 255) / 256, 152 * 8), 256, 0, s>>>(
+        n_nodes, ar.at<uint64_t>(o_rp), ar.at<uint32_t>(o_hubs), ar.at<uint32_t>(o_nh));
+    KCK(launch_rows<ROWS_ALIGN>(p, s), "align launch");
     cudaEventRecord(e1, s);
-    KCK(cudaGetLastError(), "align launch");
-    KCK(cudaMemcpyAsync(out, dout.p, (size_t)n_nodes * dims * 4, cudaMemcpyDeviceToHost, s), "download");
-    KCK(cudaStreamSynchronize(s), "align");
+    KCK(download((char*)out, p.out, out_bytes, pages, s), "align");
     cudaEventElapsedTime(&g_knn_ms, e0, e1);
     return EP_OK;
 }

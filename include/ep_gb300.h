@@ -236,7 +236,7 @@ int ep_batch_step(ep_ctx* ctx, const ep_batch_samples* samples, float lr, uint32
  * memory (cudaHostAlloc / cudaHostRegister, e.g. a pinned torch tensor) and
  * dims is a multiple of 4, a kernel writes the rows into it directly at the
  * host link's rate; otherwise the rows go through a device staging buffer
- * allocated on first use and one copy. */
+ * allocated on first use and are copied. */
 int ep_get_table(ep_ctx* ctx, float* out);
 
 /* Launch shapes in use (no counterpart in the reference): the reducer's items
@@ -352,8 +352,8 @@ int ep_align(int device, uint64_t n_nodes, const uint64_t* row_ptr, const uint32
 const char* ep_knn_last_error(void);
 
 /* Measurement hook (no counterpart in the reference): CUDA-event time in ms
- * of the GPU kernel of this host thread's last ep_knn_cosine (the top-k
- * kernel) or ep_align call. */
+ * of the GPU kernels of this host thread's last ep_knn_cosine (the top-k
+ * kernels) or ep_align call. */
 float ep_knn_last_kernel_ms(void);
 
 /* ---- host-side graph construction (src/graph.rs) --------------------- */
