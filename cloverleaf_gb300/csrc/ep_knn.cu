@@ -365,25 +365,35 @@ __device__ __forceinline__ uint64_t swz_offset(uint64_t row, uint32_t k, uint32_
     return tile * nkb * kb_bytes + kb * kb_bytes + (r >> 3) * 1024u + (r & 7u) * 128u + ((c ^ (r & 7u)) << 4) + e * 2u;
 }
 
-__global__ void __launch_bounds__(256) k_norm_swz(uint64_t n, uint64_t n_tiled, uint32_t d, uint32_t dpad,
+// Rows r0 up to n_tiled (x starts at row r0), a warp per row; a row's values
+// are loaded once, all of them in flight (dims <= 256: up to 8 per lane).
+__global__ void __launch_bounds__(256) k_norm_swz(uint64_t r0, uint64_t n, uint64_t n_tiled, uint32_t d, uint32_t dpad,
                                                   uint32_t tlog, const float* __restrict__ x,
                                                   unsigned char* __restrict__ y) {
     const int lane = threadIdx.x & 31;
-    const uint64_t r = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const uint64_t r = r0 + (((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     if (r >= n_tiled) return;
     const bool in = r < n;
+    float t[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const uint32_t k = (uint32_t)(lane + 32 * i);
+        t[i] = in && k < d ? x[(r - r0) * d + k] : 0.f;
+    }
     float ss = 0.f;
-    if (in)
-        for (uint32_t k = lane; k < d; k += 32) {
-            const float t = x[r * d + k];
-            ss += t * t;
-        }
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+        if ((uint32_t)(lane + 32 * i) < d) ss += t[i] * t[i];
     ss = warp_sum<float>(ss);
     const float inv = ss > 0.f ? 1.f / sqrtf(ss) : 0.f;
     const uint32_t nkb = dpad / 64;
-    for (uint32_t k = lane; k < dpad; k += 32) {
-        const float v = (in && k < d) ? x[r * d + k] * inv : 0.f;
-        *reinterpret_cast<__nv_bfloat16*>(y + swz_offset(r, k, nkb, tlog)) = __float2bfloat16_rn(v);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const uint32_t k = (uint32_t)(lane + 32 * i);
+        if (k < dpad) {
+            const float v = (in && k < d) ? t[i] * inv : 0.f;
+            *reinterpret_cast<__nv_bfloat16*>(y + swz_offset(r, k, nkb, tlog)) = __float2bfloat16_rn(v);
+        }
     }
 }
 
@@ -407,6 +417,8 @@ __global__ void __launch_bounds__(256) k_norm_swz(uint64_t n, uint64_t n_tiled, 
 // skipping blocks of 16 or 32 values whose maximum cannot enter; the slices'
 // lists are merged per query at the end.  Operands sit in shared memory as K-major,
 // 128-byte-swizzled tiles.
+// The database may be split (blockIdx.y, tiles_per tiles each, from tile t0
+// on): every split's slice lists go to `part` and k_merge_topk joins them.
 // All waits are bounded; a timeout sets an abort flag that ends every role's
 // loop, the copies and MMAs still in flight are waited for, and the error
 // word is set.
@@ -568,9 +580,10 @@ __device__ __forceinline__ float kth_value(const float (&vals)[KMAX], uint32_t k
 
 template <int KMAX>
 __global__ void __launch_bounds__(KnnRoles<KMAX>::THREADS, 1)
-    k_cos_topk(const unsigned char* __restrict__ Q, uint64_t nq, const unsigned char* __restrict__ D, uint64_t ndb,
+    k_cos_topk(const unsigned char* __restrict__ Q, uint64_t nq, const unsigned char* __restrict__ Dall, uint64_t ndb,
                uint32_t dpad, const uint64_t* __restrict__ qself, uint32_t k, uint32_t* __restrict__ idx_out,
-               float* __restrict__ sim_out, uint32_t* __restrict__ err) {
+               float* __restrict__ sim_out, uint32_t* __restrict__ err, uint32_t t0, uint32_t t1, uint32_t tiles_per,
+               uint32_t split0, uint2* __restrict__ part) {
     using R = KnnRoles<KMAX>;
     extern __shared__ unsigned char knn_smem_raw[];
     __shared__ uint64_t bar_a, bar_full[KNN_STAGES], bar_empty[KNN_STAGES], bar_acc_full[KNN_ACC],
@@ -584,7 +597,10 @@ __global__ void __launch_bounds__(KnnRoles<KMAX>::THREADS, 1)
     unsigned char* sA = smem;
     auto sB = [&](uint32_t st) { return smem + a_bytes + st * KNN_B_KB; };
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint64_t ntiles = (ndb + KNN_BN - 1) / KNN_BN, nstages = ntiles * nkb;
+    const uint32_t first = t0 + blockIdx.y * tiles_per;              // this split's tiles [first, last)
+    const uint32_t last = min(t1, first + tiles_per);
+    const uint64_t ntiles = first < last ? last - first : 0, nstages = ntiles * nkb;
+    const unsigned char* D = Dall + (uint64_t)first * nkb * KNN_B_KB;
 
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)),
@@ -729,7 +745,7 @@ __global__ void __launch_bounds__(KnnRoles<KMAX>::THREADS, 1)
                     unsigned cand = 0;
 #pragma unroll
                     for (int t = 0; t < R::BW; ++t) cand |= (__uint_as_float(r[cb][t]) > thr ? 1u : 0u) << t;
-                    const uint32_t col0 = (uint32_t)j * KNN_BN + (uint32_t)(slice * R::CW + bl * R::BW);
+                    const uint32_t col0 = (first + (uint32_t)j) * KNN_BN + (uint32_t)(slice * R::CW + bl * R::BW);
                     while (cand) {
                         const int t = __ffs(cand) - 1;
                         cand &= cand - 1;
@@ -764,6 +780,14 @@ __global__ void __launch_bounds__(KnnRoles<KMAX>::THREADS, 1)
                 const uint64_t sg = s_issued - 1;
                 mbar_wait(&bar_empty[sg % KNN_STAGES], (uint32_t)((sg / KNN_STAGES) & 1), &never);
             }
+        }
+    } else if (part) {
+        // the first k entries of every slice's list, for k_merge_topk
+        if (warp < R::EPI && myq < nq) {
+            uint2* to = part + (((uint64_t)(split0 + blockIdx.y) * nq + myq) * R::SLICES + slice) * k;
+#pragma unroll
+            for (int i = 0; i < KMAX; ++i)
+                if ((uint32_t)i < k) to[i] = make_uint2(__float_as_uint(vals[i]), ids[i]);
         }
     } else {
         // merge the slices' sorted lists per query (the stages are free now)
@@ -805,30 +829,83 @@ __global__ void __launch_bounds__(KnnRoles<KMAX>::THREADS, 1)
     }
 }
 
-// compile-time selection by k
+// Joins the sorted lists of one query (splits x slices lists of k entries),
+// a warp per query: k rounds of picking the best head.  Among equal
+// similarities the lower slice comes first, then the lower row: the order in
+// which one CTA over the whole database admits them (its slice lists keep
+// row order, and are joined slice by slice).
+__global__ void __launch_bounds__(128) k_merge_topk(const uint2* __restrict__ part, uint64_t nq, uint32_t splits,
+                                                    uint32_t slices, uint32_t k, uint32_t* __restrict__ idx_out,
+                                                    float* __restrict__ sim_out) {
+    extern __shared__ uint8_t merge_pos[];               // [warps][lists]: entries taken of each list
+    const int lane = threadIdx.x & 31;
+    const uint64_t q = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (q >= nq) return;
+    const uint32_t lists = splits * slices;
+    uint8_t* pos = merge_pos + (size_t)(threadIdx.x >> 5) * lists;
+    for (uint32_t l = lane; l < lists; l += 32) pos[l] = 0;
+    for (uint32_t r = 0; r < k; ++r) {
+        float bv = -INFINITY;
+        uint32_t bid = 0xffffffffu, bsl = 0xffffffffu, bl = 0xffffffffu;
+        auto better = [&](float v, uint32_t sl, uint32_t id) {
+            return v > bv || (v == bv && v > -INFINITY && (sl < bsl || (sl == bsl && id < bid)));
+        };
+        for (uint32_t l = lane; l < lists; l += 32) {
+            const uint32_t i = pos[l], sl = l % slices;
+            if (i >= k) continue;
+            const uint2 e = part[(((uint64_t)(l / slices)) * nq + q) * slices * k + (uint64_t)sl * k + i];
+            if (better(__uint_as_float(e.x), sl, e.y)) { bv = __uint_as_float(e.x); bid = e.y; bsl = sl; bl = l; }
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const float v = __shfl_xor_sync(FULL, bv, o);
+            const uint32_t id = __shfl_xor_sync(FULL, bid, o), sl = __shfl_xor_sync(FULL, bsl, o), l = __shfl_xor_sync(FULL, bl, o);
+            if (better(v, sl, id)) { bv = v; bid = id; bsl = sl; bl = l; }
+        }
+        if (bl != 0xffffffffu && (uint32_t)lane == (bl & 31u)) ++pos[bl];
+        if (lane == 0) {
+            idx_out[q * k + r] = bid;
+            sim_out[q * k + r] = bv;
+        }
+    }
+}
+
+// One launch of k_cos_topk over database tiles [t0, t1) in `splits` splits;
+// part null: the whole database, straight to the results.
+struct KnnArgs {
+    const unsigned char *Q, *D;
+    uint64_t nq, ndb;
+    uint32_t dpad;
+    const uint64_t* qself;
+    uint32_t k;
+    uint32_t* idx;
+    float* sim;
+    uint32_t* err;
+    uint2* part;
+};
+
 template <int KMAX>
-int knn_run(const unsigned char* Q, uint64_t nq, const unsigned char* D, uint64_t ndb, uint32_t dpad,
-            const uint64_t* qself, uint32_t k, uint32_t* idx, float* sim, uint32_t* err, cudaStream_t s) {
+cudaError_t knn_launch(const KnnArgs& a, uint32_t t0, uint32_t t1, uint32_t splits, uint32_t split0, cudaStream_t s) {
     // query tile + KNN_STAGES K-block stages (reused at the end for the slices' lists)
-    const size_t tiles = (size_t)(dpad / 64) * KNN_A_KB + (size_t)KNN_STAGES * KNN_B_KB;
+    const size_t tiles = (size_t)(a.dpad / 64) * KNN_A_KB + (size_t)KNN_STAGES * KNN_B_KB;
     const size_t lists = (size_t)KnnRoles<KMAX>::SLICES * KNN_BM * KMAX * 8;
     const size_t smem = std::max(tiles, lists) + 1024;
-    KCK(cudaFuncSetAttribute(k_cos_topk<KMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-        "knn shared memory");
-    const unsigned grid = (unsigned)((nq + KNN_BM - 1) / KNN_BM);
-    cudaEvent_t e0, e1;
-    KCK(cudaEventCreate(&e0), "events");
-    KCK(cudaEventCreate(&e1), "events");
-    cudaEventRecord(e0, s);
-    k_cos_topk<KMAX><<<grid, KnnRoles<KMAX>::THREADS, smem, s>>>(Q, nq, D, ndb, dpad, qself, k, idx, sim, err);
-    cudaEventRecord(e1, s);
-    cudaError_t e = cudaGetLastError();
-    if (e == cudaSuccess) e = cudaEventSynchronize(e1);
-    if (e == cudaSuccess) cudaEventElapsedTime(&g_knn_ms, e0, e1);
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
-    KCK(e, "knn launch");
-    return EP_OK;
+    const cudaError_t e = cudaFuncSetAttribute(k_cos_topk<KMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    const dim3 grid((unsigned)((a.nq + KNN_BM - 1) / KNN_BM), splits);
+    const uint32_t per = (t1 - t0 + splits - 1) / splits;
+    k_cos_topk<KMAX><<<grid, KnnRoles<KMAX>::THREADS, smem, s>>>(a.Q, a.nq, a.D, a.ndb, a.dpad, a.qself, a.k, a.idx, a.sim,
+                                                                a.err, t0, t1, per, split0, a.part);
+    return cudaGetLastError();
+}
+
+// compile-time selection by k: the shortest list that holds it (insertion and
+// the k-th-value scan cost O(KMAX))
+cudaError_t knn_launch_k(const KnnArgs& a, uint32_t t0, uint32_t t1, uint32_t splits, uint32_t split0, cudaStream_t s) {
+    return a.k <= 8    ? knn_launch<8>(a, t0, t1, splits, split0, s)
+           : a.k <= 12 ? knn_launch<12>(a, t0, t1, splits, split0, s)
+           : a.k <= 16 ? knn_launch<16>(a, t0, t1, splits, split0, s)
+                       : knn_launch<32>(a, t0, t1, splits, split0, s);
 }
 
 }  // namespace
@@ -946,48 +1023,83 @@ extern "C" int ep_knn_cosine(int device, uint64_t n_db, uint32_t dims, const flo
     const uint32_t dpad = (dims + 63) / 64 * 64;
     const uint64_t q_tile_bytes = (uint64_t)(dpad / 64) * 128 * KNN_BM, db_tile_bytes = (uint64_t)(dpad / 64) * 128 * KNN_BN;
     const uint64_t db_tiles = (n_db + KNN_BN - 1) / KNN_BN, q_tiles = (n_q + KNN_BM - 1) / KNN_BM;
-    cudaStream_t s;
+    // Plan.  One CTA per 128 queries over the whole database fills the chip
+    // from about 128 query tiles on; fewer tiles split the database, so that
+    // tiles x splits come near the 152 SMs, and take it in chunks of about
+    // 32 MB, each searched while the next one is uploaded and normalised.
+    // 8,192 x 262,144 x 256, top 10 (64 CTAs, 1.89 ms of search, after a 1.5 ms
+    // upload): the call 4.25 -> 2.7 ms; 739 x 48,046 x 48, top 20: 1.31 -> 0.54.
+    const uint64_t db_bytes = n_db * dims * 4;
+    uint32_t chunks = 1, splits = 1;                   // splits per chunk
+    if (q_tiles <= 76 && db_tiles >= 8) {
+        splits = (uint32_t)std::min<uint64_t>(152 / q_tiles, db_tiles / 4);
+        chunks = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>({16, db_bytes >> 25, db_tiles / (4ull * splits)}));
+    }
+    const bool split = splits * chunks > 1;
+    const uint32_t slices = k <= 16 ? KnnRoles<16>::SLICES : KnnRoles<32>::SLICES;
+    cudaStream_t s, up;
     KCK(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking), "stream");
     struct SG { cudaStream_t s; ~SG() { cudaStreamDestroy(s); } } sg{s};
-    DevMem draw, dq, dD, dQ, dself, didx, dsim, derr;
-    const uint64_t nmax = std::max(n_db, n_q);
-    KCK(draw.alloc(nmax * dims * 4), "alloc");
-    KCK(dD.alloc(std::max<uint64_t>(db_tiles, 1) * db_tile_bytes), "alloc");
-    KCK(dQ.alloc(q_tiles * q_tile_bytes), "alloc");
-    KCK(didx.alloc(n_q * k * 4), "alloc");
-    KCK(dsim.alloc(n_q * k * 4), "alloc");
-    KCK(derr.alloc(4), "alloc");
-    KCK(cudaMemsetAsync(derr.p, 0, 4, s), "clear");
-    if (q_self) {
-        KCK(dself.alloc(n_q * 8), "alloc");
-        KCK(cudaMemcpyAsync(dself.p, q_self, n_q * 8, cudaMemcpyHostToDevice, s), "upload");
+    KCK(cudaStreamCreateWithFlags(&up, cudaStreamNonBlocking), "stream");
+    SG ug{up};
+    struct EV {
+        cudaEvent_t e = nullptr;
+        ~EV() { if (e) cudaEventDestroy(e); }
+    };
+    std::vector<EV> ready(chunks), t_from(chunks), t_to(chunks);
+    for (uint32_t c = 0; c < chunks; ++c) {
+        KCK(cudaEventCreateWithFlags(&ready[c].e, cudaEventDisableTiming), "events");
+        KCK(cudaEventCreate(&t_from[c].e), "events");
+        KCK(cudaEventCreate(&t_to[c].e), "events");
     }
-    if (n_db) {
-        KCK(cudaMemcpyAsync(draw.p, db, n_db * dims * 4, cudaMemcpyHostToDevice, s), "upload");
-        k_norm_swz<<<(unsigned)((db_tiles * KNN_BN * 32 + 255) / 256), 256, 0, s>>>(
-            n_db, db_tiles * KNN_BN, dims, dpad, 8, (const float*)draw.p, (unsigned char*)dD.p);
-        KCK(cudaGetLastError(), "normalise");
-    }
-    KCK(cudaMemcpyAsync(draw.p, q, n_q * dims * 4, cudaMemcpyHostToDevice, s), "upload");
-    k_norm_swz<<<(unsigned)((q_tiles * KNN_BM * 32 + 255) / 256), 256, 0, s>>>(n_q, q_tiles * KNN_BM, dims, dpad, 7,
-                                                                              (const float*)draw.p,
-                                                                              (unsigned char*)dQ.p);
+    Arena ar;
+    const uint64_t chunk_tiles = (db_tiles + chunks - 1) / chunks, chunk_rows = chunk_tiles * KNN_BN;
+    const size_t o_err = ar.reserve(4), o_raw = ar.reserve(std::min(n_db, chunk_rows) * dims * 4), o_qraw = ar.reserve(n_q * dims * 4),
+                 o_D = ar.reserve(std::max<uint64_t>(db_tiles, 1) * db_tile_bytes), o_Q = ar.reserve(q_tiles * q_tile_bytes),
+                 o_idx = ar.reserve(n_q * k * 4), o_sim = ar.reserve(n_q * k * 4), o_self = ar.reserve(q_self ? n_q * 8 : 0),
+                 o_part = ar.reserve(split ? (uint64_t)chunks * splits * n_q * slices * k * 8 : 0);
+    KCK(ar.mem.alloc(ar.used), "alloc");
+    KCK(cudaMemsetAsync(ar.at<void>(o_err), 0, 4, s), "clear");
+    KCK(upload(ar.at<void>(o_self), q_self, q_self ? n_q * 8 : 0, s), "upload");
+    KCK(upload(ar.at<void>(o_qraw), q, n_q * dims * 4, s), "upload");
+    k_norm_swz<<<(unsigned)((q_tiles * KNN_BM * 32 + 255) / 256), 256, 0, s>>>(0, n_q, q_tiles * KNN_BM, dims, dpad, 7,
+                                                                              ar.at<float>(o_qraw),
+                                                                              ar.at<unsigned char>(o_Q));
     KCK(cudaGetLastError(), "normalise");
-    const uint64_t* qs = q_self ? (const uint64_t*)dself.p : nullptr;
-    // the shortest list that holds k: insertion and the k-th-value scan cost O(KMAX)
-    const unsigned char *Qp = (const unsigned char*)dQ.p, *Dp = (const unsigned char*)dD.p;
-    uint32_t *ip = (uint32_t*)didx.p, *ep = (uint32_t*)derr.p;
-    float* sp = (float*)dsim.p;
-    int rc = k <= 8    ? knn_run<8>(Qp, n_q, Dp, n_db, dpad, qs, k, ip, sp, ep, s)
-             : k <= 12 ? knn_run<12>(Qp, n_q, Dp, n_db, dpad, qs, k, ip, sp, ep, s)
-             : k <= 16 ? knn_run<16>(Qp, n_q, Dp, n_db, dpad, qs, k, ip, sp, ep, s)
-                       : knn_run<32>(Qp, n_q, Dp, n_db, dpad, qs, k, ip, sp, ep, s);
-    if (rc) return rc;
+    KnnArgs a{ar.at<unsigned char>(o_Q), ar.at<unsigned char>(o_D), n_q, n_db, dpad,
+              q_self ? ar.at<uint64_t>(o_self) : nullptr, k, ar.at<uint32_t>(o_idx), ar.at<float>(o_sim),
+              ar.at<uint32_t>(o_err), split ? ar.at<uint2>(o_part) : nullptr};
+    for (uint32_t c = 0; c < chunks; ++c) {
+        const uint64_t tile0 = std::min<uint64_t>(db_tiles, c * chunk_tiles), tile1 = std::min(db_tiles, tile0 + chunk_tiles);
+        const uint64_t row0 = std::min<uint64_t>(n_db, c * chunk_rows), row1 = std::min(n_db, row0 + chunk_rows);
+        KCK(upload(ar.at<float>(o_raw), db + row0 * dims, (row1 - row0) * dims * 4, up), "upload");   // after the chunk before
+        if (tile1 > tile0)
+            k_norm_swz<<<(unsigned)((tile1 - tile0) * KNN_BN * 32 / 256), 256, 0, up>>>(
+                tile0 * KNN_BN, n_db, tile1 * KNN_BN, dims, dpad, 8, ar.at<float>(o_raw), ar.at<unsigned char>(o_D));
+        KCK(cudaGetLastError(), "normalise");
+        cudaEventRecord(ready[c].e, up);
+        cudaStreamWaitEvent(s, ready[c].e, 0);
+        cudaEventRecord(t_from[c].e, s);
+        KCK(knn_launch_k(a, (uint32_t)tile0, (uint32_t)tile1, splits, c * splits, s), "knn launch");
+        cudaEventRecord(t_to[c].e, s);
+    }
+    if (split) {
+        const uint32_t lists = chunks * splits * slices;
+        k_merge_topk<<<(unsigned)((n_q + 3) / 4), 128, 4 * (size_t)lists, s>>>(a.part, n_q, chunks * splits, slices, k, a.idx,
+                                                                             a.sim);
+        KCK(cudaGetLastError(), "knn merge");
+    }
     uint32_t herr = 0;
-    KCK(cudaMemcpyAsync(idx_out, didx.p, n_q * k * 4, cudaMemcpyDeviceToHost, s), "download");
-    KCK(cudaMemcpyAsync(sim_out, dsim.p, n_q * k * 4, cudaMemcpyDeviceToHost, s), "download");
-    KCK(cudaMemcpyAsync(&herr, derr.p, 4, cudaMemcpyDeviceToHost, s), "download");
+    ResultPages pi(idx_out, host_bytes(idx_out, n_q * k * 4)), ps(sim_out, host_bytes(sim_out, n_q * k * 4));
+    KCK(download((char*)idx_out, a.idx, n_q * k * 4, pi, s), "download");
+    KCK(download((char*)sim_out, a.sim, n_q * k * 4, ps, s), "download");
+    KCK(cudaMemcpyAsync(&herr, ar.at<void>(o_err), 4, cudaMemcpyDeviceToHost, s), "download");
     KCK(cudaStreamSynchronize(s), "knn");
+    g_knn_ms = 0.f;
+    for (uint32_t c = 0; c < chunks; ++c) {
+        float ms = 0.f;
+        if (cudaEventElapsedTime(&ms, t_from[c].e, t_to[c].e) == cudaSuccess) g_knn_ms += ms;
+    }
     if (herr) return knn_fail(EP_ERR_DEVICE, "tensor-core wait timed out");
     return EP_OK;
 }

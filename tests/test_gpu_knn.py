@@ -205,3 +205,32 @@ def test_knn_cosine_argument_limits():
     z = np.zeros((3, 8), np.float32)
     idx, sim = _native.knn_cosine(z, rng.standard_normal((2, 8)).astype(np.float32), 3)
     assert sorted(idx[0].tolist()) == [0, 1, 2] and np.allclose(sim, 0.0)
+
+
+@pytest.mark.parametrize("k", [1, 10, 32])
+@pytest.mark.parametrize("n_db,dims", [(256 * 8 - 1, 64), (256 * 9, 20), (256 * 40 + 3, 200), (140_000, 256)])
+def test_split_database_matches_the_whole(n_db, dims, k):
+    # few queries split the database over CTAs (and over upload chunks, at the
+    # largest size); 9,800 queries (77 tiles) search it in one piece.  Equal
+    # rows on both sides of every split and slice: the ids and similarities
+    # must be the same bit for bit, ties in the same order
+    rng = np.random.default_rng(n_db + k)
+    db = rng.standard_normal((n_db, dims), dtype=np.float32)
+    twin = rng.integers(0, n_db, n_db // 3)
+    db[rng.integers(0, n_db, n_db // 3)] = db[twin]                 # duplicates: exact ties
+    q = db[rng.integers(0, n_db, 9_800)]
+    whole_ids, whole_sim = _native.knn_cosine(db, q, k)
+    for n_q in (1, 130, 1_000):
+        ids, sim = _native.knn_cosine(db, q[:n_q], k)
+        assert np.array_equal(ids, whole_ids[:n_q]) and np.array_equal(sim, whole_sim[:n_q])
+
+
+def test_split_database_with_few_rows_to_find():
+    # more neighbours asked for than rows qualify: the rest of the slots empty
+    rng = np.random.default_rng(3)
+    db = np.full((256 * 8, 16), np.nan, np.float32)
+    db[[5, 700, 2040]] = rng.standard_normal((3, 16), dtype=np.float32)
+    ids, sim = _native.knn_cosine(db, db[[700, 5]], 6, q_self=np.array([700, 5], np.uint64))
+    for i, row in enumerate(ids):
+        assert set(row[:2].tolist()) == {5, 700, 2040} - {(700, 5)[i]}
+        assert (row[2:] == 0xffffffff).all() and np.isneginf(sim[i, 2:]).all()
