@@ -157,6 +157,7 @@ SIGNATURES = {
     "ep_knn_last_error": (ctypes.c_char_p, []),
     "ep_knn_last_kernel_ms": (ctypes.c_float, []),
     "ep_ag_forward": (ctypes.c_int, [_P, ctypes.POINTER(EpBatchSamples), ctypes.c_int, _P, _P, _P]),
+    "ep_ag_stage": (ctypes.c_int, [_P, ctypes.POINTER(EpBatchSamples), ctypes.c_int, _P, _P]),
     "ep_ag_backward": (ctypes.c_int, [_P, _P, _P, _P]),
     "ep_get_split": (ctypes.c_int, [_P, _P, _P, ctypes.POINTER(_U32), ctypes.POINTER(_U32)]),
     "ep_get_launch_shape": (ctypes.c_int, [_P, _P]),
@@ -371,6 +372,11 @@ class Context:
         s, keep = samples
         check(lib().ep_ag_forward(self._h, ctypes.byref(s), precision, ctypes.c_void_p(table_ptr),
                                   ctypes.c_void_p(loss_ptr), ctypes.c_void_p(stream)), self._h, "ep_ag_forward")
+
+    def ag_stage(self, samples, precision, table_ptr, stream):
+        s, keep = samples
+        check(lib().ep_ag_stage(self._h, ctypes.byref(s), precision, ctypes.c_void_p(table_ptr), ctypes.c_void_p(stream)),
+              self._h, "ep_ag_stage")
 
     def ag_backward(self, dloss_ptr, grad_ptr, stream):
         check(lib().ep_ag_backward(self._h, ctypes.c_void_p(dloss_ptr), ctypes.c_void_p(grad_ptr),

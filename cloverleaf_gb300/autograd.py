@@ -43,8 +43,7 @@ class _Fn(torch.autograd.Function):
         stream = torch.cuda.current_stream(table.device).cuda_stream
         owner = ctx.owner
         # re-stage this batch (another call may have used the context since)
-        owner.ctx.ag_forward(ctx.samples, ctx.precision, table.data_ptr(),
-                             torch.empty_like(dloss).data_ptr(), stream)
+        owner.ctx.ag_stage(ctx.samples, ctx.precision, table.data_ptr(), stream)
         owner.ctx.ag_backward(dloss.data_ptr(), grad.data_ptr(), stream)
         return grad, None, None
 

@@ -133,6 +133,12 @@ struct ep_ctx {
     uint32_t* sorted_keys = nullptr;
     uint2* sorted_vals = nullptr;
     BatchState* h_st = nullptr;   // pinned mirror
+    BatchState* h_inj = nullptr;  // pinned state of explicit-sample runs
+    // explicit samples, packed by the host for one copy
+    uint32_t* h_pack = nullptr;
+    size_t h_pack_words = 0;
+    DevBuf pack;
+    cudaEvent_t ev_pack = nullptr;   // that copy is done
 
     // host-side view of the pass sequence (mirrors the device BatchState)
     uint32_t host_pass = 1, host_batch = 0;
@@ -149,7 +155,9 @@ struct ep_ctx {
         if (gexec) cudaGraphExecDestroy(gexec);
         if (gexec_run) cudaGraphExecDestroy(gexec_run);
         for (auto& kv : gexec_rem) cudaGraphExecDestroy(kv.second);
-        if (h_st) cudaFreeHost(h_st);
+        if (h_st) cudaFreeHost(h_st);   // with h_inj
+        if (h_pack) cudaFreeHost(h_pack);
+        if (ev_pack) cudaEventDestroy(ev_pack);
         if (ev_fork) cudaEventDestroy(ev_fork);
         if (ev_join) cudaEventDestroy(ev_join);
         if (ev_loss) cudaEventDestroy(ev_loss);
@@ -269,11 +277,13 @@ extern "C" int ep_create(const ep_config* cfg, ep_ctx** out) {
         cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_loss, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_sorted, cudaEventDisableTiming) != cudaSuccess ||
-        cudaMallocHost((void**)&c->h_st, sizeof(BatchState)) != cudaSuccess || reduce_kernels_setup() != cudaSuccess) {
+        cudaEventCreateWithFlags(&c->ev_pack, cudaEventDisableTiming) != cudaSuccess ||
+        cudaMallocHost((void**)&c->h_st, 2 * sizeof(BatchState)) != cudaSuccess || reduce_kernels_setup() != cudaSuccess) {
         g_create_err = std::string("CUDA setup failed: ") + cudaGetErrorString(cudaGetLastError());
         delete c;
         return EP_ERR_CUDA;
     }
+    c->h_inj = c->h_st + 1;
     c->dims = cfg->dims;
     c->vpl = pick_vpl(cfg->dims);
     c->dpad = ((cfg->dims + c->vpl - 1) / c->vpl) * c->vpl;
@@ -831,12 +841,14 @@ static void issue_forward(int tt, int vpl, const ForwardParams& fp, uint32_t cap
 }
 
 // Sort the emitted items and reduce them; tt selects the kernel family.
-static void sort_and_reduce(ep_ctx* c, BatchState* st, int tt, int out_mode, void* table, cudaStream_t s) {
+static void sort_and_reduce(ep_ctx* c, BatchState* st, int tt, int out_mode, void* table, cudaStream_t s,
+                            void* gdense) {
     launch_radix_sort(st, c->item_f.as<uint32_t>(), c->key_alt.as<uint32_t>(), c->item_src.as<uint32_t>(),
                       c->item_c.as<float>(), c->idx.as<uint2>(), c->idx_alt.as<uint2>(), c->hist.as<uint32_t>(),
                       c->items_cap, (int)bits_for(c->n_feat), &c->sorted_keys, &c->sorted_vals, s);
     if (out_mode == OUT_DENSE) cudaMemsetAsync(c->n_touched.p, 0, 4, s);
     ReduceParams rp = reduce_params(c, st, out_mode, table);
+    if (gdense) rp.gdense = gdense;
     launch_reduce(tt, (int)c->vpl, rp, c->items_cap, s);
     launch_fixup(tt, (int)c->vpl, rp, c->items_cap, s);
 }
@@ -1380,6 +1392,31 @@ extern "C" int ep_synchronize(ep_ctx* c) {
 // ---------------------------------------------------------------------------
 // Explicit-sample paths (parity hooks and the autograd binding)
 // ---------------------------------------------------------------------------
+// The samples of a batch as the host packs them, back to back (32-bit words):
+// anchors [B], neighbour offsets [B + 1], neighbours [nn], their weights [nn],
+// negatives [B * R].  One warp per anchor spreads them over the batch's slots.
+__global__ void __launch_bounds__(256) k_stage_samples(const uint32_t* __restrict__ pack, uint32_t B, uint32_t nn, uint32_t R,
+                                                       uint32_t Ks, uint32_t* __restrict__ anchors,
+                                                       uint32_t* __restrict__ nbr, float* __restrict__ nbr_w,
+                                                       uint32_t* __restrict__ nbr_cnt, uint32_t* __restrict__ neg) {
+    const uint32_t lane = threadIdx.x & 31u, a = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (a >= B) return;
+    const uint32_t* ptr = pack + B;
+    const uint32_t* ids = ptr + B + 1;
+    const uint32_t* w = ids + nn;
+    const uint32_t* ng = w + nn;
+    const uint32_t b = ptr[a], n = ptr[a + 1] - b;
+    if (lane == 0) {
+        anchors[a] = pack[a];
+        nbr_cnt[a] = n;
+    }
+    for (uint32_t j = lane; j < n; j += 32) {
+        nbr[(uint64_t)a * Ks + j] = ids[b + j];
+        nbr_w[(uint64_t)a * Ks + j] = __uint_as_float(w[b + j]);
+    }
+    for (uint32_t j = lane; j < R; j += 32) neg[(uint64_t)a * R + j] = ng[(uint64_t)a * R + j];
+}
+
 static int stage_samples(ep_ctx* c, const ep_batch_samples* sm, uint32_t es, cudaStream_t s) {
     if (!sm || !sm->anchors || !sm->nbr_ptr || !sm->negatives) return c->fail(EP_ERR_INVALID_ARG, "null sample arrays");
     if (!c->graph_ok || !c->feats_ok) return c->fail(EP_ERR_STATE, "upload the graph and the features first");
@@ -1391,39 +1428,55 @@ static int stage_samples(ep_ctx* c, const ep_batch_samples* sm, uint32_t es, cud
         K = std::max(K, sm->nbr_ptr[a + 1] - sm->nbr_ptr[a]);
         if (sm->anchors[a] >= c->n_nodes) return c->fail(EP_ERR_INVALID_ARG, "anchor id out of range");
     }
-    const uint32_t nn = sm->nbr_ptr[B];
-    if (nn && (!sm->nbr || !sm->nbr_w)) return c->fail(EP_ERR_INVALID_ARG, "null neighbour arrays");
-    for (uint32_t j = 0; j < nn; ++j)
-        if (sm->nbr[j] >= c->n_nodes) return c->fail(EP_ERR_INVALID_ARG, "neighbour id out of range");
-    for (uint64_t j = 0; j < (uint64_t)B * c->R; ++j)
-        if (sm->negatives[j] >= c->n_nodes) return c->fail(EP_ERR_INVALID_ARG, "negative id out of range");
+    // neighbours are those of [nbr_ptr[0], nbr_ptr[B]); offsets are packed from 0
+    const uint32_t n0 = sm->nbr_ptr[0], nn = sm->nbr_ptr[B] - n0;
+    if (sm->nbr_ptr[B] && (!sm->nbr || !sm->nbr_w)) return c->fail(EP_ERR_INVALID_ARG, "null neighbour arrays");
+    if (!all_below(sm->nbr, sm->nbr_ptr[B], c->n_nodes)) return c->fail(EP_ERR_INVALID_ARG, "neighbour id out of range");
+    if (!all_below(sm->negatives, (uint64_t)B * c->R, c->n_nodes))
+        return c->fail(EP_ERR_INVALID_ARG, "negative id out of range");
     const uint64_t items = (uint64_t)B * c->max_feat * (1ull + c->R + K);
     c->typ_items = (uint64_t)((double)c->n_fids / (double)c->n_nodes * ((double)B * (1. + c->R) + nn));
     int rc = ensure_bufs(c, B, K, items, es, true);
     if (rc) return rc;
-    const uint32_t Ks = c->buf_K;
-    std::vector<uint32_t> nb((size_t)B * Ks, 0u), cnt(B);
-    std::vector<float> nw((size_t)B * Ks, 0.f);
-    for (uint32_t a = 0; a < B; ++a) {
-        cnt[a] = sm->nbr_ptr[a + 1] - sm->nbr_ptr[a];
-        for (uint32_t j = 0; j < cnt[a]; ++j) {
-            nb[(size_t)a * Ks + j] = sm->nbr[sm->nbr_ptr[a] + j];
-            nw[(size_t)a * Ks + j] = sm->nbr_w[sm->nbr_ptr[a] + j];
-        }
+    // one page-locked copy of everything
+    const size_t words = 2 * (size_t)B + 1 + 2 * (size_t)nn + (size_t)B * c->R;
+    if (c->h_pack_words < words) {
+        if (c->h_pack) cudaFreeHost(c->h_pack);
+        c->h_pack = nullptr;
+        c->h_pack_words = 0;
+        CK(cudaMallocHost((void**)&c->h_pack, 2 * words * 4), "staging memory");
+        c->h_pack_words = 2 * words;
+    } else {
+        CK(cudaEventSynchronize(c->ev_pack), "staging memory");      // the last copy from it
     }
-    CK(cudaMemcpyAsync(c->anchors.p, sm->anchors, (size_t)B * 4, cudaMemcpyHostToDevice, s), "stage anchors");
-    CK(cudaMemcpyAsync(c->nbr.p, nb.data(), nb.size() * 4, cudaMemcpyHostToDevice, s), "stage neighbours");
-    CK(cudaMemcpyAsync(c->nbr_w.p, nw.data(), nw.size() * 4, cudaMemcpyHostToDevice, s), "stage weights");
-    CK(cudaMemcpyAsync(c->nbr_cnt.p, cnt.data(), (size_t)B * 4, cudaMemcpyHostToDevice, s), "stage counts");
-    CK(cudaMemcpyAsync(c->neg.p, sm->negatives, (size_t)B * c->R * 4, cudaMemcpyHostToDevice, s), "stage negatives");
-    CK(cudaStreamSynchronize(s), "stage samples");   // host vectors go out of scope
+    if (!c->pack.ensure(words * 4)) return c->fail(EP_ERR_OOM, "staging allocation failed");
+    uint32_t* p = c->h_pack;
+    memcpy(p, sm->anchors, (size_t)B * 4);
+    p += B;
+    for (uint32_t a = 0; a <= B; ++a) p[a] = sm->nbr_ptr[a] - n0;
+    p += B + 1;
+    if (nn) {
+        memcpy(p, sm->nbr + n0, (size_t)nn * 4);
+        memcpy(p + nn, sm->nbr_w + n0, (size_t)nn * 4);
+    }
+    memcpy(p + 2 * (size_t)nn, sm->negatives, (size_t)B * c->R * 4);
+    CK(cudaMemcpyAsync(c->pack.p, c->h_pack, words * 4, cudaMemcpyHostToDevice, s), "stage samples");
+    CK(cudaEventRecord(c->ev_pack, s), "stage samples");
+    k_stage_samples<<<(B + 7) / 8, 256, 0, s>>>(c->pack.as<uint32_t>(), B, nn, c->R, c->buf_K, c->anchors.as<uint32_t>(),
+                                                c->nbr.as<uint32_t>(), c->nbr_w.as<float>(), c->nbr_cnt.as<uint32_t>(),
+                                                c->neg.as<uint32_t>());
+    CK(cudaGetLastError(), "stage samples");
     return EP_OK;
 }
 
-// Runs count -> scan -> forward -> sort -> reduce for staged samples.
+// Runs count -> scan -> forward -> sort -> reduce for staged samples; without
+// `reduce` the losses only (count -> forward).  gdense: where OUT_DENSE's rows
+// go (null: the context's buffer).
 static int run_injected(ep_ctx* c, uint32_t B, int tt, const void* table, void* loss_out, const void* dloss,
-                        int out_mode, void* adam_table, float lr, uint32_t pass, cudaStream_t s) {
-    BatchState h{};
+                        int out_mode, void* adam_table, float lr, uint32_t pass, cudaStream_t s, bool reduce = true,
+                        void* gdense = nullptr) {
+    BatchState& h = *c->h_inj;      // page-locked; every run ends with a wait
+    h = BatchState{};
     h.pass = pass;
     h.step = 1;
     h.n_anchors = B;
@@ -1431,23 +1484,25 @@ static int run_injected(ep_ctx* c, uint32_t B, int tt, const void* table, void* 
     h.bc1 = 1.f - powf(0.9f, (float)pass + 1.f);
     h.bc2 = 1.f - powf(0.999f, (float)pass + 1.f);
     h.noise_sigma = c->cfg.noise > 1e-9f ? c->cfg.noise : 0.f;   // injected steps: the configured scale
-    BatchState* st = c->st_inj.as<BatchState>();
     if (!c->st_inj.ensure(sizeof(BatchState))) return c->fail(EP_ERR_OOM, "state allocation failed");
-    st = c->st_inj.as<BatchState>();
+    BatchState* st = c->st_inj.as<BatchState>();
     CK(cudaMemcpyAsync(st, &h, sizeof(h), cudaMemcpyHostToDevice, s), "inject state");
     SampleParams sp = sample_params(c, st, false, true);
+    sp.batch_cap = B;
     launch_sample(sp, s);
-    launch_scan_occ(st, c->occ.as<uint32_t>(), B, c->items_cap, s);
-    ForwardParams fp = forward_params(c, st, table, true, false);
+    if (reduce) launch_scan_occ(st, c->occ.as<uint32_t>(), B, c->items_cap, s);
+    ForwardParams fp = forward_params(c, st, table, reduce, false);
     fp.loss_out = loss_out;
     fp.dloss = (const float*)dloss;
     fp.dloss_f64 = tt == TT_F64;
     issue_forward(tt, (int)c->vpl, fp, B, s);
-    sort_and_reduce(c, st, tt, out_mode, adam_table, s);
-    if (out_mode == OUT_DENSE && adam_table)
-        launch_adam_dense(tt, (int)c->vpl, st, adam_table, c->m.as<float>(), c->v.as<float>(), c->gdense.as<float>(),
-                          c->touched.as<uint32_t>(), c->n_touched.as<uint32_t>(), c->dpad,
-                          (uint32_t)std::min<uint64_t>(c->n_feat, c->items_cap), c->cfg.seed, s);
+    if (reduce) {
+        sort_and_reduce(c, st, tt, out_mode, adam_table, s, gdense);
+        if (out_mode == OUT_DENSE && adam_table)
+            launch_adam_dense(tt, (int)c->vpl, st, adam_table, c->m.as<float>(), c->v.as<float>(), c->gdense.as<float>(),
+                              c->touched.as<uint32_t>(), c->n_touched.as<uint32_t>(), c->dpad,
+                              (uint32_t)std::min<uint64_t>(c->n_feat, c->items_cap), c->cfg.seed, s);
+    }
     CK(cudaGetLastError(), "injected batch launch");
     CK(cudaMemcpyAsync(&h, st, sizeof(h), cudaMemcpyDeviceToHost, s), "read state");
     CK(cudaStreamSynchronize(s), "injected batch");
@@ -1634,8 +1689,15 @@ extern "C" int ep_ag_forward(ep_ctx* c, const ep_batch_samples* sm, int precisio
     cudaStream_t s = stream ? (cudaStream_t)stream : c->stream;
     int rc = ag_prepare(c, sm, precision, table_dev, s);
     if (rc) return rc;
+    // the losses alone: items, sort and reduction belong to the backward
     return run_injected(c, c->ag_n, precision ? TT_F64 : TT_F32, c->ag_table_ptr, loss_dev, nullptr, OUT_DENSE, nullptr, 0.f,
-                        1, s);
+                        1, s, false);
+}
+
+extern "C" int ep_ag_stage(ep_ctx* c, const ep_batch_samples* sm, int precision, const void* table_dev, void* stream) {
+    if (!c || !table_dev) return c ? c->fail(EP_ERR_INVALID_ARG, "null pointer") : EP_ERR_INVALID_ARG;
+    cudaSetDevice(c->device);
+    return ag_prepare(c, sm, precision, table_dev, stream ? (cudaStream_t)stream : c->stream);
 }
 
 extern "C" int ep_ag_backward(ep_ctx* c, const void* dloss_dev, void* grad_dev, void* stream) {
@@ -1645,9 +1707,12 @@ extern "C" int ep_ag_backward(ep_ctx* c, const void* dloss_dev, void* grad_dev, 
     cudaStream_t s = stream ? (cudaStream_t)stream : c->stream;
     const int tt = c->ag_precision ? TT_F64 : TT_F32;
     const size_t es = c->ag_precision ? 8 : 4;
-    int rc = run_injected(c, c->ag_n, tt, c->ag_table_ptr, c->loss.p, dloss_dev, OUT_DENSE, nullptr, 0.f, 1, s);
-    if (rc) return rc;
     CK(cudaMemsetAsync(grad_dev, 0, (size_t)c->n_feat * c->dims * es, s), "clear gradient");
+    // unpadded rows: the reduction writes the touched rows in place
+    const bool direct = c->dims == c->dpad && ((uintptr_t)grad_dev % 16) == 0;
+    int rc = run_injected(c, c->ag_n, tt, c->ag_table_ptr, c->loss.p, dloss_dev, OUT_DENSE, nullptr, 0.f, 1, s, true,
+                          direct ? grad_dev : nullptr);
+    if (rc || direct) return rc;
     launch_pack_rows(es, c->gdense.p, c->touched.as<uint32_t>(), c->n_touched.as<uint32_t>(), c->dpad, c->dims, grad_dev, 1,
                      (uint32_t)std::min<uint64_t>(c->n_feat, c->items_cap), s);
     CK(cudaGetLastError(), "gradient scatter");

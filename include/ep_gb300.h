@@ -291,10 +291,15 @@ int ep_get_table_static(ep_ctx* ctx, uint64_t first_row, uint64_t n_rows, float*
  * ep_ag_forward computes per-anchor losses (loss_dev, n_anchors values of the
  * precision) for explicit samples against table_dev (n_feat*dims);
  * ep_ag_backward consumes dloss_dev (n_anchors values) and writes the dense
- * gradient dL/dtable into grad_dev (n_feat*dims, overwritten).  Both run on
- * `stream` (a cudaStream_t, NULL = the context stream). */
+ * gradient dL/dtable into grad_dev (n_feat*dims, overwritten), for the samples
+ * and the table of the context's last ep_ag_forward or ep_ag_stage, which
+ * must still be there.  ep_ag_stage sets these without computing the losses
+ * (a backward that comes after other calls on the context).  All run on
+ * `stream` (a cudaStream_t, NULL = the context stream); ep_ag_stage does not
+ * wait for it, so the backward after it takes the same stream. */
 int ep_ag_forward(ep_ctx* ctx, const ep_batch_samples* samples, int precision,
                   const void* table_dev, void* loss_dev, void* stream);
+int ep_ag_stage(ep_ctx* ctx, const ep_batch_samples* samples, int precision, const void* table_dev, void* stream);
 int ep_ag_backward(ep_ctx* ctx, const void* dloss_dev, void* grad_dev, void* stream);
 
 /* Self-check (no counterpart in the reference): rounds n element pairs
