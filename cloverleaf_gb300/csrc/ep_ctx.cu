@@ -71,7 +71,7 @@ struct ep_ctx {
     // second branch: a batch's fix-ups beside the next batch's sampling
     cudaStream_t fix = nullptr;
     cudaStream_t fix2 = nullptr;   // the long spans' fix-ups, beside the short ones on `fix`
-    cudaEvent_t ev_red = nullptr, ev_fix = nullptr, ev_fix2 = nullptr, ev_direct = nullptr;
+    cudaEvent_t ev_red = nullptr, ev_fix = nullptr, ev_fix2 = nullptr, ev_direct = nullptr, ev_start = nullptr, ev_adam = nullptr;
     bool fix_pending = false;   // the last issued fix-ups have not been joined yet
     std::string err;
 
@@ -97,6 +97,7 @@ struct ep_ctx {
     uint64_t items_cap = 0;
     uint64_t typ_items = 0;   // items the batches in flight are expected to emit (launch shapes only)
     uint64_t train_items = 0; // the same of a training batch
+    uint32_t train_K = 0, inj_K = 0;   // most neighbours of a training anchor / of the staged samples
     uint32_t buf_B = 0, buf_K = 0, buf_es = 0;
     uint32_t chunk = 128;
     // FUSED form's Adam placement: 0 = by the reducing warp as each feature
@@ -166,6 +167,8 @@ struct ep_ctx {
         if (ev_fix) cudaEventDestroy(ev_fix);
         if (ev_fix2) cudaEventDestroy(ev_fix2);
         if (ev_direct) cudaEventDestroy(ev_direct);
+        if (ev_start) cudaEventDestroy(ev_start);
+        if (ev_adam) cudaEventDestroy(ev_adam);
         if (fix) cudaStreamDestroy(fix);
         if (fix2) cudaStreamDestroy(fix2);
         if (side) cudaStreamDestroy(side);
@@ -272,6 +275,8 @@ extern "C" int ep_create(const ep_config* cfg, ep_ctx** out) {
         cudaEventCreateWithFlags(&c->ev_red, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_fix, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_fix2, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&c->ev_start, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&c->ev_adam, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_direct, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming) != cudaSuccess ||
@@ -691,6 +696,7 @@ static int prepare_train(ep_ctx* c) {
     c->chunk = chunk;
     if (rc) return rc;
     c->Bcap = B;
+    c->train_K = K;
     c->Kcap = c->buf_K;
     if (!c->graph_batches_set) c->graph_batches = pick_graph_batches(c->steps_per_pass, c->cfg.passes);
     c->prepared = true;
@@ -745,6 +751,12 @@ static SampleParams sample_params(ep_ctx* c, BatchState* st, bool eval, int inje
     sp.sample_warps = c->sample_warps;
     sp.injected = injected;
     sp.eval = eval;
+    sp.begin = !injected;
+    sp.total_steps = eval ? 1 : c->total_steps;
+    sp.warmup = eval ? 0 : c->warmup;
+    sp.alpha = c->cfg.alpha;
+    sp.noise = eval ? 0.f : c->cfg.noise;
+    sp.noise_decay = eval ? 1.f : noise_decay(c);
     sp.feistel_half = feistel_half(sp.n_order);
     sp.anchors = c->anchors.as<uint32_t>();
     sp.nbr = c->nbr.as<uint32_t>();
@@ -835,9 +847,18 @@ static ReduceParams reduce_params(ep_ctx* c, BatchState* st, int out_mode, void*
     return rp;
 }
 
+// Whether an anchor of up to K neighbours may exceed the staged gather's
+// tables, by the longest feature list.
+static bool may_defer(const ep_ctx* c, uint64_t K) {
+    const uint64_t nodes = 1 + K + c->R;
+    return nodes > NODE_CAP || nodes * c->max_feat > OCC_CAP || c->R + 2 > ROLE_CAP || c->n_fids > 0xffffffffull;
+}
+
 // The forward kernels in order on one stream.
-static void issue_forward(int tt, int vpl, const ForwardParams& fp, uint32_t cap, cudaStream_t s) {
-    for (int part : {FWD_GATHER, FWD_DIRECT, FWD_LOSS}) launch_forward(tt, vpl, fp, cap, s, part);
+static void issue_forward(int tt, int vpl, const ForwardParams& fp, uint32_t cap, bool direct, cudaStream_t s) {
+    launch_forward(tt, vpl, fp, cap, s, FWD_GATHER);
+    if (direct) launch_forward(tt, vpl, fp, cap, s, FWD_DIRECT);
+    launch_forward(tt, vpl, fp, cap, s, FWD_LOSS);
 }
 
 // Sort the emitted items and reduce them; tt selects the kernel family.
@@ -845,7 +866,7 @@ static void sort_and_reduce(ep_ctx* c, BatchState* st, int tt, int out_mode, voi
                             void* gdense) {
     launch_radix_sort(st, c->item_f.as<uint32_t>(), c->key_alt.as<uint32_t>(), c->item_src.as<uint32_t>(),
                       c->item_c.as<float>(), c->idx.as<uint2>(), c->idx_alt.as<uint2>(), c->hist.as<uint32_t>(),
-                      c->items_cap, (int)bits_for(c->n_feat), &c->sorted_keys, &c->sorted_vals, s);
+                      c->items_cap, (int)bits_for(c->n_feat), false, &c->sorted_keys, &c->sorted_vals, s);
     if (out_mode == OUT_DENSE) cudaMemsetAsync(c->n_touched.p, 0, 4, s);
     ReduceParams rp = reduce_params(c, st, out_mode, table);
     if (gdense) rp.gdense = gdense;
@@ -862,11 +883,14 @@ static int fused_out_mode(const ep_ctx* c) {
     return c->fused_mode == 2 ? OUT_QUEUE : OUT_ADAM;
 }
 
+// Whether replayed batches sort by one kernel per pass (k_radix_pass).
+static bool one_kernel_sort(const ep_ctx* c) { return c->train_items <= RADIX_ONE_ITEMS; }
+
 // Kernels launched per training batch.
 static uint32_t kernels_per_batch(const ep_ctx* c, bool fork) {
     const uint32_t b = bits_for(c->n_feat);
-    const uint32_t radix = 3 * (b ? (b + 7) / 8 : 1);
-    return 3 /* begin, sample, scan */ + 3 /* forward: staged, direct gather; loss */ + (fork ? 1 : 0) /* emit */ + radix +
+    const uint32_t radix = (fork && one_kernel_sort(c) ? 1 : 3) * (b ? (b + 7) / 8 : 1);
+    return 2 /* sample, scan */ + 2 /* gather, loss */ + (may_defer(c, c->train_K) ? 1 : 0) /* direct gather */ + (fork ? 1 : 0) /* emit */ + radix +
            3 /* reduce, fixup x2 */ +
            (c->cfg.form == EP_FORM_PLAIN_FP32 || c->fused_mode == 1 ? 1 : 0) + 1 /* end */;
 }
@@ -877,17 +901,25 @@ static uint32_t kernels_per_batch(const ep_ctx* c, bool fork) {
 // sorted on the side stream beside the gathers and the loss (which then skip
 // the emission and read neither), and k_batch_end follows the loss there; the
 // reduction waits for the sorted items.  The fix-ups run on the fix stream
-// beside the next batch's k_batch_begin, sampler and scan (which read neither
+// beside the next batch's sampler and scan (which read neither
 // the table nor what the fix-ups read: those use k_reduce's copy of the item
 // count and Adam constants), and that batch's gathers and item emission wait
 // for them; the last batch of a capture (last) joins its fix-ups before it
-// ends.
+// ends.  The dense Adam kernel (PLAIN form) follows the fix-ups on their
+// stream: it too reads the copies, and the next batch's gathers wait for it.
 static void issue_train_batch(ep_ctx* c, cudaEvent_t* ev = nullptr, bool fork = false, bool last = true) {
     BatchState* st = c->st.as<BatchState>();
     cudaStream_t s = c->stream;
     const bool plain = c->cfg.form == EP_FORM_PLAIN_FP32 || c->fused_mode == 1;
-    launch_batch_begin(st, c->n_train, c->Bcap, c->steps_per_pass, c->total_steps, c->warmup, c->cfg.alpha, 0,
-                       c->cfg.noise, noise_decay(c), s);
+    // one-kernel sort passes, counted by the emission (small batches)
+    const bool counted = fork && one_kernel_sort(c);
+    if (counted) {
+        // the counts are cleared while the batch is sampled; the last batch's
+        // sort, on the same stream, is done with them
+        cudaEventRecord(c->ev_start, s);
+        cudaStreamWaitEvent(c->side, c->ev_start, 0);
+        radix_clear(c->hist.as<uint32_t>(), c->items_cap, (int)bits_for(c->n_feat), c->side);
+    }
     SampleParams sp = sample_params(c, st, false, false);
     launch_sample(sp, s);
     if (!fork) launch_scan_occ(st, c->occ.as<uint32_t>(), c->Bcap, c->items_cap, s);
@@ -898,31 +930,39 @@ static void issue_train_batch(ep_ctx* c, cudaEvent_t* ev = nullptr, bool fork = 
         // which run with emission off and read neither; then k_batch_end
         cudaEventRecord(c->ev_fork, s);
         cudaStreamWaitEvent(c->side, c->ev_fork, 0);
-        if (plain) cudaMemsetAsync(c->n_touched.p, 0, 4, c->side);   // the last batch's Adam kernel has read it
         launch_scan_occ(st, c->occ.as<uint32_t>(), c->Bcap, c->items_cap, c->side);
-        if (c->fix_pending) {   // the previous batch's fix-ups: the table, and the sorted items they read
-            cudaStreamWaitEvent(s, c->ev_fix, 0);
+        if (c->fix_pending) {
+            // the previous batch's fix-ups and Adam step: the table (gathers),
+            // and the sorted items that the fix-ups read (emission)
+            cudaEvent_t table_done = plain ? c->ev_adam : c->ev_fix;
+            cudaStreamWaitEvent(s, table_done, 0);
             cudaStreamWaitEvent(s, c->ev_fix2, 0);
             cudaStreamWaitEvent(c->side, c->ev_fix, 0);
             cudaStreamWaitEvent(c->side, c->ev_fix2, 0);
-            cudaStreamWaitEvent(c->fix2, c->ev_fix, 0);
+            cudaStreamWaitEvent(c->fix2, table_done, 0);
             c->fix_pending = false;
+        } else if (plain) {
+            cudaMemsetAsync(c->n_touched.p, 0, 4, c->side);
         }
         ForwardParams fe = forward_params(c, st, c->table.p, true, false);
+        if (counted) fe.hist = c->hist.as<uint32_t>();
         launch_emit(fe, c->Bcap, c->side);
         launch_radix_sort(st, c->item_f.as<uint32_t>(), c->key_alt.as<uint32_t>(), c->item_src.as<uint32_t>(),
                           c->item_c.as<float>(), c->idx.as<uint2>(), c->idx_alt.as<uint2>(), c->hist.as<uint32_t>(),
-                          c->items_cap, (int)bits_for(c->n_feat), &c->sorted_keys, &c->sorted_vals, c->side);
+                          c->items_cap, (int)bits_for(c->n_feat), counted, &c->sorted_keys, &c->sorted_vals, c->side);
         cudaEventRecord(c->ev_sorted, c->side);
         ForwardParams fp = forward_params(c, st, c->table.p, false, false);
         fp.means_dead = 1;
         // the direct gathers beside the staged ones, on the long fix-ups'
         // stream (behind the previous batch's fix-ups: they update the table)
-        cudaStreamWaitEvent(c->fix2, c->ev_fork, 0);
-        launch_forward(c->tt, (int)c->vpl, fp, c->Bcap, c->fix2, FWD_DIRECT);
-        cudaEventRecord(c->ev_direct, c->fix2);
+        const bool direct = may_defer(c, c->train_K);
+        if (direct) {
+            cudaStreamWaitEvent(c->fix2, c->ev_fork, 0);
+            launch_forward(c->tt, (int)c->vpl, fp, c->Bcap, c->fix2, FWD_DIRECT);
+            cudaEventRecord(c->ev_direct, c->fix2);
+        }
         launch_forward(c->tt, (int)c->vpl, fp, c->Bcap, s, FWD_GATHER);
-        cudaStreamWaitEvent(s, c->ev_direct, 0);
+        if (direct) cudaStreamWaitEvent(s, c->ev_direct, 0);
         launch_forward(c->tt, (int)c->vpl, fp, c->Bcap, s, FWD_LOSS);
         cudaEventRecord(c->ev_loss, s);
         cudaStreamWaitEvent(c->side, c->ev_loss, 0);
@@ -933,11 +973,11 @@ static void issue_train_batch(ep_ctx* c, cudaEvent_t* ev = nullptr, bool fork = 
     } else {
         ForwardParams fp = forward_params(c, st, c->table.p, true, false);
         fp.means_dead = 1;
-        issue_forward(c->tt, (int)c->vpl, fp, c->Bcap, s);
+        issue_forward(c->tt, (int)c->vpl, fp, c->Bcap, may_defer(c, c->train_K), s);
         if (ev) cudaEventRecord(ev[EP_STAGE_FORWARD], s);
         launch_radix_sort(st, c->item_f.as<uint32_t>(), c->key_alt.as<uint32_t>(), c->item_src.as<uint32_t>(),
                           c->item_c.as<float>(), c->idx.as<uint2>(), c->idx_alt.as<uint2>(), c->hist.as<uint32_t>(),
-                          c->items_cap, (int)bits_for(c->n_feat), &c->sorted_keys, &c->sorted_vals, s);
+                          c->items_cap, (int)bits_for(c->n_feat), false, &c->sorted_keys, &c->sorted_vals, s);
         if (ev) cudaEventRecord(ev[EP_STAGE_SORT], s);
     }
     if (plain && !fork) cudaMemsetAsync(c->n_touched.p, 0, 4, s);
@@ -945,17 +985,29 @@ static void issue_train_batch(ep_ctx* c, cudaEvent_t* ev = nullptr, bool fork = 
     ReduceParams rp = reduce_params(c, st, plain ? OUT_DENSE : fused_out_mode(c), c->table.p);
     launch_reduce(c->tt, (int)c->vpl, rp, c->items_cap, s);
     if (ev) cudaEventRecord(ev[EP_STAGE_REDUCE], s);
-    if (fork && !plain) {
+    const auto adam_dense = [&](cudaStream_t on) {
+        launch_adam_dense(c->tt, (int)c->vpl, st, c->table.p, c->m.as<float>(), c->v.as<float>(), c->gdense.as<float>(),
+                          c->touched.as<uint32_t>(), c->n_touched.as<uint32_t>(), c->dpad,
+                          (uint32_t)std::min<uint64_t>(c->n_feat, c->items_cap), c->cfg.seed, on);
+    };
+    if (fork) {
         cudaEventRecord(c->ev_red, s);
         cudaStreamWaitEvent(c->fix, c->ev_red, 0);
         cudaStreamWaitEvent(c->fix2, c->ev_red, 0);
         launch_fixup(c->tt, (int)c->vpl, rp, c->items_cap, c->fix, 1);    // short spans
         launch_fixup(c->tt, (int)c->vpl, rp, c->items_cap, c->fix2, 2);   // long spans, beside them
-        cudaEventRecord(c->ev_fix, c->fix);
         cudaEventRecord(c->ev_fix2, c->fix2);
+        cudaEventRecord(c->ev_fix, c->fix);
+        if (plain) {
+            cudaStreamWaitEvent(c->fix, c->ev_fix2, 0);
+            adam_dense(c->fix);
+            if (!last) cudaMemsetAsync(c->n_touched.p, 0, 4, c->fix);   // for the next batch
+            cudaEventRecord(c->ev_adam, c->fix);
+        }
         if (last) {
             cudaStreamWaitEvent(s, c->ev_fix, 0);
             cudaStreamWaitEvent(s, c->ev_fix2, 0);
+            if (plain) cudaStreamWaitEvent(s, c->ev_adam, 0);
         } else {
             c->fix_pending = true;
         }
@@ -969,10 +1021,7 @@ static void issue_train_batch(ep_ctx* c, cudaEvent_t* ev = nullptr, bool fork = 
         cudaStreamWaitEvent(s, c->ev_fix2, 0);
     }
     if (ev) cudaEventRecord(ev[EP_STAGE_FIXUP], s);
-    if (plain)
-        launch_adam_dense(c->tt, (int)c->vpl, st, c->table.p, c->m.as<float>(), c->v.as<float>(), c->gdense.as<float>(),
-                          c->touched.as<uint32_t>(), c->n_touched.as<uint32_t>(), c->dpad,
-                          (uint32_t)std::min<uint64_t>(c->n_feat, c->items_cap), c->cfg.seed, s);
+    if (plain && !fork) adam_dense(s);
     if (ev) cudaEventRecord(ev[EP_STAGE_ADAM], s);
     if (fork) cudaStreamWaitEvent(s, c->ev_join, 0);
     else launch_batch_end(st, c->loss.p, c->status.as<int32_t>(), c->nbr_cnt.as<uint32_t>(), c->Bcap, c->steps_per_pass, 0, 0, s);
@@ -1247,11 +1296,10 @@ static int run_validation(ep_ctx* c, double* mean_out) {
     CK(cudaMemcpyAsync(st, &h, sizeof(h), cudaMemcpyHostToDevice, c->stream), "eval state");
     const uint32_t nb = (c->n_valid + c->Bcap - 1) / c->Bcap;
     for (uint32_t b = 0; b < nb; ++b) {
-        launch_batch_begin(st, c->n_valid, c->Bcap, nb, 1, 0, c->cfg.alpha, 0, 0.f, 1.f, c->stream);
         SampleParams sp = sample_params(c, st, true, false);
         launch_sample(sp, c->stream);
         ForwardParams fp = forward_params(c, st, c->table.p, false, true);
-        issue_forward(c->tt, (int)c->vpl, fp, c->Bcap, c->stream);
+        issue_forward(c->tt, (int)c->vpl, fp, c->Bcap, may_defer(c, c->train_K), c->stream);
         launch_batch_end(st, c->loss.p, c->status.as<int32_t>(), c->nbr_cnt.as<uint32_t>(), c->Bcap, nb, 1, 0, c->stream);
     }
     CK(cudaGetLastError(), "validation launch");
@@ -1435,6 +1483,7 @@ static int stage_samples(ep_ctx* c, const ep_batch_samples* sm, uint32_t es, cud
     if (!all_below(sm->negatives, (uint64_t)B * c->R, c->n_nodes))
         return c->fail(EP_ERR_INVALID_ARG, "negative id out of range");
     const uint64_t items = (uint64_t)B * c->max_feat * (1ull + c->R + K);
+    c->inj_K = K;
     c->typ_items = (uint64_t)((double)c->n_fids / (double)c->n_nodes * ((double)B * (1. + c->R) + nn));
     int rc = ensure_bufs(c, B, K, items, es, true);
     if (rc) return rc;
@@ -1495,7 +1544,7 @@ static int run_injected(ep_ctx* c, uint32_t B, int tt, const void* table, void* 
     fp.loss_out = loss_out;
     fp.dloss = (const float*)dloss;
     fp.dloss_f64 = tt == TT_F64;
-    issue_forward(tt, (int)c->vpl, fp, B, s);
+    issue_forward(tt, (int)c->vpl, fp, B, may_defer(c, c->inj_K), s);
     if (reduce) {
         sort_and_reduce(c, st, tt, out_mode, adam_table, s, gdense);
         if (out_mode == OUT_DENSE && adam_table)
@@ -1592,7 +1641,9 @@ extern "C" int ep_sample_validation(ep_ctx* c, uint32_t first, uint32_t n, uint3
     BatchState* st = c->st_inj.as<BatchState>();
     cudaStream_t s = c->stream;
     CK(cudaMemcpyAsync(st, &h, sizeof(h), cudaMemcpyHostToDevice, s), "validation state");
-    launch_sample(sample_params(c, st, true, 0), s);   // the validation pass's sampler, as run_validation launches it
+    SampleParams sp = sample_params(c, st, true, 0);   // the validation pass's sampler, for the positions given
+    sp.begin = 0;
+    launch_sample(sp, s);
     CK(cudaGetLastError(), "sample launch");
     std::vector<uint32_t> hn((size_t)n * c->Kcap), hc(n);
     std::vector<float> hw((size_t)n * c->Kcap);

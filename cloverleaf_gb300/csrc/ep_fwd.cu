@@ -146,34 +146,35 @@ __device__ __forceinline__ uint32_t permute(uint32_t pos, uint32_t n, uint32_t h
 }
 
 // ---------------------------------------------------------------------------
-// k_batch_begin: batch range, learning rate and Adam bias corrections.
+// Start of a batch (one thread of k_sample's extra CTA; the sampling warps
+// take the range from the batch index themselves): batch range, learning rate
+// and Adam bias corrections.
 // ---------------------------------------------------------------------------
-__global__ void k_batch_begin(BatchState* st, uint32_t n_order, uint32_t cap, uint64_t total,
-                              uint64_t warmup, float alpha, int injected, float noise, float noise_decay) {
-    pdl_wait();
-    pdl_trigger();
-    if (threadIdx.x != 0) return;
-    if (!injected) {
-        uint32_t b0 = st->batch * cap;
-        st->b0 = b0;
-        st->n_anchors = b0 < n_order ? min(cap, n_order - b0) : 0;
-    }
+__device__ __forceinline__ uint32_t batch_anchors(const SampleParams& p, uint32_t b0) {
+    return b0 < p.n_order ? min(p.batch_cap, p.n_order - b0) : 0;
+}
+
+__device__ void begin_batch(const SampleParams& p) {
+    BatchState* st = p.st;
+    const uint32_t b0 = st->batch * p.batch_cap;
+    st->b0 = b0;
+    st->n_anchors = batch_anchors(p, b0);
     // LRScheduler::CosDecay(alpha/100, alpha, warmup, total) (mod.rs:133-137)
-    const float min_alpha = alpha / 100.f;
+    const float min_alpha = p.alpha / 100.f;
     const uint64_t s = st->step;
     float lr;
-    if (s > warmup) {
-        float ratio = (float)s / (float)total;
-        lr = min_alpha + 0.5f * (alpha - min_alpha) * (1.f + cosf(3.14159265358979323846f * ratio));
+    if (s > p.warmup) {
+        float ratio = (float)s / (float)p.total_steps;
+        lr = min_alpha + 0.5f * (p.alpha - min_alpha) * (1.f + cosf(3.14159265358979323846f * ratio));
     } else {
-        float ratio = (float)s / (float)warmup;
-        lr = min_alpha + ratio * (alpha - min_alpha);
+        float ratio = (float)s / (float)p.warmup;
+        lr = min_alpha + ratio * (p.alpha - min_alpha);
     }
     st->lr = lr;
     st->step_cur = (uint32_t)s;
     // gradient noise: LRScheduler::exp_decay(0, noise, decay) at this step
-    // (mod.rs:140-146; scheduler.rs:50-52); injected batches keep their value
-    if (!injected) st->noise_sigma = noise > 1e-9f ? fmaxf(noise * powf(noise_decay, (float)s), 0.f) : 0.f;
+    // (mod.rs:140-146; scheduler.rs:50-52)
+    st->noise_sigma = p.noise > 1e-9f ? fmaxf(p.noise * powf(p.noise_decay, (float)s), 0.f) : 0.f;
     const float t = (float)st->pass + 1.f;
     st->bc1 = 1.f - powf(0.9f, t);
     st->bc2 = 1.f - powf(0.999f, t);
@@ -380,14 +381,8 @@ __device__ void ares_select(const SampleParams& p, uint64_t rs, uint32_t deg, fl
     }
 }
 
-// Tables of the staged gather; an anchor beyond any of these takes the direct
-// path (k_sample decides, from the counts it has at hand).
-constexpr uint32_t NODE_CAP = 64;     // 1 + neighbours + negatives
-constexpr uint32_t OCC_CAP = 512;     // feature occurrences of one anchor
-constexpr uint32_t ROLE_CAP = 34;     // R + 2
-
 // ---------------------------------------------------------------------------
-// k_sample: one warp per anchor.
+// k_sample: one warp per anchor, and a CTA more that starts the batch.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) k_sample(SampleParams p) {
     __shared__ uint32_t s_hist[8][256];   // per warp: ares_select's histogram; ares_hubs' keys
@@ -397,7 +392,12 @@ __global__ void __launch_bounds__(256) k_sample(SampleParams p) {
     const int lane = threadIdx.x & 31;
     const uint32_t a = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     BatchState* st = p.st;
-    const uint32_t n = st->n_anchors;
+    if (p.begin && blockIdx.x == gridDim.x - 1) {
+        if (threadIdx.x == 0) begin_batch(p);
+        return;
+    }
+    const uint32_t b0 = p.begin ? st->batch * p.batch_cap : st->b0;
+    const uint32_t n = p.begin ? batch_anchors(p, b0) : st->n_anchors;
     const SampleCfg& c = p.cfg;
     const uint32_t salt = p.eval ? 0xffffffffu : (uint32_t)st->step;
     uint32_t v = 0;
@@ -405,7 +405,7 @@ __global__ void __launch_bounds__(256) k_sample(SampleParams p) {
         if (p.injected) {
             v = p.anchors[a];
         } else {
-            const uint32_t pos = st->b0 + a;
+            const uint32_t pos = b0 + a;
             uint32_t idx = pos;
             if (!p.eval) {
                 uint32_t k[4];
@@ -772,6 +772,14 @@ __device__ __forceinline__ void fma_row(A (&acc)[VPL], A c, const A (&r)[VPL]) {
     axpy_slice<A, VPL>(acc, c, r);
 }
 
+// One gradient item; with p.hist, it is counted for the sort's first pass too.
+__device__ __forceinline__ void emit_item(const ForwardParams& p, uint64_t at, uint32_t f, uint32_t src, float c) {
+    p.item_f[at] = f;
+    p.item_src[at] = src;
+    p.item_c[at] = c;
+    if (p.hist) atomicAdd(&p.hist[(at / SORT_TILE) * 256u + (f & 255u)], 1u);
+}
+
 // Gathers one role: the (weighted) mean numerator over every feature
 // occurrence of `count` nodes, returning the weight total.  Emits one item
 // per occurrence at item positions pos, pos+1, ... (role-major, node order,
@@ -815,9 +823,7 @@ __device__ A gather_role(const ForwardParams& p, const T* __restrict__ table, co
             uint32_t f = 0;
             if (active) f = p.fids[(((uint64_t)fs_hi << 32) | fs_lo) + (o - excl_q)];
             if (emit && active) {
-                p.item_f[pos + o] = f;
-                p.item_src[pos + o] = src;
-                p.item_c[pos + o] = cq;
+                emit_item(p, pos + o, f, src, cq);
             }
             const uint32_t m = min(32u, total - ob);
             uint32_t j = 0;
@@ -879,9 +885,7 @@ __device__ A gather_role_fd(const ForwardParams& p, const T* __restrict__ table,
                 f = p.fids[fs + j0 + lane];
                 if (emit) {
                     const uint64_t oo = pos + __popc(m & ((1u << lane) - 1u));
-                    p.item_f[oo] = f;
-                    p.item_src[oo] = src;
-                    p.item_c[oo] = c;
+                    emit_item(p, oo, f, src, c);
                 }
             }
             unsigned mm = m;
@@ -1037,9 +1041,7 @@ __device__ void stage_anchor(const ForwardParams& p, GatherTables& S, uint32_t a
                             const uint32_t f = p.fids[(uint64_t)fs + j0 + lane];
                             S.occ[oo] = make_uint2(f, __float_as_uint(S.node_c[q0]));
                             if (emit) {
-                                p.item_f[pos + oo] = f;
-                                p.item_src[pos + oo] = sbase + node_role(q0, cnt);
-                                p.item_c[pos + oo] = S.node_c[q0];
+                                emit_item(p, pos + oo, f, sbase + node_role(q0, cnt), S.node_c[q0]);
                             }
                         }
                         o += __popc(km);
@@ -1086,9 +1088,7 @@ __device__ void stage_anchor(const ForwardParams& p, GatherTables& S, uint32_t a
                     const float c = S.node_c[q];
                     S.occ[oo] = make_uint2(f, __float_as_uint(c));
                     if (emit) {
-                        p.item_f[pos + oo] = f;
-                        p.item_src[pos + oo] = sbase + node_role(q, cnt);
-                        p.item_c[pos + oo] = c;
+                        emit_item(p, pos + oo, f, sbase + node_role(q, cnt), c);
                     }
                 }
             }
@@ -1126,9 +1126,7 @@ __device__ void stage_anchor(const ForwardParams& p, GatherTables& S, uint32_t a
                 const float c = S.node_c[q_of[b]];
                 S.occ[o] = make_uint2(fid[b], __float_as_uint(c));
                 if (emit) {
-                    p.item_f[pos + o] = fid[b];
-                    p.item_src[pos + o] = sbase + node_role(q_of[b], cnt);
-                    p.item_c[pos + o] = c;
+                    emit_item(p, pos + o, fid[b], sbase + node_role(q_of[b], cnt), c);
                 }
             }
         }
@@ -1351,7 +1349,7 @@ __global__ void __launch_bounds__(256) k_fwd_direct(const __grid_constant__ Forw
 
 // k_fwd_gather_queue: the staged gather as a persistent grid (gather_ctas
 // CTAs).  Each warp takes the next anchor from the batch's work queue
-// (BatchState::fwd_next, zeroed by k_batch_begin) until none is left, so a
+// (BatchState::fwd_next, zeroed by k_sample) until none is left, so a
 // warp that drew short anchors takes more of them and no wave waits on its
 // slowest warp.  MINB CTAs per SM (2 or 3, from the grid size) set the
 // register budget of the loop (the one-shot kernel is at its 64-register
@@ -1947,18 +1945,11 @@ void launch_split(uint32_t* train, uint32_t n_train, uint32_t* valid, uint32_t n
 // ---------------------------------------------------------------------------
 // Launchers
 // ---------------------------------------------------------------------------
-void launch_batch_begin(BatchState* st, uint32_t n_order, uint32_t cap, uint32_t steps_per_pass,
-                        uint64_t total, uint64_t warmup, float alpha, int injected, float noise, float noise_decay,
-                        cudaStream_t s) {
-    (void)steps_per_pass;
-    launch_chain(k_batch_begin, 1, 32, 0, s, st, n_order, cap, total, warmup, alpha, injected, noise, noise_decay);
-}
-
 void launch_sample(const SampleParams& p, cudaStream_t s) {
     // warp per anchor in CTAs of sample_warps warps (1-8; 0 = 8)
     const uint32_t w = p.sample_warps >= 1 && p.sample_warps <= 8 ? p.sample_warps : 8;
     const uint32_t blocks = (p.batch_cap + w - 1) / w;
-    launch_chain(k_sample, blocks, 32 * w, 0, s, p);
+    launch_chain(k_sample, blocks + (p.begin ? 1 : 0), 32 * w, 0, s, p);
 }
 
 void launch_scan_occ(BatchState* st, uint32_t* occ, uint32_t cap, uint64_t items_cap, cudaStream_t s) {

@@ -4,8 +4,8 @@
 // Per-batch data flow on the device (stream launches in this order; replayed
 // graphs run the scan, item emission and sort on a side stream beside the
 // gathers and the loss, and the fix-ups beside the next batch's sampling):
-//   k_batch_begin  -> BatchState (batch range, lr, Adam bias corrections)
-//   k_sample       -> anchors, sampled neighbours, negatives, occurrence counts
+//   k_sample       -> BatchState (batch range, lr, Adam bias corrections),
+//                     anchors, sampled neighbours, negatives, occurrence counts
 //   k_scan_occ     -> exclusive item offsets per anchor
 //   k_fwd_gather   -> role means and one item (feature, role-src, count) per
 //                     feature occurrence, written at deterministic offsets
@@ -51,7 +51,7 @@ struct BatchState {
     uint32_t pass;          // 1-based pass index
     uint32_t batch;         // batch index within the pass
     uint64_t step;          // global optimizer step, starts at 1 (mod.rs:153)
-    uint32_t step_cur;      // low bits of the step of the batch in flight (set by k_batch_begin), read
+    uint32_t step_cur;      // low bits of the step of the batch in flight (set by k_sample), read
                             // by the Adam kernels while k_batch_end may already advance `step`
     uint32_t b0;            // first position of this batch in the pass order
     uint32_t n_anchors;     // anchors in this batch
@@ -59,8 +59,8 @@ struct BatchState {
     float bc1, bc2;         // 1 - beta^t with t = pass + 1 (optimizer.rs:50)
     uint32_t error;         // ERR_* bits, sticky
     uint32_t n_items;       // items emitted by this batch
-    uint32_t fwd_next;      // work queue of the persistent gather: next anchor to take (k_batch_begin zeroes it)
-    uint32_t red_next;      // work queue of the persistent reducer: next chunk to take (k_batch_begin zeroes it)
+    uint32_t fwd_next;      // work queue of the persistent gather: next anchor to take (k_sample zeroes it)
+    uint32_t red_next;      // work queue of the persistent reducer: next chunk to take (k_sample zeroes it)
     float noise_sigma;      // gradient-noise scale of this step (0 = off)
     // per-batch outputs of k_batch_end
     float batch_err;        // sum(loss kept) / n_anchors (0 when none kept)
@@ -69,16 +69,25 @@ struct BatchState {
     double pass_err_sum;
     uint32_t pass_batches;
     uint32_t n_long[2];     // long spans queued by k_reduce for k_fixup_long, by the step's parity: a
-                            // batch's k_batch_begin zeroes its own while the previous batch's
+                            // batch's k_sample zeroes its own while the previous batch's
                             // k_fixup_long may still read the other
     // the batch's item count and Adam constants as k_reduce found them: the
     // fix-up and dense Adam kernels read these, so that in replayed graphs
-    // the next batch's k_batch_begin and sampler may run beside them
+    // the next batch's sampler may run beside them
     uint32_t fx_items, fx_step;
     float fx_lr, fx_bc1, fx_bc2, fx_sigma;
     unsigned long long anchors, kept, nan_anchors, items, gathered, unique_rows, sampled;
     double valid_sum;
 };
+
+// Tables of the staged gather; an anchor beyond any of these takes the direct
+// path (k_sample decides, from the counts it has at hand).
+constexpr uint32_t NODE_CAP = 64;     // 1 + neighbours + negatives
+constexpr uint32_t OCC_CAP = 512;     // feature occurrences of one anchor
+constexpr uint32_t ROLE_CAP = 34;     // R + 2
+
+constexpr uint32_t SORT_TILE = 2048;  // items a CTA of the radix sort takes at a time
+constexpr uint64_t RADIX_ONE_ITEMS = 200'000;   // typical batches up to this many items: one kernel per pass
 
 // Feature dropout (max_features): EP_SAMPLE_* kind, Fixed count k,
 // Probability p and its key threshold p * 2^32, and the Philox key.
@@ -122,7 +131,9 @@ struct SampleParams {
                             // 2: anchors provided, neighbours and negatives sampled
     int eval;               // validation: fixed sampling stream, no shuffle
     uint32_t feistel_half;  // half-width in bits of the permutation domain
-    uint32_t feistel_key[4];
+    int begin;              // the launch starts a batch: its range, learning rate, bias corrections and counters
+    uint64_t total_steps, warmup;
+    float alpha, noise, noise_decay;
     // outputs
     uint32_t* anchors;
     uint32_t* nbr;
@@ -172,6 +183,7 @@ struct ForwardParams {
     uint32_t* item_f;
     uint32_t* item_src;
     float* item_c;
+    uint32_t* hist;         // optional: digit counts per SORT_TILE items of the sort's first pass
 };
 
 struct ReduceParams {
@@ -214,9 +226,6 @@ struct ReduceParams {
 };
 
 // ---- launchers (defined in the kernel translation units) -----------------
-void launch_batch_begin(BatchState* st, uint32_t n_order, uint32_t batch_cap,
-                        uint32_t steps_per_pass, uint64_t total_steps, uint64_t warmup,
-                        float alpha, int injected, float noise, float noise_decay, cudaStream_t s);
 void launch_sample(const SampleParams& p, cudaStream_t s);
 void launch_scan_occ(BatchState* st, uint32_t* occ, uint32_t cap, uint64_t items_cap,
                      cudaStream_t s);
@@ -226,9 +235,13 @@ enum ForwardPart : int { FWD_GATHER = 0, FWD_DIRECT = 1, FWD_LOSS = 2 };
 void launch_forward(int tt, int vpl, const ForwardParams& p, uint32_t cap, cudaStream_t s, int part);
 // the item emission alone (k_fwd_emit)
 void launch_emit(const ForwardParams& p, uint32_t cap, cudaStream_t s);
+// counted: the first pass's digit counts are in hist already (ForwardParams::
+// hist) and the counts of the later passes zeroed (radix_clear): one kernel
+// per pass; else three.
 void launch_radix_sort(BatchState* st, uint32_t* keys, uint32_t* keys_alt, const uint32_t* item_src,
                        const float* item_c, uint2* vals, uint2* vals_alt, uint32_t* hist, uint64_t cap,
-                       int key_bits, uint32_t** sorted_keys, uint2** sorted_vals, cudaStream_t s);
+                       int key_bits, bool counted, uint32_t** sorted_keys, uint2** sorted_vals, cudaStream_t s);
+void radix_clear(uint32_t* hist, uint64_t cap, int key_bits, cudaStream_t s);
 void launch_reduce(int tt, int vpl, const ReduceParams& p, uint64_t items_cap, cudaStream_t s);
 // part: 0 both fix-up kernels in order, 1 the short spans (k_fixup), 2 the
 // long spans (k_fixup_long); the two parts are independent

@@ -403,3 +403,26 @@ def test_reducer_split_gives_the_same_table(monkeypatch, form, n_feat):
         tables.append((ctx.get_table(prob["n_feat"], 36), st["unique_rows"], st["gathered_rows"]))
     for t, u, g in tables[1:]:
         assert np.array_equal(tables[0][0], t) and (u, g) == tables[0][1:]
+
+
+@pytest.mark.parametrize("form", [_native.FORM_FUSED_BF16, _native.FORM_PLAIN_FP32])
+@pytest.mark.parametrize("n_feat,batch", [(200, 7), (200, 400), (40_000, 130), (70_000, 500)])
+def test_one_kernel_sort_passes_match_three(form, n_feat, batch):
+    # small batches in replayed graphs sort by one kernel per pass, counted by
+    # the item emission; stream launches by three.  1, 2 and 3 passes; less
+    # than one tile of items, and several with a ragged last one
+    from tests._cases import random_problem
+    prob = random_problem(95, n=2000, n_feat=n_feat, dims=20, deg=(1, 20), feats=(1, 12))
+    out = []
+    for graphs in (1, 0):
+        cfg = _native.default_config()
+        cfg.use_graphs, cfg.form = graphs, form
+        cfg.dims, cfg.negatives, cfg.loss, cfg.gamma = 20, 3, _native.LOSS_STARSPACE, 0.5
+        cfg.batch_size, cfg.passes, cfg.valid_pct = batch, 1, 0.0
+        ctx = _native.Context(cfg)
+        ctx.upload_graph(prob["rows"], prob["cols"], None)
+        ctx.upload_features(prob["fptr"], prob["fids"], n_feat)
+        ctx.set_table(None)
+        st = ctx.train_batches(11)
+        out.append((ctx.get_table(n_feat, 20), st["kept_anchors"], st["items"], st["gathered_rows"], st["unique_rows"]))
+    assert out[0][1] > 0 and out[0][1:] == out[1][1:] and np.array_equal(out[0][0], out[1][0])
