@@ -179,6 +179,14 @@ struct RowIO {
         for (int i = 0; i < NV; ++i) r.v[i] = __ldg(src + i);
         return r;
     }
+    // this lane's slice at `at` (shared memory)
+    static __device__ __forceinline__ Raw load_shared(const T* at) {
+        Raw r;
+        const V* src = reinterpret_cast<const V*>(at);
+#pragma unroll
+        for (int i = 0; i < NV; ++i) r.v[i] = src[i];
+        return r;
+    }
     template <typename A>
     static __device__ __forceinline__ void fma(A (&acc)[VPL], A c, const Raw& r) {
         if constexpr (std::is_same<T, __nv_bfloat16>::value && std::is_same<A, float>::value && VPL >= 2) {

@@ -233,7 +233,31 @@ struct WarpQueue {
     uint32_t* f;           // feature of each slot
     size_t sb;             // slot bytes
     uint32_t head, n;
+    // OUT_STREAM: an mbarrier per slot (its copies landed) and, in bit s, the
+    // parity of slot s's current round
+    unsigned long long* bar;
+    uint32_t phase;
 };
+
+// OUT_STREAM: OUT_QUEUE with the direction rows read through a shared-memory
+// ring as well: STREAM_ROWS rows deep, each lane copying its own slices
+// (cp.async) in groups of STREAM_G, so that rows in flight cost no registers
+// (3 rows in OUT_QUEUE).  A finished row's Adam state comes by three bulk
+// copies on its slot's mbarrier, apart from the cp.async groups, so that
+// neither waits for the other.  For slices of 16 bytes, whose rows are 16-byte
+// multiples (BF16 tables of 129 to 256 dims).  Where the direction rows exceed
+// L2 their latency is what the reducer waits for: reduce stage 672 -> 603 us
+// at 32,768 anchors (302 MB of directions); 131 us either way at 8,192 (50
+// MB).  Narrower slices lose by the second trip through shared memory (100
+// dims: 51 -> 74 us).
+constexpr int OUT_STREAM = 4;
+template <typename T, int VPL>
+constexpr bool streams() { return std::is_same<T, __nv_bfloat16>::value && VPL == 8; }
+constexpr int STREAM_ROWS = 8, STREAM_G = 2;
+constexpr size_t STREAM_BYTES = (size_t)STREAM_ROWS * 32 * 16;    // row ring of a warp
+constexpr uint32_t QUEUE_WAIT_LIMIT = 1u << 22;                   // mbarrier polls before a wait gives up
+
+__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
@@ -271,9 +295,24 @@ __device__ __forceinline__ void queue_slot_ptrs(const WarpQueue& q, uint32_t slo
     t = reinterpret_cast<T*>(v + dpad);
 }
 
+// OUT_STREAM: waits (whole warp, bounded) for the copies of a slot; on giving
+// up, raises the error bit.
+__device__ __forceinline__ bool queue_wait(const ReduceParams& p, const WarpQueue& q, uint32_t slot) {
+    const uint32_t bar = smem_addr(q.bar + slot), parity = (q.phase >> slot) & 1u;
+    uint32_t done = 0;
+    for (uint32_t it = 0; it < QUEUE_WAIT_LIMIT && !done; ++it)
+        asm volatile(
+            "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
+            : "=r"(done)
+            : "r"(bar), "r"(parity)
+            : "memory");
+    if (!done) atomicOr(&p.st->error, ERR_RING_TIMEOUT);
+    return __all_sync(FULL, done);
+}
+
 // Adam on the oldest slot (optimizer.rs:43-81).  The caller has waited for
-// that slot's copies.
-template <typename T, int VPL>
+// that slot's copies (OUT_STREAM waits here).
+template <typename T, int VPL, bool STREAM>
 __device__ __forceinline__ void queue_pop(const ReduceParams& p, WarpQueue& q, int lane, bool lane_on,
                                           const AdamStep& as) {
     if constexpr (sizeof(T) != 8) {
@@ -281,8 +320,13 @@ __device__ __forceinline__ void queue_pop(const ReduceParams& p, WarpQueue& q, i
         float *gs, *ms, *vs;
         T* ts;
         queue_slot_ptrs<T, VPL>(q, q.head, dpad, gs, ms, vs, ts);
+        bool ok = true;
+        if constexpr (STREAM) {
+            ok = queue_wait(p, q, q.head);
+            q.phase ^= 1u << q.head;
+        }
         const uint32_t f = q.f[q.head];
-        if (lane_on) {
+        if (lane_on && ok) {
             float gg[VPL], mm[VPL], vv[VPL], ee[VPL];
             RowIO<float, VPL>::load_generic(gs, lane, gg);
             if constexpr (QueueAsync<T, VPL>::value) {
@@ -297,6 +341,7 @@ __device__ __forceinline__ void queue_pop(const ReduceParams& p, WarpQueue& q, i
             }
             adam_apply<T, VPL>((T*)p.table, p.m, p.v, f, dpad, gg, mm, vv, ee, as, p.seed, lane);
         }
+        if constexpr (STREAM) __syncwarp();   // the slot's reads before its next copies
     }
     q.head = q.head + 1 == QN ? 0u : q.head + 1;
     --q.n;
@@ -305,7 +350,7 @@ __device__ __forceinline__ void queue_pop(const ReduceParams& p, WarpQueue& q, i
 // Queues a finished (NaN-free) row, then, when every slot is taken, updates
 // the oldest: the new row's copies are issued first, so they are in flight
 // while the oldest row is updated as well as while the next rows reduce.
-template <typename T, typename A, int VPL>
+template <typename T, typename A, int VPL, bool STREAM>
 __device__ __forceinline__ void queue_push(const ReduceParams& p, WarpQueue& q, uint32_t f, const A (&acc)[VPL], int lane,
                                            bool lane_on, const AdamStep& as) {
     uint32_t slot = q.head + q.n;
@@ -316,30 +361,47 @@ __device__ __forceinline__ void queue_push(const ReduceParams& p, WarpQueue& q, 
     queue_slot_ptrs<T, VPL>(q, slot, dpad, gs, ms, vs, ts);
     if (lane_on) {
         store_row<float, VPL, A>(gs, lane, acc);
-        if constexpr (QueueAsync<T, VPL>::value) {
+        if constexpr (!STREAM && QueueAsync<T, VPL>::value) {
             const uint64_t o = (uint64_t)f * dpad + (uint64_t)lane * VPL;
             cp_slice<VPL * 4>(ms + lane * VPL, p.m + o);
             cp_slice<VPL * 4>(vs + lane * VPL, p.v + o);
             cp_slice<VPL * (int)sizeof(T)>(ts + lane * VPL, (const T*)p.table + o);
         }
     }
-    cp_async_commit();
+    if constexpr (STREAM) {
+        if (lane == 0) {
+            const uint32_t bar = smem_addr(q.bar + slot), mb = dpad * 4u, tb = dpad * (uint32_t)sizeof(T);
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(2 * mb + tb) : "memory");
+            const uint64_t o = (uint64_t)f * dpad;
+            const void* src[3] = {p.m + o, p.v + o, (const T*)p.table + o};
+            const uint32_t dst[3] = {smem_addr(ms), smem_addr(vs), smem_addr(ts)};
+            const uint32_t len[3] = {mb, mb, tb};
+#pragma unroll
+            for (int i = 0; i < 3; ++i)
+                asm volatile(
+                    "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst[i]),
+                    "l"(src[i]), "r"(len[i]), "r"(bar)
+                    : "memory");
+        }
+    } else {
+        cp_async_commit();
+    }
     if (lane == 0) q.f[slot] = f;
     ++q.n;
     if (q.n == QN) {
-        cp_async_wait<QN - 1>();
+        if constexpr (!STREAM) cp_async_wait<QN - 1>();
         __syncwarp();
-        queue_pop<T, VPL>(p, q, lane, lane_on, as);
+        queue_pop<T, VPL, STREAM>(p, q, lane, lane_on, as);
     }
 }
 
 // Updates every queued slot (end of the warp's work).
-template <typename T, int VPL>
+template <typename T, int VPL, bool STREAM>
 __device__ __forceinline__ void queue_flush(const ReduceParams& p, WarpQueue& q, int lane, bool lane_on,
                                             const AdamStep& as) {
     cp_async_wait<0>();
     __syncwarp();
-    while (q.n) queue_pop<T, VPL>(p, q, lane, lane_on, as);
+    while (q.n) queue_pop<T, VPL, STREAM>(p, q, lane, lane_on, as);
 }
 
 // ---------------------------------------------------------------------------
@@ -390,8 +452,6 @@ __host__ __device__ constexpr size_t ring_slot_bytes(uint32_t dpad) {
     return (size_t)dpad * (3 * sizeof(float) + sizeof(T));   // g, m, v (FP32) + table row; 16-byte multiples
 }
 __host__ __device__ constexpr size_t ring_hdr_bytes() { return (sizeof(RingHdr) + 127) & ~(size_t)127; }
-
-__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
 __device__ __forceinline__ uint32_t ring_test(unsigned long long* bar, uint32_t parity) {
     uint32_t done;
@@ -523,12 +583,12 @@ __device__ __forceinline__ void finish_row(const ReduceParams& p, uint32_t f, co
 #pragma unroll
         for (int k = 0; k < VPL; ++k) bad = bad || (acc[k] != acc[k]);
         if (!__any_sync(FULL, bad)) ring_push<T, A, VPL>(p, rh, ring_slots, f, acc, lane, lane_on);
-    } else if constexpr (MODE == OUT_QUEUE) {
+    } else if constexpr (MODE == OUT_QUEUE || MODE == OUT_STREAM) {
         // rows containing NaN get no Adam step (optimizer.rs:56): not queued
         bool bad = false;
 #pragma unroll
         for (int k = 0; k < VPL; ++k) bad = bad || (acc[k] != acc[k]);
-        if (!__any_sync(FULL, bad)) queue_push<T, A, VPL>(p, *q, f, acc, lane, lane_on, as);
+        if (!__any_sync(FULL, bad)) queue_push<T, A, VPL, MODE == OUT_STREAM>(p, *q, f, acc, lane, lane_on, as);
     } else if constexpr (MODE == OUT_DENSE) {
         if (lane_on) store_row<A, VPL, A>((A*)p.gdense + (uint64_t)f * p.dpad, lane, acc);
         if (fin) {
@@ -659,8 +719,9 @@ __device__ __forceinline__ void reduce_body(const ReduceParams& p, uint32_t spli
 // boundaries; a feature is finished when the stream reaches the first kept
 // item of the next one.
 template <typename T, typename A, int VPL, int MODE>
-__global__ void __launch_bounds__(MODE == OUT_RING ? RING_MAX_WARPS * 32 : (MODE == OUT_QUEUE ? QUEUE_THREADS : RED_THREADS),
-                                  MODE == OUT_RING ? 1 : (VPL >= 16 ? 1 : (MODE == OUT_DENSE ? 3 : (MODE == OUT_QUEUE ? 4 : 2))))
+__global__ void __launch_bounds__(
+    MODE == OUT_RING ? RING_MAX_WARPS * 32 : (MODE == OUT_QUEUE || MODE == OUT_STREAM ? QUEUE_THREADS : RED_THREADS),
+    MODE == OUT_RING ? 1 : (VPL >= 16 ? 1 : (MODE == OUT_DENSE ? 3 : (MODE == OUT_QUEUE || MODE == OUT_STREAM ? 4 : 2))))
     k_reduce(ReduceParams p) {
     pdl_wait();
     pdl_trigger();
@@ -712,13 +773,25 @@ __device__ __forceinline__ void reduce_body(const ReduceParams& p, uint32_t spli
     const uint32_t warp = threadIdx.x >> 5;
     RedEntry<A>* ents;
     uint2* segs;
+    unsigned char* rows = nullptr;    // OUT_STREAM: this lane's slices of the row ring
     {
         size_t off = 0;
-        if constexpr (MODE == OUT_QUEUE) off = queue_list_offset<T>(p.dpad, blockDim.x >> 5);
+        if constexpr (MODE == OUT_QUEUE || MODE == OUT_STREAM) off = queue_list_offset<T>(p.dpad, blockDim.x >> 5);
         if constexpr (MODE == OUT_RING) off = ring_hdr_bytes() + (size_t)p.ring_slots * ring_slot_bytes<T>(p.dpad);
         unsigned char* lb = red_queue + off + (size_t)warp * list_bytes<A>();
         ents = reinterpret_cast<RedEntry<A>*>(lb);
         segs = reinterpret_cast<uint2*>(lb + RW * sizeof(RedEntry<A>));
+        if constexpr (MODE == OUT_STREAM) {
+            // then the warps' row rings and their slots' mbarriers
+            unsigned char* rings = red_queue + off + (size_t)(blockDim.x >> 5) * list_bytes<A>();
+            rows = rings + (size_t)warp * STREAM_BYTES + lane * 16;
+            q.bar = reinterpret_cast<unsigned long long*>(rings + (size_t)(blockDim.x >> 5) * STREAM_BYTES) + warp * QN;
+            q.phase = 0;
+            if (lane < (int)QN)
+                asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(q.bar + lane)) : "memory");
+            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+            __syncwarp();
+        }
     }
     if constexpr (MODE == OUT_RING) {
         if (threadIdx.x == 0) {
@@ -986,6 +1059,52 @@ __device__ __forceinline__ void reduce_body(const ReduceParams& p, uint32_t spli
                 }
             }
             uint32_t next_b = j < je ? segs[j].y : 0xffffffffu;
+            if constexpr (MODE == OUT_STREAM) {
+                static_assert(MODE != OUT_STREAM || !SPLIT, "whole chunks");
+                constexpr int S = STREAM_ROWS / STREAM_G;      // stages of STREAM_G rows
+                constexpr int STAGE = STREAM_G * 32 * 16;
+                // copies the rows of the STREAM_G items from i on into a stage
+                auto fetch = [&](uint32_t i, unsigned char* to) {
+#pragma unroll
+                    for (int u = 0; u < STREAM_G; ++u)
+                        if (i + u < nk)
+                            cp_slice<16>(to + u * 32 * 16,
+                                         dir + (uint64_t)ents[i + u].src * p.dpad + (uint32_t)(lane_ld * VPL));
+                    cp_async_commit();
+                };
+                unsigned char *in = rows, *from = rows;        // stage to fill next, stage to use next
+                for (int t = 0; t + 1 < S; ++t) {
+                    fetch(t * STREAM_G, in);
+                    in += STAGE;
+                }
+                for (; k < nk; k += STREAM_G) {
+                    cp_async_wait<S - 2>();                    // the stage of item k landed (this lane's slices)
+                    fetch(k + (S - 1) * STREAM_G, in);         // into the stage used last
+                    in = in == rows + (S - 1) * STAGE ? rows : in + STAGE;
+                    typename IO::Raw r[STREAM_G];
+#pragma unroll
+                    for (int u = 0; u < STREAM_G; ++u) r[u] = IO::load_shared(reinterpret_cast<const D*>(from + u * 32 * 16));
+                    from = from == rows + (S - 1) * STAGE ? rows : from + STAGE;
+                    if (k + STREAM_G <= nk && k + STREAM_G <= next_b) {   // no feature starts among these
+#pragma unroll
+                        for (int u = 0; u < STREAM_G; ++u) IO::template fma<A>(acc, ents[k + u].w, r[u]);
+                        any_kept = true;
+                        continue;
+                    }
+#pragma unroll
+                    for (int u = 0; u < STREAM_G; ++u) {
+                        if (k + u < nk) {
+                            while (k + u >= next_b) {
+                                close_open(segs[j].x);
+                                ++j;
+                                next_b = j < je ? segs[j].y : 0xffffffffu;
+                            }
+                            IO::template fma<A>(acc, ents[k + u].w, r[u]);
+                            any_kept = true;
+                        }
+                    }
+                }
+            } else {
             for (; k < kend; k += NF) {
                 uint32_t src[NF];
                 A wv[NF];
@@ -1021,6 +1140,7 @@ __device__ __forceinline__ void reduce_body(const ReduceParams& p, uint32_t spli
                         any_kept = true;
                     }
                 }
+            }
             }
             // features of the window with no kept item after their start
             for (; j < je; ++j) close_open(segs[j].x);
@@ -1058,7 +1178,7 @@ __device__ __forceinline__ void reduce_body(const ReduceParams& p, uint32_t spli
         }
     }
     if constexpr (MODE == OUT_DENSE) fin_flush(p, fin, n_fin, lane);
-    if constexpr (MODE == OUT_QUEUE) queue_flush<T, VPL>(p, q, lane, lane_on, as);
+    if constexpr (MODE == OUT_QUEUE || MODE == OUT_STREAM) queue_flush<T, VPL, MODE == OUT_STREAM>(p, q, lane, lane_on, as);
     if constexpr (MODE == OUT_RING) {
         __syncwarp();
         if (lane == 0) {
@@ -1342,6 +1462,12 @@ static size_t queue_smem(uint32_t dpad) {
     return queue_list_offset<T>(dpad, QUEUE_THREADS / 32) + (size_t)(QUEUE_THREADS / 32) * list_bytes<A>();
 }
 
+// OUT_STREAM: the same, the row rings and the mbarriers.
+template <typename T, typename A>
+static size_t stream_smem(uint32_t dpad) {
+    return queue_smem<T, A>(dpad) + (size_t)(QUEUE_THREADS / 32) * (STREAM_BYTES + QN * sizeof(unsigned long long));
+}
+
 template <typename T, typename A, int VPL>
 static void red_launch(const ReduceParams& p, uint64_t cap, cudaStream_t s, int which) {
     const uint32_t nch = reduce_chunks(cap, p.chunk);
@@ -1368,14 +1494,19 @@ static void red_launch(const ReduceParams& p, uint64_t cap, cudaStream_t s, int 
             uint32_t qctas = (warps + QUEUE_THREADS / 32 - 1) / (QUEUE_THREADS / 32);
             if (qctas > 2 * RED_MAX_CTAS) qctas = 2 * RED_MAX_CTAS;
             if (p.red_ctas) qctas = std::min(qctas, p.red_ctas);
-            bool q5 = false;
+            bool done = false;
             if constexpr (VPL <= 8) {
                 if (p.queue_ctas_per_sm >= 5) {
                     launch_chain(k_reduce_q5<T, A, VPL>, qctas, QUEUE_THREADS, queue_smem<T, A>(p.dpad), s, p);
-                    q5 = true;
+                    done = true;
                 }
             }
-            if (!q5) launch_chain(k_reduce<T, A, VPL, OUT_QUEUE>, qctas, QUEUE_THREADS, queue_smem<T, A>(p.dpad), s, p);
+            if (!done) {
+                if constexpr (streams<T, VPL>())
+                    launch_chain(k_reduce<T, A, VPL, OUT_STREAM>, qctas, QUEUE_THREADS, stream_smem<T, A>(p.dpad), s, p);
+                else
+                    launch_chain(k_reduce<T, A, VPL, OUT_QUEUE>, qctas, QUEUE_THREADS, queue_smem<T, A>(p.dpad), s, p);
+            }
         } else if (p.out_mode == OUT_RING) {
             if constexpr (sizeof(T) != 8) {
                 // persistent: every CTA resident at once (one per SM at 16 warps)
@@ -1415,9 +1546,15 @@ static cudaError_t fixl_setup() {
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(k_fixup_long<T, A, VPL, OUT_ADAM>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_reduce<T, A, VPL, OUT_QUEUE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)queue_smem<T, A>(VPL * 32));
+    if constexpr (streams<T, VPL>()) {
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(k_reduce<T, A, VPL, OUT_STREAM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)stream_smem<T, A>(VPL * 32));
+    } else {
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(k_reduce<T, A, VPL, OUT_QUEUE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)queue_smem<T, A>(VPL * 32));
+    }
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(k_reduce_split<T, A, VPL, OUT_QUEUE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)queue_smem<T, A>(VPL * 32));
