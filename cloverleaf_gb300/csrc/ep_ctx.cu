@@ -1033,6 +1033,18 @@ static void advance_host_batch(ep_ctx* c) {
     if (++c->host_batch >= c->steps_per_pass) { c->host_batch = 0; ++c->host_pass; }
 }
 
+// Whether batches are replayed.  A graph costs about 300 us to build and
+// destroy; replaying saves the launches of a small batch (about 30 us) and the
+// overlap of its branches (about 15% of a large one, taken as 0.3 us per
+// thousand items of 256 dims).  9,206 nodes, 20 FP32 dims, whole learn call in
+// us, replayed / launched: 8 batches 3,028 / 2,603, 10 2,670 / 2,731, 30 3,774
+// / 4,323.
+static bool replays(const ep_ctx* c) {
+    const double batches = (double)c->steps_per_pass * std::max<uint32_t>(c->cfg.passes, 1);
+    const double batch_us = (double)c->train_items * c->dims / 256. * 3e-4;
+    return c->cfg.use_graphs && batches * (30. + 0.15 * batch_us) >= 300.;
+}
+
 static int launch_train_batch(ep_ctx* c);
 
 // Issues n consecutive training batches.  With graphs, runs of graph_batches
@@ -1207,7 +1219,7 @@ static int capture_batches(ep_ctx* c, uint32_t batches, cudaGraphExec_t* out) {
 // Builds, ahead of a run of n batches, the graphs that run will replay, so
 // that the one-time capture and instantiation stay outside its timing.
 static int prepare_graphs(ep_ctx* c, uint32_t n) {
-    if (!c->cfg.use_graphs || n == 0) return EP_OK;
+    if (!replays(c) || n == 0) return EP_OK;
     if (c->cfg.autotune && !tune_from_cache(c)) {
         std::vector<TuneChoice> s1;
         uint32_t need = 0;
@@ -1232,7 +1244,7 @@ static int launch_train_run(ep_ctx* c, uint32_t n) {
         int rc = autotune(c, n);
         if (rc) return rc;
     }
-    const bool use_graph = c->cfg.use_graphs;
+    const bool use_graph = replays(c);
     const uint32_t k = c->graph_batches;
     while (n) {
         if (use_graph && k > 1 && n >= k) {
@@ -1268,7 +1280,7 @@ static int launch_train_run(ep_ctx* c, uint32_t n) {
 }
 
 static int launch_train_batch(ep_ctx* c) {
-    const bool use_graph = c->cfg.use_graphs;
+    const bool use_graph = replays(c);
     if (use_graph) {
         if (!c->gexec) {
             int rc = capture_batches(c, 1, &c->gexec);

@@ -366,7 +366,7 @@ def test_gather_split_gives_the_same_table(monkeypatch, max_features):
             cfg = _native.default_config()
             cfg.use_graphs, cfg.form = graphs, form
             cfg.dims, cfg.negatives, cfg.loss, cfg.gamma = 52, 7, _native.LOSS_STARSPACE, 0.5
-            cfg.batch_size, cfg.passes, cfg.valid_pct = 300, 1, 0.0
+            cfg.batch_size, cfg.passes, cfg.valid_pct = 300, 10, 0.0
             cfg.max_nodes_kind, cfg.max_nodes = _native.SAMPLE_FIXED, 20.0
             if max_features is not None:
                 cfg.max_features = max_features
@@ -418,7 +418,7 @@ def test_one_kernel_sort_passes_match_three(form, n_feat, batch):
         cfg = _native.default_config()
         cfg.use_graphs, cfg.form = graphs, form
         cfg.dims, cfg.negatives, cfg.loss, cfg.gamma = 20, 3, _native.LOSS_STARSPACE, 0.5
-        cfg.batch_size, cfg.passes, cfg.valid_pct = batch, 1, 0.0
+        cfg.batch_size, cfg.passes, cfg.valid_pct = batch, 10, 0.0   # batches enough for replaying to pay
         ctx = _native.Context(cfg)
         ctx.upload_graph(prob["rows"], prob["cols"], None)
         ctx.upload_features(prob["fptr"], prob["fids"], n_feat)
