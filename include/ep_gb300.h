@@ -100,8 +100,8 @@ typedef struct ep_config {
                                     bit-identical; 2 also reducer chunk sizes, whose
                                     summation order then depends on timing.  Setting a
                                     shape through EP_FUSED_MODE, EP_REDUCE_CHUNK,
-                                    EP_GATHER_CTAS or EP_RING_* in the environment
-                                    turns tuning off */
+                                    EP_GATHER_CTAS, EP_GATHER_SPLIT, EP_RED_SPLIT or
+                                    EP_RING_* in the environment turns tuning off */
     float ppr_restart_p;         /* EP_LOSS_PPR walk restart probability in [0, 1] */
 } ep_config;
 
