@@ -22,6 +22,7 @@
 #include <omp.h>
 #endif
 
+#include <sys/mman.h>
 #include <unistd.h>
 
 #include "../../include/ep_gb300.h"
@@ -614,7 +615,11 @@ namespace ep {
 
 namespace {
 constexpr size_t PAGE_PIECE = 1u << 20;      // bytes a thread takes at a time (divides a slab)
-constexpr size_t SMALL_PIECE = 1u << 16;
+#ifdef MADV_POPULATE_WRITE
+constexpr int POPULATE_WRITE = MADV_POPULATE_WRITE;
+#else
+constexpr int POPULATE_WRITE = 23;           // Linux 5.14
+#endif
 }
 
 ResultPages::ResultPages(void* p, size_t bytes)
@@ -625,7 +630,7 @@ ResultPages::ResultPages(void* p, size_t bytes)
         return;
     }
     const unsigned cores = std::max(1u, std::thread::hardware_concurrency());
-    const size_t want = std::min<size_t>({8, cores, pieces_});
+    const size_t want = std::min<size_t>({THREADS, cores, pieces_});
     try {
         left_.reset(new std::atomic<uint32_t>[slabs()]);
         for (size_t i = 0; i < slabs(); ++i)
@@ -642,17 +647,16 @@ ResultPages::~ResultPages() {
     for (auto& t : threads_) t.join();
 }
 
-void ResultPages::touch(size_t from, size_t to) {
+// The pages that hold bytes [from, to); errors leave them to the copy.
+void ResultPages::populate(size_t from, size_t to) {
     if (from >= to) return;
-    volatile char* c = p_;
-    if (from == 0) c[0] = 0;
-    const uintptr_t base = (uintptr_t)p_;
-    for (uintptr_t a = (base + from + page_ - 1) / page_ * page_; a < base + to; a += page_) c[a - base] = 0;
+    const uintptr_t a = ((uintptr_t)p_ + from) / page_ * page_, b = ((uintptr_t)p_ + to + page_ - 1) / page_ * page_;
+    (void)madvise((void*)a, b - a, POPULATE_WRITE);
 }
 
 void ResultPages::work() {
     for (size_t i = next_++; i < pieces_; i = next_++) {
-        touch(i * PAGE_PIECE, std::min(bytes_, (i + 1) * PAGE_PIECE));
+        populate(i * PAGE_PIECE, std::min(bytes_, (i + 1) * PAGE_PIECE));
         left_[i / (SLAB / PAGE_PIECE)].fetch_sub(1, std::memory_order_release);
     }
 }
@@ -662,9 +666,10 @@ void ResultPages::wait(size_t i) {
         later_ = false;
         // the whole OpenMP team or none of it: a smaller one would make the
         // runtime end the others' threads and start them again later (0.6 ms)
-        const int64_t n = (int64_t)((bytes_ + SMALL_PIECE - 1) / SMALL_PIECE);
-#pragma omp parallel for if (n > 128) schedule(static)
-        for (int64_t k = 0; k < n; ++k) touch((size_t)k * SMALL_PIECE, std::min(bytes_, ((size_t)k + 1) * SMALL_PIECE));
+        const size_t part = (bytes_ + THREADS - 1) / THREADS;
+#pragma omp parallel for if (bytes_ > 8 * PAGE_PIECE) schedule(static, 1)
+        for (int64_t k = 0; k < (int64_t)THREADS; ++k)
+            populate(std::min(bytes_, (size_t)k * part), std::min(bytes_, ((size_t)k + 1) * part));
         return;
     }
     if (!left_ || i >= slabs()) return;

@@ -11,15 +11,19 @@
 
 namespace ep {
 
-// Makes the pages of a result array, which is about to be overwritten whole,
-// resident from a few threads while the device computes: a zero is stored in
-// each page, slab by slab.  Pages of a fresh array that a device-to-host copy
-// meets first are faulted in one by one through the host's page tables: a
-// 4 MB download took 2.2 ms into a fresh array and 0.04 ms into a resident
-// one, 205 MB 7.5 and 1.15 ms.  (A load before the store would map the shared
-// zero page, whose replacement makes the device drop its translations: 26 us
-// a page.)  Arrays below THREADED, where starting threads costs more than
-// they save (0.4 ms), are made resident by wait(), on the OpenMP threads.
+// Makes the pages of a result array resident from a few threads while the
+// device computes, slab by slab, with MADV_POPULATE_WRITE: the contents stay
+// as they are, so the array may overlap an input, and a call that fails before
+// its download leaves it unchanged.  Pages of a fresh array that a
+// device-to-host copy meets first are faulted in one by one through the host's
+// page tables: a 4 MB download took 2.2 ms into a fresh array and 0.04 ms into
+// a resident one, 205 MB 7.5 and 1.15 ms.  (An atomic addition of zero keeps
+// the contents too, but maps the shared zero page first, whose replacement
+// makes the device drop its translations: 24 us a page of 64 KB.)  205 MB take
+// 2.2 ms on four threads; on eight they stand in each other's way, 7.3 ms.
+// Where the kernel does not know the advice the pages are left to the copy.
+// Arrays below THREADED, where starting threads costs more than they save
+// (0.4 ms), are made resident by wait(), on the OpenMP threads.
 class ResultPages {
 public:
     static constexpr size_t SLAB = 32u << 20, THREADED = 48u << 20;
@@ -34,7 +38,9 @@ public:
     void wait(size_t i);
 
 private:
-    void touch(size_t from, size_t to);
+    static constexpr size_t THREADS = 4;
+
+    void populate(size_t from, size_t to);
     void work();
 
     char* p_;
