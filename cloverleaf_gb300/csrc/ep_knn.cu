@@ -913,15 +913,16 @@ cudaError_t knn_launch_k(const KnnArgs& a, uint32_t t0, uint32_t t1, uint32_t sp
 
 using namespace ep;
 
-extern "C" int ep_embed_features(int device, uint64_t n_nodes, const uint64_t* fptr, const uint32_t* fids,
-                                 const float* fweight, uint32_t n_feat, uint32_t dims, const float* table,
-                                 float* out) {
-    if (!fptr || !out || (n_nodes && !table && n_feat) || dims == 0 || dims > 512)
-        return knn_fail(EP_ERR_INVALID_ARG, "invalid arguments (dims must be in [1, 512])");
-    if (!monotone(fptr, n_nodes)) return knn_fail(EP_ERR_INVALID_ARG, "fptr is not monotone");
+// The result of a call that checks its ids on the way to the device: one that
+// got no device or no memory is refused for a bad id all the same.
+static int refused(int rc, const uint32_t* ids, uint64_t n, uint64_t bound, const char* msg) {
+    if (rc == EP_OK || rc == EP_ERR_INVALID_ARG || all_below(ids, n, bound)) return rc;
+    return knn_fail(EP_ERR_INVALID_ARG, msg);
+}
+
+static int embed_run(int device, uint64_t n_nodes, const uint64_t* fptr, const uint32_t* fids,
+                     const float* fweight, uint32_t n_feat, uint32_t dims, const float* table, float* out) {
     const uint64_t nf = fptr[n_nodes];
-    for (uint64_t j = 0; !n_nodes && j < nf; ++j)      // no node reads them, but they are the caller's
-        if (fids[j] >= n_feat) return knn_fail(EP_ERR_INVALID_ARG, "feature id out of range");
     KCK(cudaSetDevice(device), "select device");
     if (!n_nodes) return EP_OK;
     cudaStream_t s;
@@ -953,16 +954,21 @@ extern "C" int ep_embed_features(int device, uint64_t n_nodes, const uint64_t* f
     return EP_OK;
 }
 
-extern "C" int ep_align(int device, uint64_t n_nodes, const uint64_t* row_ptr, const uint32_t* cols,
-                        const float* w_cdf, uint32_t dims, const float* emb, float alpha, uint64_t max_neighbors,
-                        float* out) {
-    if (!row_ptr || (n_nodes && (!emb || !out)) || dims == 0 || dims > 512)
+extern "C" int ep_embed_features(int device, uint64_t n_nodes, const uint64_t* fptr, const uint32_t* fids,
+                                 const float* fweight, uint32_t n_feat, uint32_t dims, const float* table,
+                                 float* out) {
+    if (!fptr || !out || (n_nodes && !table && n_feat) || dims == 0 || dims > 512)
         return knn_fail(EP_ERR_INVALID_ARG, "invalid arguments (dims must be in [1, 512])");
-    if (alpha > 1.f || alpha != alpha) return knn_fail(EP_ERR_INVALID_ARG, "alpha must be <= 1 (negative: adaptive)");
+    if (!monotone(fptr, n_nodes)) return knn_fail(EP_ERR_INVALID_ARG, "fptr is not monotone");
+    if (!n_nodes && !all_below(fids, fptr[0], n_feat))      // no node reads them, but they are the caller's
+        return knn_fail(EP_ERR_INVALID_ARG, "feature id out of range");
+    return refused(embed_run(device, n_nodes, fptr, fids, fweight, n_feat, dims, table, out), fids, fptr[n_nodes], n_feat,
+                   "feature id out of range");
+}
+
+static int align_run(int device, uint64_t n_nodes, const uint64_t* row_ptr, const uint32_t* cols,
+                     const float* w_cdf, uint32_t dims, const float* emb, float alpha, uint64_t max_neighbors, float* out) {
     const uint64_t ne = row_ptr[n_nodes];
-    if (ne && (!cols || !w_cdf)) return knn_fail(EP_ERR_INVALID_ARG, "null edge arrays");
-    if (!monotone(row_ptr, n_nodes)) return knn_fail(EP_ERR_INVALID_ARG, "row_ptr is not monotone");
-    if (!n_nodes && ne) return knn_fail(EP_ERR_INVALID_ARG, "column id out of range");
     KCK(cudaSetDevice(device), "select device");
     if (!n_nodes) return EP_OK;
     cudaStream_t s;
@@ -1006,6 +1012,20 @@ extern "C" int ep_align(int device, uint64_t n_nodes, const uint64_t* row_ptr, c
     KCK(download((char*)out, p.out, out_bytes, pages, s), "align");
     cudaEventElapsedTime(&g_knn_ms, e0, e1);
     return EP_OK;
+}
+
+extern "C" int ep_align(int device, uint64_t n_nodes, const uint64_t* row_ptr, const uint32_t* cols,
+                        const float* w_cdf, uint32_t dims, const float* emb, float alpha, uint64_t max_neighbors,
+                        float* out) {
+    if (!row_ptr || (n_nodes && (!emb || !out)) || dims == 0 || dims > 512)
+        return knn_fail(EP_ERR_INVALID_ARG, "invalid arguments (dims must be in [1, 512])");
+    if (alpha > 1.f || alpha != alpha) return knn_fail(EP_ERR_INVALID_ARG, "alpha must be <= 1 (negative: adaptive)");
+    const uint64_t ne = row_ptr[n_nodes];
+    if (ne && (!cols || !w_cdf)) return knn_fail(EP_ERR_INVALID_ARG, "null edge arrays");
+    if (!monotone(row_ptr, n_nodes)) return knn_fail(EP_ERR_INVALID_ARG, "row_ptr is not monotone");
+    if (!n_nodes && ne) return knn_fail(EP_ERR_INVALID_ARG, "column id out of range");
+    return refused(align_run(device, n_nodes, row_ptr, cols, w_cdf, dims, emb, alpha, max_neighbors, out), cols, ne, n_nodes,
+                   "column id out of range");
 }
 
 extern "C" int ep_knn_cosine(int device, uint64_t n_db, uint32_t dims, const float* db, uint64_t n_q,

@@ -220,3 +220,23 @@ def test_evaluation_wrappers_check_shapes():
         _native.knn_cosine(np.zeros((5, 8), np.float32), np.zeros((2, 8), np.float32), 3, q_self=[0])
     with pytest.raises(ValueError):
         _native.embed_features(np.array([0, 3], np.uint64), np.array([0, 1], np.uint32), np.zeros((4, 8), np.float32))
+
+
+@pytest.mark.parametrize("n", [50, 60_000])
+def test_bad_ids_are_named_without_a_device(native, n):
+    # ids are checked on the way to the device (on it, above 131,072 of them);
+    # a call that gets none (device 99) is refused for a bad id all the same
+    rows = np.arange(n + 1, dtype=np.uint64) * 3
+    cols = np.random.default_rng(n).integers(0, n, 3 * n).astype(np.uint32)
+    cdf = np.tile(np.float32([0.3, 0.6, 1.0]), n)
+    emb = np.ones((n, 4), np.float32)
+    calls = {"align": lambda c: _native.align(rows, c, cdf, emb, alpha=0.5, device=99),
+             "embed": lambda c: _native.embed_features(rows, c, emb, device=99)}
+    for call in calls.values():
+        with pytest.raises(_native.NativeError, match="select device"):
+            call(cols)
+        bad = cols.copy()
+        bad[-1] = n
+        with pytest.raises(_native.NativeError, match="id out of range") as e:
+            call(bad)
+        assert e.value.code == -1           # EP_ERR_INVALID_ARG
