@@ -136,16 +136,38 @@ cudaError_t download(char* out, const void* d_out, size_t bytes, ResultPages& pa
 // coefficients come 32 at a time across the lanes; U rows are in flight.
 // Bound by the row reads from L2 (ROWS_ALIGN, 200,000 nodes, 4M edges x 128:
 // 2 GB).
-// Rows of more than HUB_ROWS edges, whose sums are one long chain, are left
-// to the first HUB_CTAS CTAs of the grid: a CTA per hub and slice of 32
-// elements, whose warps load and weigh HUB_TILE rows at a time into shared
-// memory while one warp adds up the tile before, in edge order.  (4.1 ms
-// before, all of it the 10,000-edge hub's chain with one row in flight.)
+// The longest rows, whose sums are one long chain, are left to the first
+// HUB_CTAS CTAs of the grid: a CTA per hub and slice of 32 elements, whose
+// warps load and weigh HUB_TILE rows at a time into shared memory while one
+// warp adds up the tile before, in edge order.  (4.1 ms before, all of it the
+// 10,000-edge hub's chain with one row in flight.)
 // ---------------------------------------------------------------------------
 enum RowsMode : int { ROWS_MEAN = 0, ROWS_WEIGHTED = 1, ROWS_ALIGN = 2 };
-constexpr uint32_t HUB_ROWS = 256;
 constexpr unsigned HUB_CTAS = 152;
 constexpr uint32_t HUB_TILE = 128;
+
+// Which rows are hubs.  The warps of all rows run at once, each as long as its
+// row; the HUB_CTAS CTAs share all hubs' slices.  So the hubs are the rows
+// above the smallest length T = HUB_ROWS x 2^b at which the hubs' slices
+// together are in proportion to T:
+//   edges(rows above T) x slices <= T x share,
+// with a share four times as large above 128 elements, where a warp has half
+// the rows in flight and each is twice as long.  A graph whose rows are all
+// long has no hubs.  Kernel time in us with every row above 256 a hub / by
+// this rule / without hubs: 4,000 nodes of 1,000 edges x 128 1,300 / 210 /
+// 211; 20,000 of 400 x 128 3,300 / 287 / 289; 300 of 3,000 x 128 245 / 259 /
+// 256; one of 10,000 among 100,000 133 / 138 / 978; 200,000 nodes of a power
+// law with a 6,000-edge hub x 128 618 / 544 / 1,089 and x 256 1,102 / 1,042 /
+// 2,823, with a 44,000-edge hub x 128 843 / 649 / 6,628.
+constexpr uint32_t HUB_ROWS = 256;
+constexpr int HUB_CLASSES = 25;              // the last: more than 2^32 edges
+__host__ __device__ constexpr uint64_t hub_share(uint32_t d) { return d <= 128 ? 4640u : 4u * 4640u; }
+
+struct Hubs {
+    unsigned long long edges[HUB_CLASSES];   // class b: edges of the rows of (HUB_ROWS << b, HUB_ROWS << (b + 1)]
+    unsigned long long above;                // T
+    uint32_t n;                              // hubs
+};
 
 struct RowsParams {
     uint64_t n;                  // nodes
@@ -156,8 +178,8 @@ struct RowsParams {
     const float* table;
     float alpha;
     uint64_t kmax;
-    const uint32_t* hubs;        // nodes of more than HUB_ROWS edges
-    const uint32_t* n_hubs;
+    uint32_t* hubs;              // nodes of the hubs
+    Hubs* hub;
     float* out;
 };
 
@@ -175,7 +197,7 @@ __device__ void hub_rows(const RowsParams& p) {
     const int lane = threadIdx.x & 31;
     const uint32_t w = threadIdx.x >> 5;
     const uint32_t slices = (p.d + 31) / 32;
-    const uint64_t n = (uint64_t)*p.n_hubs * slices;
+    const uint64_t n = (uint64_t)p.hub->n * slices;
     for (uint64_t it = blockIdx.x; it < n; it += HUB_CTAS) {
         const uint64_t v = p.hubs[it / slices];
         const uint32_t k = (uint32_t)(it % slices) * 32u + lane;
@@ -247,8 +269,8 @@ __global__ void __launch_bounds__(256) k_rows(const RowsParams p) {
     if (v >= p.n) return;
     const uint32_t d = p.d;
     const uint64_t b = p.ptr[v], deg = p.ptr[v + 1] - b;
-    if (MODE == ROWS_ALIGN && deg > HUB_ROWS) return;
     const uint64_t m = MODE == ROWS_ALIGN && p.kmax < deg ? p.kmax : deg;
+    if (MODE == ROWS_ALIGN && m > p.hub->above) return;
     float acc[NV][E];
 #pragma unroll
     for (int i = 0; i < NV; ++i)
@@ -328,11 +350,40 @@ __global__ void __launch_bounds__(256) k_rows(const RowsParams p) {
     }
 }
 
-// The nodes of more than HUB_ROWS edges, in any order.
-__global__ void __launch_bounds__(256) k_find_hubs(uint64_t n, const uint64_t* __restrict__ ptr, uint32_t* __restrict__ hubs,
-                                                   uint32_t* __restrict__ n_hubs) {
-    for (uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (uint64_t)gridDim.x * blockDim.x)
-        if (ptr[v + 1] - ptr[v] > HUB_ROWS) hubs[atomicAdd(n_hubs, 1u)] = (uint32_t)v;
+// The edges of each class of long rows (Hubs::edges, zeroed before).
+__global__ void __launch_bounds__(256) k_hub_edges(const RowsParams p) {
+    __shared__ unsigned long long sum[HUB_CLASSES];
+    __shared__ uint32_t any;
+    if (threadIdx.x == 0) any = 0;
+    if (threadIdx.x < HUB_CLASSES) sum[threadIdx.x] = 0;
+    __syncthreads();
+    for (uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v < p.n; v += (uint64_t)gridDim.x * blockDim.x) {
+        const uint64_t m = min(p.ptr[v + 1] - p.ptr[v], p.kmax);
+        if (m <= HUB_ROWS) continue;
+        const int b = 63 - __clzll((long long)((m - 1) / HUB_ROWS));
+        atomicAdd(&sum[min(b, HUB_CLASSES - 1)], (unsigned long long)m);
+        any = 1;
+    }
+    __syncthreads();
+    if (any && threadIdx.x < HUB_CLASSES && sum[threadIdx.x]) atomicAdd(&p.hub->edges[threadIdx.x], sum[threadIdx.x]);
+}
+
+// The hubs, in any order, and the length they exceed.
+__global__ void __launch_bounds__(256) k_find_hubs(const RowsParams p) {
+    __shared__ uint64_t above;
+    if (threadIdx.x == 0) {
+        const uint64_t slices = (p.d + 31) / 32;
+        uint64_t left = 0;                   // edges of the rows above T
+        for (int b = 0; b < HUB_CLASSES; ++b) left += p.hub->edges[b];
+        uint64_t t = HUB_ROWS;
+        for (int b = 0; b < HUB_CLASSES && left * slices > hub_share(p.d) * t; ++b, t *= 2) left -= p.hub->edges[b];
+        above = left ? t : ~0ull;
+        if (blockIdx.x == 0) p.hub->above = above;
+    }
+    __syncthreads();
+    if (above == ~0ull) return;
+    for (uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v < p.n; v += (uint64_t)gridDim.x * blockDim.x)
+        if (min(p.ptr[v + 1] - p.ptr[v], p.kmax) > above) p.hubs[atomicAdd(&p.hub->n, 1u)] = (uint32_t)v;
 }
 
 template <int MODE>
@@ -976,7 +1027,7 @@ static int align_run(int device, uint64_t n_nodes, const uint64_t* row_ptr, cons
     struct SG { cudaStream_t s; ~SG() { cudaStreamDestroy(s); } } sg{s};
     Arena ar;
     const size_t out_bytes = (size_t)n_nodes * dims * 4;
-    const size_t o_bad = ar.reserve(4), o_nh = ar.reserve(4), o_rp = ar.reserve((n_nodes + 1) * 8), o_cols = ar.reserve(ne * 4),
+    const size_t o_bad = ar.reserve(4), o_nh = ar.reserve(sizeof(Hubs)), o_rp = ar.reserve((n_nodes + 1) * 8), o_cols = ar.reserve(ne * 4),
                  o_cdf = ar.reserve(ne * 4), o_emb = ar.reserve(out_bytes),
                  o_hubs = ar.reserve((ne / (HUB_ROWS + 1) + 1) * 4), o_out = ar.reserve(out_bytes);
     KCK(ar.mem.alloc(ar.used), "alloc");
@@ -997,16 +1048,17 @@ static int align_run(int device, uint64_t n_nodes, const uint64_t* row_ptr, cons
     p.alpha = alpha;
     p.kmax = max_neighbors ? max_neighbors : ~0ull;
     p.hubs = ar.at<uint32_t>(o_hubs);
-    p.n_hubs = ar.at<uint32_t>(o_nh);
+    p.hub = ar.at<Hubs>(o_nh);
     p.out = ar.at<float>(o_out);
     cudaEvent_t e0, e1;
     KCK(cudaEventCreate(&e0), "events");
     KCK(cudaEventCreate(&e1), "events");
     struct EG { cudaEvent_t a, b; ~EG() { cudaEventDestroy(a); cudaEventDestroy(b); } } eg{e0, e1};
-    KCK(cudaMemsetAsync(ar.at<void>(o_nh), 0, 4, s), "clear");
+    KCK(cudaMemsetAsync(p.hub, 0, sizeof(Hubs), s), "clear");
     cudaEventRecord(e0, s);
-    k_find_hubs<<<(unsigned)std::min<uint64_t>((n_nodes + 255) / 256, 152 * 8), 256, 0, s>>>(
-        n_nodes, ar.at<uint64_t>(o_rp), ar.at<uint32_t>(o_hubs), ar.at<uint32_t>(o_nh));
+    const unsigned scan = (unsigned)std::min<uint64_t>((n_nodes + 255) / 256, 152 * 8);
+    k_hub_edges<<<scan, 256, 0, s>>>(p);
+    k_find_hubs<<<scan, 256, 0, s>>>(p);
     KCK(launch_rows<ROWS_ALIGN>(p, s), "align launch");
     cudaEventRecord(e1, s);
     KCK(download((char*)out, p.out, out_bytes, pages, s), "align");

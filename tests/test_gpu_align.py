@@ -89,3 +89,61 @@ def test_align_neighbour_cap_beyond_degree_and_zero_alpha(oracle):
     assert np.array_equal(a, b)
     z = np.nonzero(np.diff(rows) == 0)[0]
     assert len(z) and not a[z].any()                 # no edges and alpha 0: zero rows
+
+
+def _by_degree(seed, deg, dims):
+    """A graph of 40 nodes of up to 20 edges and one of each given degree; CDF weights; a row per node."""
+    rng = np.random.default_rng(seed)
+    d = np.concatenate([rng.integers(0, 21, 40), np.asarray(deg)])
+    rng.shuffle(d)
+    rows = np.zeros(len(d) + 1, np.uint64)
+    rows[1:] = np.cumsum(d)
+    cols = rng.integers(0, len(d), int(rows[-1])).astype(np.uint32)
+    cdf = np.zeros(len(cols), np.float32)
+    for v in range(len(d)):
+        s, e = int(rows[v]), int(rows[v + 1])
+        if e > s:
+            c = np.cumsum(rng.uniform(0.1, 5.0, e - s), dtype=np.float32)
+            cdf[s:e] = c / c[-1]
+    return rows, cols, cdf, rng.standard_normal((len(d), dims)).astype(np.float32)
+
+
+@pytest.mark.parametrize("dims", [1, 33, 128, 130, 256, 300])
+@pytest.mark.parametrize("max_neighbors", [None, 8, 255, 256, 257, 400])
+def test_align_hubs(oracle, dims, max_neighbors):
+    # few long rows (shared out to whole CTAs): around the shortest hub, around
+    # tiles of 128 rows, a neighbour cap on either side of it
+    rows, cols, cdf, emb = _by_degree(dims, [255, 256, 257, 383, 384, 385, 512, 513, 5000], dims)
+    got = _native.align(rows, cols, cdf, emb, alpha=0.35, max_neighbors=max_neighbors)
+    assert np.array_equal(got, oracle.align(rows, cols, cdf, emb, alpha=0.35, max_neighbors=max_neighbors))
+
+
+@pytest.mark.parametrize("dims,n,deg", [(16, 3000, 300), (128, 2500, 600), (256, 1200, 600), (36, 300, 3000)])
+def test_align_when_most_rows_are_long(oracle, dims, n, deg):
+    # no hubs, or only the longest row: the others are a warp's work however
+    # long; the longest is above and below twice their length
+    for longest in (deg, 40 * deg):
+        rows, cols, cdf, emb = _by_degree(n, [deg] * n + [longest], dims)
+        got = _native.align(rows, cols, cdf, emb, alpha=0.35)
+        assert np.array_equal(got, oracle.align(rows, cols, cdf, emb, alpha=0.35))
+
+
+def test_alignment_takes_no_longer_for_many_hubs_than_row_by_row():
+    # 4,000 nodes of 1,000 edges: 0.21 ms a warp per node, 1.3 ms by 152 CTAs
+    # a slice of a node at a time.  Against a graph of as many edges in rows
+    # of 200, which are no hubs: 0.2 ms; three times that leaves room for both
+    from cloverleaf_gb300._native import lib
+    rng = np.random.default_rng(1)
+    best = {}
+    for deg in (200, 1000):
+        n = 4_000_000 // deg
+        rows = np.arange(n + 1, dtype=np.uint64) * deg
+        cols = rng.integers(0, 4000, n * deg).astype(np.uint32)
+        cdf = np.tile(((np.arange(deg) + 1) / deg).astype(np.float32), n)
+        emb = rng.standard_normal((n, 128)).astype(np.float32)
+        ms = []
+        for _ in range(5):
+            _native.align(rows, cols, cdf, emb, alpha=0.5)
+            ms.append(lib().ep_knn_last_kernel_ms())
+        best[deg] = min(ms)
+    assert best[1000] < 3 * best[200], best
