@@ -279,13 +279,28 @@ __device__ void ares_small(const SampleParams& p, uint64_t rs, uint32_t deg, flo
 // anchors of a 60,000-node power-law graph with 2 hard negatives, 101 us a
 // batch at the start, 65 us with ares_small's cheaper blocks and the row scan
 // of the hard negatives, 49 us with the hubs shared (what is left is the
-// walks' chain of loads).
+// walks' chain of loads).  The CTA's hubs follow one another, at about 9 ns an
+// edge, where a warp by itself takes 21 and all of them run at once: they are
+// shared while together they are no longer than twice the longest
+// (hubs_shared).  A batch of 1,000 anchors of 1,000 edges each, sampling stage:
+// 156 us shared, 43 us by their own warps.
 constexpr uint32_t HUB_DEG = 512, HUB_KEYS = 256;
 
 struct HubAnchor {
     uint64_t rs;
     uint32_t v, deg;    // deg 0: none
 };
+
+// Whether the CTA's hubs are sampled by all its warps (uniform over the CTA).
+__device__ __forceinline__ bool hubs_shared(const HubAnchor* hubs) {
+    uint64_t sum = 0;
+    uint32_t most = 0;
+    for (uint32_t h = 0; h < blockDim.x >> 5; ++h) {
+        sum += hubs[h].deg;
+        most = max(most, hubs[h].deg);
+    }
+    return sum <= 2ull * most;
+}
 
 __device__ void ares_hubs(const SampleParams& p, const HubAnchor* hubs, uint32_t salt, float* keys, int lane) {
     const uint32_t w = threadIdx.x >> 5, nw = blockDim.x >> 5, r = p.cfg.K;
@@ -431,8 +446,10 @@ __global__ void __launch_bounds__(256) k_sample(SampleParams p) {
             s_hub[threadIdx.x >> 5] = h;
         }
         __syncthreads();
-        hub = s_hub[threadIdx.x >> 5].deg != 0;
-        ares_hubs(p, s_hub, salt, reinterpret_cast<float*>(&s_hist[0][0]), lane);
+        if (hubs_shared(s_hub)) {
+            hub = s_hub[threadIdx.x >> 5].deg != 0;
+            ares_hubs(p, s_hub, salt, reinterpret_cast<float*>(&s_hist[0][0]), lane);
+        }
     }
     if (a >= n) return;
     if (p.injected != 1) {

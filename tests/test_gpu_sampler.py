@@ -123,3 +123,59 @@ def test_negatives_are_uniform_over_training_ids():
     observed = counts[train]
     assert stats.chisquare(observed).pvalue > 1e-4
     assert observed.sum() == 200 * R * steps
+
+
+def _weighted_ctx(deg, K, batch=64, n_total=400, seed=1):
+    """A context sampling K of the weighted edges of anchors 0.. of the given degrees."""
+    rng = np.random.default_rng(seed)
+    d = np.concatenate([np.asarray(deg), np.full(n_total - len(deg), 1)])
+    rows = np.zeros(n_total + 1, np.uint64)
+    rows[1:] = np.cumsum(d)
+    cols = rng.integers(0, n_total, int(rows[-1])).astype(np.uint32)
+    cdf = np.zeros(len(cols), np.float32)
+    for v in range(n_total):
+        s, e = int(rows[v]), int(rows[v + 1])
+        c = np.cumsum(rng.uniform(0.1, 5.0, e - s), dtype=np.float32)
+        cdf[s:e] = c / c[-1]
+    cfg = _native.default_config()
+    cfg.dims, cfg.negatives, cfg.loss, cfg.gamma = 8, 2, _native.LOSS_STARSPACE, 0.5
+    cfg.batch_size, cfg.passes, cfg.valid_pct = batch, 1, 0.0
+    cfg.max_nodes_kind, cfg.max_nodes = _native.SAMPLE_FIXED, float(K)
+    cfg.weighted_neighbor_sampling = cfg.weighted_neighbor_averaging = 1
+    ctx = _native.Context(cfg)
+    ctx.upload_graph(rows, cols, cdf)
+    ctx.upload_features(np.arange(n_total + 1, dtype=np.uint64), np.zeros(n_total, np.uint32), 97)
+    ctx.set_table(None)
+    return ctx
+
+
+@pytest.mark.parametrize("K", [1, 10, 32])
+def test_hubs_sampled_by_the_cta_or_by_their_warps(monkeypatch, K):
+    # anchors of more than 512 edges in CTAs of eight: all of them, one of
+    # them, none, two of one length (twice the longest: by the CTA), two and a
+    # little more (by their warps); a warp to a CTA has each to itself
+    deg = ([600] * 8 + [3000] + [40] * 7 + [512] * 8 + [700, 700] + [5] * 6 + [2000, 2000, 513] + [512] * 5 +
+           [513, 9000, 700, 800, 600, 40, 900, 1000] + [10_000])
+    out = []
+    for warps in ("8", "1", "3"):
+        monkeypatch.setenv("EP_SAMPLE_WARPS", warps)
+        ctx = _weighted_ctx(deg, K)
+        out.append([ctx.sample(np.arange(len(deg), dtype=np.uint32), step, K) for step in (1, 2)])
+    for other in out[1:]:
+        for a, b in zip(out[0], other):
+            for x, y in zip(a, b):
+                assert np.array_equal(x, y)
+    cnt = out[0][0][0]
+    assert (cnt == np.minimum(K, deg)).all()
+
+
+def test_batches_of_hubs_are_sampled_side_by_side(monkeypatch):
+    # every anchor a hub: eight of a CTA one after the other took 3.5 times as
+    # long as a CTA to each
+    stage = {}
+    for warps in ("8", "1"):
+        monkeypatch.setenv("EP_SAMPLE_WARPS", warps)
+        ctx = _weighted_ctx([1000] * 3000, 10, batch=1000, n_total=3000)
+        ctx.profile_batches(3)
+        stage[warps] = min(ctx.profile_batches(1)[0]["sample"] for _ in range(6))
+    assert stage["8"] < 2 * stage["1"], stage
