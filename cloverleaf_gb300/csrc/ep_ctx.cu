@@ -884,7 +884,7 @@ static int fused_out_mode(const ep_ctx* c) {
 }
 
 // Whether replayed batches sort by one kernel per pass (k_radix_pass).
-static bool one_kernel_sort(const ep_ctx* c) { return c->train_items <= RADIX_ONE_ITEMS; }
+static bool one_kernel_sort(const ep_ctx* c) { return c->train_items <= RADIX_ONE_ITEMS && c->items_cap <= RADIX_ONE_CAP; }
 
 // Kernels launched per training batch.
 static uint32_t kernels_per_batch(const ep_ctx* c, bool fork) {

@@ -87,7 +87,15 @@ constexpr uint32_t OCC_CAP = 512;     // feature occurrences of one anchor
 constexpr uint32_t ROLE_CAP = 34;     // R + 2
 
 constexpr uint32_t SORT_TILE = 2048;  // items a CTA of the radix sort takes at a time
-constexpr uint64_t RADIX_ONE_ITEMS = 200'000;   // typical batches up to this many items: one kernel per pass
+// Replayed batches sort by one kernel per pass (k_radix_pass) where a typical
+// batch has up to RADIX_ONE_ITEMS items and no batch can have more than
+// RADIX_ONE_CAP: every CTA reads the counts of all tiles, so the work grows
+// with the square of the items.  A whole replayed batch with three kernels per
+// pass / one, us: 41,000 items 65.7 / 59.6, 106,000 86.5 / 81.2, 164,000 89.3 /
+// 86.2, 212,000 114 / 125, 309,000 121 / 141, 954,000 184 / 237, 1.3 M 220 /
+// 306; a 7 M-item batch (a hub of 1.2 M edges, all neighbours taken) 575 / 607
+// ms, though the typical batch of that graph is the smallest of these.
+constexpr uint64_t RADIX_ONE_ITEMS = 175'000, RADIX_ONE_CAP = 1'000'000;
 
 // Feature dropout (max_features): EP_SAMPLE_* kind, Fixed count k,
 // Probability p and its key threshold p * 2^32, and the Philox key.

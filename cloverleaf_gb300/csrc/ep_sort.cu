@@ -39,7 +39,8 @@ static uint64_t sort_tiles(uint64_t cap) { return cap ? (cap + SORT_TILE - 1) / 
 static int sort_passes(int key_bits) { return key_bits <= 0 ? 1 : (key_bits + 7) / 8; }
 
 size_t radix_hist_entries(uint64_t cap) {
-    return (size_t)(256 * sort_tiles(cap) * MAX_PASSES) + 256;   // counts of every pass, digit totals
+    // the counts of every pass where one kernel per pass may be used, else of one; the digit totals
+    return (size_t)(256 * sort_tiles(cap) * (cap <= RADIX_ONE_CAP ? MAX_PASSES : 1)) + 256;
 }
 
 void radix_clear(uint32_t* hist, uint64_t cap, int key_bits, cudaStream_t s) {
@@ -192,9 +193,10 @@ __global__ void __launch_bounds__(SORT_THREADS) k_radix_scatter(const uint32_t* 
 // pass's counts; a CTA (a thread per digit) adds up the digit's counts over
 // all tiles and over the tiles before its own, scans the totals, and scatters
 // its tile, counting the next pass's digits at the items' new places in
-// next_hist.  The adding grows with the square of the tiles: for batches of up
-// to RADIX_ONE_ITEMS items.  A replayed batch of 22,000 items (sbm10k, 2
-// passes) 54.5 -> 46.3 us, of 162,000 (cl1m, 3 passes) 103 -> 97 us.
+// next_hist.  The adding grows with the square of the tiles, so it is for small
+// batches only (RADIX_ONE_ITEMS, RADIX_ONE_CAP).  A replayed batch of 22,000
+// items (sbm10k, 2 passes) 54.5 -> 46.3 us, of 164,000 (cl1m, 3 passes) 89.3
+// -> 86.2 us.
 __global__ void __launch_bounds__(SORT_THREADS) k_radix_pass(const uint32_t* __restrict__ keys_in,
                                                              const uint2* __restrict__ vals_in,
                                                              const uint32_t* __restrict__ item_src,

@@ -426,3 +426,39 @@ def test_one_kernel_sort_passes_match_three(form, n_feat, batch):
         st = ctx.train_batches(11)
         out.append((ctx.get_table(n_feat, 20), st["kept_anchors"], st["items"], st["gathered_rows"], st["unique_rows"]))
     assert out[0][1] > 0 and out[0][1:] == out[1][1:] and np.array_equal(out[0][0], out[1][0])
+
+
+@pytest.mark.parametrize("form", [_native.FORM_FUSED_BF16, _native.FORM_PLAIN_FP32])
+def test_one_kernel_sort_passes_only_where_no_batch_is_large(form):
+    # the one-kernel passes do work in the square of a batch's items: a graph
+    # whose typical batch is small, but where one hub's neighbourhood is not,
+    # sorts by three kernels per pass (2 passes here), as the launch counts say
+    def graph(hub):
+        n = 250_000
+        rows, cols = np.arange(n + 1, dtype=np.uint64), np.zeros(n, np.uint32)
+        if hub:     # node 0 next to all others
+            rows[1:] += n - 2
+            cols = np.concatenate([np.arange(1, n), np.zeros(n - 1)]).astype(np.uint32)
+        rng = np.random.default_rng(11)
+        fptr = np.arange(n + 1, dtype=np.uint64) * 5
+        return rows, cols, fptr, rng.integers(0, 40_000, 5 * n).astype(np.uint32)
+
+    kernels, out = {}, []
+    for hub, graphs in ((False, 1), (True, 1), (True, 0)):
+        rows, cols, fptr, fids = graph(hub)
+        cfg = _native.default_config()
+        cfg.use_graphs, cfg.form = graphs, form
+        cfg.dims, cfg.negatives, cfg.loss, cfg.gamma = 16, 3, _native.LOSS_STARSPACE, 0.5
+        cfg.batch_size, cfg.passes, cfg.valid_pct = 64, 1, 0.0
+        ctx = _native.Context(cfg)
+        ctx.upload_graph(rows, cols, None)
+        ctx.upload_features(fptr, fids, 40_000)
+        ctx.set_table(None)
+        st = ctx.train_batches(16)
+        assert st["kept_anchors"] > 0
+        kernels[hub, graphs] = st["launches"] / 16
+        if hub:
+            out.append((ctx.get_table(40_000, 16), st["kept_anchors"], st["items"], st["unique_rows"]))
+    # two more kernels in each pass, and the direct gather of anchors beyond the tables
+    assert kernels[True, 1] - kernels[False, 1] == 2 * 2 + 1, kernels
+    assert out[0][1:] == out[1][1:] and np.array_equal(out[0][0], out[1][0])
