@@ -143,6 +143,7 @@ struct ep_ctx {
 
     // host-side view of the pass sequence (mirrors the device BatchState)
     uint32_t host_pass = 1, host_batch = 0;
+    uint64_t issued = 0;     // training batches issued since the run was prepared
     uint64_t launches = 0;   // kernels issued by training batches (graph replays count their kernels)
     bool state_ok = false;
 
@@ -699,6 +700,7 @@ static int prepare_train(ep_ctx* c) {
     c->train_K = K;
     c->Kcap = c->buf_K;
     if (!c->graph_batches_set) c->graph_batches = pick_graph_batches(c->steps_per_pass, c->cfg.passes);
+    c->issued = 0;
     c->prepared = true;
     return EP_OK;
 }
@@ -1030,22 +1032,26 @@ static void issue_train_batch(ep_ctx* c, cudaEvent_t* ev = nullptr, bool fork = 
 }
 
 static void advance_host_batch(ep_ctx* c) {
+    ++c->issued;
     if (++c->host_batch >= c->steps_per_pass) { c->host_batch = 0; ++c->host_pass; }
 }
 
-// Whether batches are replayed.  A graph costs about 300 us to build and
-// destroy; replaying saves the launches of a small batch (about 30 us) and the
-// overlap of its branches (about 15% of a large one, taken as 0.3 us per
+// Whether a run of n batches is replayed.  A graph costs about 300 us to build
+// and destroy; replaying saves the launches of a small batch (about 30 us) and
+// the overlap of its branches (about 15% of a large one, taken as 0.3 us per
 // thousand items of 256 dims).  9,206 nodes, 20 FP32 dims, whole learn call in
 // us, replayed / launched: 8 batches 3,028 / 2,603, 10 2,670 / 2,731, 30 3,774
-// / 4,323.
-static bool replays(const ep_ctx* c) {
-    const double batches = (double)c->steps_per_pass * std::max<uint32_t>(c->cfg.passes, 1);
+// / 4,323.  The batches that count are those of the configured passes, or, on
+// a context driven for longer, those issued so far and this run's: 5 batches a
+// pass, one pass, 1,000 batches asked for, 48.8 us a batch replayed, 61.2
+// launched.
+static bool replays(const ep_ctx* c, uint32_t n) {
+    const double batches = std::max((double)c->steps_per_pass * std::max<uint32_t>(c->cfg.passes, 1), (double)c->issued + n);
     const double batch_us = (double)c->train_items * c->dims / 256. * 3e-4;
     return c->cfg.use_graphs && batches * (30. + 0.15 * batch_us) >= 300.;
 }
 
-static int launch_train_batch(ep_ctx* c);
+static int launch_train_batch(ep_ctx* c, bool use_graph);
 
 // Issues n consecutive training batches.  With graphs, runs of graph_batches
 // batches replay one graph holding that many copies of the batch (the
@@ -1097,7 +1103,7 @@ void apply_choice(ep_ctx* c, const TuneChoice& t) {
 
 // Times each candidate on real batches; returns the fastest (or the current
 // shape when a launch fails, with rc set).
-static int tune_stage(ep_ctx* c, const std::vector<TuneChoice>& cands, TuneChoice* pick) {
+static int tune_stage(ep_ctx* c, const std::vector<TuneChoice>& cands, TuneChoice* pick, bool use_graph) {
     if (cands.size() < 2) {
         if (!cands.empty()) *pick = cands[0];
         return EP_OK;
@@ -1109,9 +1115,9 @@ static int tune_stage(ep_ctx* c, const std::vector<TuneChoice>& cands, TuneChoic
     int rc = EP_OK;
     for (size_t i = 0; i < cands.size() && !rc; ++i) {
         apply_choice(c, cands[i]);
-        for (uint32_t b = 0; b < kTuneWarm && !rc; ++b) rc = launch_train_batch(c);
+        for (uint32_t b = 0; b < kTuneWarm && !rc; ++b) rc = launch_train_batch(c, use_graph);
         cudaEventRecord(e0, c->stream);
-        for (uint32_t b = 0; b < kTuneTimed && !rc; ++b) rc = launch_train_batch(c);
+        for (uint32_t b = 0; b < kTuneTimed && !rc; ++b) rc = launch_train_batch(c, use_graph);
         cudaEventRecord(e1, c->stream);
         if (rc) break;
         if (cudaEventSynchronize(e1) != cudaSuccess) { rc = c->cuda_fail(cudaGetLastError(), "tuning"); break; }
@@ -1164,7 +1170,7 @@ static void tune_candidates(const ep_ctx* c, std::vector<TuneChoice>& s1, uint32
     need = (uint32_t)((s1.size() > 1 ? s1.size() : 0) + 5) * (kTuneWarm + kTuneTimed);
 }
 
-static int autotune(ep_ctx* c, uint32_t& n) {
+static int autotune(ep_ctx* c, uint32_t& n, bool use_graph) {
     if (tune_from_cache(c)) return EP_OK;
     const TuneChoice cur = {c->chunk, c->fused_mode, c->gather_ctas, c->ring_pw, c->ring_cw, c->ring_slots, c->queue_ctas,
                            c->gather_warps};
@@ -1176,7 +1182,7 @@ static int autotune(ep_ctx* c, uint32_t& n) {
     // anchor in CTAs of 2, 4 or 8 warps, or persistent at 2 or 3 CTAs per SM
     const uint32_t gathers[5][2] = {{0, 2}, {0, 4}, {0, 8}, {2 * 152, 8}, {3 * 152, 8}};
     TuneChoice pick = cur;
-    int rc = tune_stage(c, s1, &pick);
+    int rc = tune_stage(c, s1, &pick, use_graph);
     std::vector<TuneChoice> s2;
     for (const auto& g : gathers) {
         TuneChoice t = pick;
@@ -1184,7 +1190,7 @@ static int autotune(ep_ctx* c, uint32_t& n) {
         t.gwarps = g[1];
         s2.push_back(t);
     }
-    if (!rc) rc = tune_stage(c, s2, &pick);
+    if (!rc) rc = tune_stage(c, s2, &pick, use_graph);
     if (rc) {
         apply_choice(c, cur);
         return rc;
@@ -1219,7 +1225,7 @@ static int capture_batches(ep_ctx* c, uint32_t batches, cudaGraphExec_t* out) {
 // Builds, ahead of a run of n batches, the graphs that run will replay, so
 // that the one-time capture and instantiation stay outside its timing.
 static int prepare_graphs(ep_ctx* c, uint32_t n) {
-    if (!replays(c) || n == 0) return EP_OK;
+    if (!replays(c, n) || n == 0) return EP_OK;
     if (c->cfg.autotune && !tune_from_cache(c)) {
         std::vector<TuneChoice> s1;
         uint32_t need = 0;
@@ -1240,11 +1246,11 @@ static int prepare_graphs(ep_ctx* c, uint32_t n) {
 }
 
 static int launch_train_run(ep_ctx* c, uint32_t n) {
+    const bool use_graph = replays(c, n);
     if (c->cfg.autotune && !c->tuned) {
-        int rc = autotune(c, n);
+        int rc = autotune(c, n, use_graph);
         if (rc) return rc;
     }
-    const bool use_graph = replays(c);
     const uint32_t k = c->graph_batches;
     while (n) {
         if (use_graph && k > 1 && n >= k) {
@@ -1271,7 +1277,7 @@ static int launch_train_run(ep_ctx* c, uint32_t n) {
             for (uint32_t i = 0; i < n; ++i) advance_host_batch(c);
             n = 0;
         } else {
-            int rc = launch_train_batch(c);
+            int rc = launch_train_batch(c, use_graph);
             if (rc) return rc;
             --n;
         }
@@ -1279,8 +1285,7 @@ static int launch_train_run(ep_ctx* c, uint32_t n) {
     return EP_OK;
 }
 
-static int launch_train_batch(ep_ctx* c) {
-    const bool use_graph = replays(c);
+static int launch_train_batch(ep_ctx* c, bool use_graph) {
     if (use_graph) {
         if (!c->gexec) {
             int rc = capture_batches(c, 1, &c->gexec);

@@ -462,3 +462,37 @@ def test_one_kernel_sort_passes_only_where_no_batch_is_large(form):
     # two more kernels in each pass, and the direct gather of anchors beyond the tables
     assert kernels[True, 1] - kernels[False, 1] == 2 * 2 + 1, kernels
     assert out[0][1:] == out[1][1:] and np.array_equal(out[0][0], out[1][0])
+
+
+def _small_run(form, passes, graphs=1, steps=5):
+    from tests._cases import random_problem
+    prob = random_problem(94, n=steps * 60, n_feat=300, dims=16, deg=(1, 6), feats=(1, 4))
+    cfg = _native.default_config()
+    cfg.use_graphs, cfg.form = graphs, form
+    cfg.dims, cfg.negatives, cfg.loss, cfg.gamma = 16, 3, _native.LOSS_STARSPACE, 0.5
+    cfg.batch_size, cfg.passes, cfg.valid_pct, cfg.autotune = 60, passes, 0.0, 0
+    ctx = _native.Context(cfg)
+    ctx.upload_graph(prob["rows"], prob["cols"], None)
+    ctx.upload_features(prob["fptr"], prob["fids"], 300)
+    ctx.set_table(None)
+    return ctx
+
+
+@pytest.mark.parametrize("form", [_native.FORM_FUSED_BF16, _native.FORM_PLAIN_FP32])
+def test_long_runs_of_short_passes_are_replayed(form):
+    # replayed batches have other kernels than launched ones (item emission,
+    # one-kernel sort passes): the launch counts say which a run took
+    replayed = _small_run(form, passes=100).train_batches(200)["launches"] / 200
+    launched = _small_run(form, passes=100, graphs=0).train_batches(200)["launches"] / 200
+    assert replayed != launched
+    ctx = _small_run(form, passes=1)
+    assert ctx.train_batches(5)["launches"] == 5 * launched      # as configured: too short to pay
+    assert ctx.train_batches(300)["launches"] == 300 * replayed
+    # as many batches one at a time: replayed once they have come to a run that pays
+    one = _small_run(form, passes=1)
+    per = [one.train_batches(1)["launches"] for _ in range(305)]
+    assert per[0] == launched and per[-1] == replayed and per == sorted(per, key=lambda x: x == replayed)
+    ref = _small_run(form, passes=1, graphs=0)
+    ref.train_batches(305)
+    want = ref.get_table(300, 16)
+    assert np.array_equal(ctx.get_table(300, 16), want) and np.array_equal(one.get_table(300, 16), want)
