@@ -128,7 +128,7 @@ struct ep_ctx {
     bool prepared = false;
     cudaGraphExec_t gexec = nullptr;
     cudaGraphExec_t gexec_run = nullptr;   // graph_batches consecutive batches
-    std::map<uint32_t, cudaGraphExec_t> gexec_rem;   // 2 .. graph_batches - 1 consecutive batches (a run's remainder)
+    std::map<uint32_t, cudaGraphExec_t> gexec_rem;   // a run's remainder, by its batches (2 .. max(graph_batches - 1, MAX_WHOLE))
     uint32_t graph_batches = 16;
     bool graph_batches_set = false;   // by the environment
     uint32_t* sorted_keys = nullptr;
@@ -643,15 +643,34 @@ static int top_sum_bound(ep_ctx* c, uint32_t n, uint32_t top, uint64_t* out) {
 // record, instantiate, upload and destroy (2.7 ms for 30 batches of 20
 // kernels), and every replay about 20 us at its boundary, where a batch's
 // fix-ups are joined instead of running beside the next batch's sampling.  A
-// pass replays steps / g graphs of g batches and one of the remainder.
+// pass replays steps / g graphs of g batches and one of the remainder; one of
+// up to MAX_WHOLE batches may also be a single graph (g = 1, run_remainder).
+constexpr uint32_t MAX_WHOLE = 16;
+
 static uint32_t pick_graph_batches(uint32_t steps, uint32_t passes) {
     uint32_t best = 1;
     double least = 1e300;
-    for (uint32_t g = 1; g <= 16 && g <= std::max<uint32_t>(steps, 1); ++g) {
+    for (uint32_t g = steps > MAX_WHOLE ? 2 : 1; g <= 16 && g <= std::max<uint32_t>(steps, 1); ++g) {
         const double cost = 90. * (g + steps % g) + 20. * ((double)steps / g) * std::max<uint32_t>(passes, 1);
         if (cost < least) { least = cost; best = g; }
     }
     return best;
+}
+
+// The graph size is chosen for the configured passes; where those are too
+// short for graphs of several batches and a run takes the context past them,
+// for that run.
+static void plan_graphs(ep_ctx* c, uint32_t n) {
+    if (c->graph_batches_set || c->graph_batches > 1) return;
+    if (c->issued + n > (uint64_t)c->steps_per_pass * std::max<uint32_t>(c->cfg.passes, 1))
+        c->graph_batches = pick_graph_batches(n, 1);
+}
+
+// What of a run of n batches is left over for a graph of its own size, after
+// the graphs of graph_batches.
+static uint32_t run_remainder(const ep_ctx* c, uint32_t n) {
+    if (c->graph_batches > 1) return n % c->graph_batches;
+    return n <= MAX_WHOLE ? n : 0;
 }
 
 static int prepare_train(ep_ctx* c) {
@@ -1057,7 +1076,9 @@ static int launch_train_batch(ep_ctx* c, bool use_graph);
 // batches replay one graph holding that many copies of the batch (the
 // device-resident BatchState moves each copy to the next batch, crossing pass
 // boundaries as the device would); a remainder of r >= 2 batches replays a
-// graph of r batches, a single batch the one-batch graph.
+// graph of r batches, a single batch the one-batch graph.  With graphs of one
+// batch, a run of up to MAX_WHOLE replays one graph of its length, a longer one
+// the one-batch graph for each.
 //
 // The autotuner (config.autotune) times kTuneTimed batches after kTuneWarm
 // warm-up batches under each candidate launch shape and keeps the fastest.
@@ -1232,11 +1253,12 @@ static int prepare_graphs(ep_ctx* c, uint32_t n) {
         tune_candidates(c, s1, need);
         if (n >= need) return EP_OK;   // this run starts with the tuner, which rebuilds them per candidate
     }
+    plan_graphs(c, n);
     const uint32_t k = c->graph_batches;
     int rc = EP_OK;
     if (k > 1 && n >= k && !c->gexec_run) rc = capture_batches(c, k, &c->gexec_run);
-    const uint32_t r = k > 1 ? n % k : 1;
-    if (!rc && r == 1 && !c->gexec) rc = capture_batches(c, 1, &c->gexec);
+    const uint32_t r = run_remainder(c, n);
+    if (!rc && (r == 1 || (k == 1 && !r)) && !c->gexec) rc = capture_batches(c, 1, &c->gexec);
     if (!rc && r >= 2 && !c->gexec_rem.count(r)) {
         cudaGraphExec_t g = nullptr;
         rc = capture_batches(c, r, &g);
@@ -1251,7 +1273,8 @@ static int launch_train_run(ep_ctx* c, uint32_t n) {
         int rc = autotune(c, n, use_graph);
         if (rc) return rc;
     }
-    const uint32_t k = c->graph_batches;
+    if (use_graph) plan_graphs(c, n);
+    const uint32_t k = c->graph_batches, rem = run_remainder(c, n);
     while (n) {
         if (use_graph && k > 1 && n >= k) {
             if (!c->gexec_run) {
@@ -1262,7 +1285,7 @@ static int launch_train_run(ep_ctx* c, uint32_t n) {
             c->launches += (uint64_t)k * kernels_per_batch(c, true);
             for (uint32_t i = 0; i < k; ++i) advance_host_batch(c);
             n -= k;
-        } else if (use_graph && n >= 2) {
+        } else if (use_graph && n >= 2 && n == rem) {
             // the run's remainder as one graph of n batches: their fix-ups
             // overlap the next batch's sampling as in the full-size graph
             auto it = c->gexec_rem.find(n);

@@ -496,3 +496,25 @@ def test_long_runs_of_short_passes_are_replayed(form):
     ref.train_batches(305)
     want = ref.get_table(300, 16)
     assert np.array_equal(ctx.get_table(300, 16), want) and np.array_equal(one.get_table(300, 16), want)
+
+
+def test_graph_size_follows_the_run(monkeypatch):
+    # a run far past the configured passes takes graphs of several batches,
+    # not one graph of the whole run
+    ref = _small_run(_native.FORM_FUSED_BF16, passes=1, graphs=0, steps=5)
+    ref.train_batches(5 + 500 + 17)
+    want = ref.get_table(300, 16)
+    ctx = _small_run(_native.FORM_FUSED_BF16, passes=1, steps=5)
+    ctx.train_batches(5)
+    assert ctx.launch_shape()["graph_batches"] == 1
+    ctx.train_batches(500)
+    assert 2 <= ctx.launch_shape()["graph_batches"] <= 16
+    ctx.train_batches(17)
+    assert np.array_equal(ctx.get_table(300, 16), want)
+    # graphs of one batch: whole runs of up to 16, else batch by batch
+    monkeypatch.setenv("EP_GRAPH_BATCHES", "1")
+    one = _small_run(_native.FORM_FUSED_BF16, passes=1, steps=5)
+    for n in (5, 1, 17, 499):
+        one.train_batches(n)
+    assert one.launch_shape()["graph_batches"] == 1
+    assert np.array_equal(one.get_table(300, 16), want)
