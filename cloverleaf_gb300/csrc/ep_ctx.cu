@@ -139,7 +139,8 @@ struct ep_ctx {
     uint32_t* h_pack = nullptr;
     size_t h_pack_words = 0;
     DevBuf pack;
-    cudaEvent_t ev_pack = nullptr;   // that copy is done
+    cudaEvent_t ev_pack = nullptr;   // the last batch's samples (and table) are where the kernels read them
+    cudaEvent_t ev_order = nullptr;  // see follow()
 
     // host-side view of the pass sequence (mirrors the device BatchState)
     uint32_t host_pass = 1, host_batch = 0;
@@ -154,12 +155,14 @@ struct ep_ctx {
     const void* ag_table_ptr = nullptr;
 
     ~ep_ctx() {
+        if (ev_pack) cudaEventSynchronize(ev_pack);     // ep_ag_stage may be pending on a caller's stream
         if (gexec) cudaGraphExecDestroy(gexec);
         if (gexec_run) cudaGraphExecDestroy(gexec_run);
         for (auto& kv : gexec_rem) cudaGraphExecDestroy(kv.second);
         if (h_st) cudaFreeHost(h_st);   // with h_inj
         if (h_pack) cudaFreeHost(h_pack);
         if (ev_pack) cudaEventDestroy(ev_pack);
+        if (ev_order) cudaEventDestroy(ev_order);
         if (ev_fork) cudaEventDestroy(ev_fork);
         if (ev_join) cudaEventDestroy(ev_join);
         if (ev_loss) cudaEventDestroy(ev_loss);
@@ -284,6 +287,7 @@ extern "C" int ep_create(const ep_config* cfg, ep_ctx** out) {
         cudaEventCreateWithFlags(&c->ev_loss, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_sorted, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_pack, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&c->ev_order, cudaEventDisableTiming) != cudaSuccess ||
         cudaMallocHost((void**)&c->h_st, 2 * sizeof(BatchState)) != cudaSuccess || reduce_kernels_setup() != cudaSuccess) {
         g_create_err = std::string("CUDA setup failed: ") + cudaGetErrorString(cudaGetLastError());
         delete c;
@@ -516,6 +520,13 @@ extern "C" int ep_get_table(ep_ctx* c, float* out) {
     return EP_OK;
 }
 
+// What is issued to `to` from here on follows all that `from` holds.
+static cudaError_t follow(ep_ctx* c, cudaStream_t to, cudaStream_t from) {
+    if (to == from) return cudaSuccess;
+    const cudaError_t e = cudaEventRecord(c->ev_order, from);
+    return e == cudaSuccess ? cudaStreamWaitEvent(to, c->ev_order, 0) : e;
+}
+
 // (Re)allocates per-batch scratch for B anchors, K neighbour slots, `items`
 // gradient items and accumulator element size es.
 static int ensure_bufs(ep_ctx* c, uint32_t B, uint32_t K, uint64_t items, uint32_t es, bool dense) {
@@ -523,6 +534,7 @@ static int ensure_bufs(ep_ctx* c, uint32_t B, uint32_t K, uint64_t items, uint32
     items = std::max<uint64_t>(items, 1);
     bool grow = B > c->buf_B || K > c->buf_K || items > c->items_cap || es > c->buf_es;
     if (grow) {
+        CK(cudaEventSynchronize(c->ev_pack), "batch scratch");      // ep_ag_stage returns with its work pending
         B = std::max(B, c->buf_B);
         K = std::max(K, c->buf_K);
         items = std::max(items, c->items_cap);
@@ -1527,16 +1539,15 @@ static int stage_samples(ep_ctx* c, const ep_batch_samples* sm, uint32_t es, cud
     c->typ_items = (uint64_t)((double)c->n_fids / (double)c->n_nodes * ((double)B * (1. + c->R) + nn));
     int rc = ensure_bufs(c, B, K, items, es, true);
     if (rc) return rc;
-    // one page-locked copy of everything
+    // one page-locked copy of everything; the last one has left its buffers
     const size_t words = 2 * (size_t)B + 1 + 2 * (size_t)nn + (size_t)B * c->R;
+    CK(cudaEventSynchronize(c->ev_pack), "staging memory");
     if (c->h_pack_words < words) {
         if (c->h_pack) cudaFreeHost(c->h_pack);
         c->h_pack = nullptr;
         c->h_pack_words = 0;
         CK(cudaMallocHost((void**)&c->h_pack, 2 * words * 4), "staging memory");
         c->h_pack_words = 2 * words;
-    } else {
-        CK(cudaEventSynchronize(c->ev_pack), "staging memory");      // the last copy from it
     }
     if (!c->pack.ensure(words * 4)) return c->fail(EP_ERR_OOM, "staging allocation failed");
     uint32_t* p = c->h_pack;
@@ -1549,12 +1560,14 @@ static int stage_samples(ep_ctx* c, const ep_batch_samples* sm, uint32_t es, cud
         memcpy(p + nn, sm->nbr_w + n0, (size_t)nn * 4);
     }
     memcpy(p + 2 * (size_t)nn, sm->negatives, (size_t)B * c->R * 4);
+    // the context's stream uploads the graph and clears and uses this scratch
+    CK(follow(c, s, c->stream), "stage samples");
     CK(cudaMemcpyAsync(c->pack.p, c->h_pack, words * 4, cudaMemcpyHostToDevice, s), "stage samples");
-    CK(cudaEventRecord(c->ev_pack, s), "stage samples");
     k_stage_samples<<<(B + 7) / 8, 256, 0, s>>>(c->pack.as<uint32_t>(), B, nn, c->R, c->buf_K, c->anchors.as<uint32_t>(),
                                                 c->nbr.as<uint32_t>(), c->nbr_w.as<float>(), c->nbr_cnt.as<uint32_t>(),
                                                 c->neg.as<uint32_t>());
     CK(cudaGetLastError(), "stage samples");
+    CK(cudaEventRecord(c->ev_pack, s), "stage samples");
     return EP_OK;
 }
 
@@ -1770,6 +1783,9 @@ static int ag_prepare(ep_ctx* c, const ep_batch_samples* sm, int precision, cons
                              c->n_feat, cudaMemcpyDeviceToDevice, s), "table staging");
         c->ag_table_ptr = c->ag_table.p;
     }
+    // what comes next may be on the context's stream, or on a third one behind it
+    CK(cudaEventRecord(c->ev_pack, s), "stage samples");
+    CK(follow(c, c->stream, s), "stage samples");
     return EP_OK;
 }
 
