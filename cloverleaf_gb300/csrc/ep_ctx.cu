@@ -1789,11 +1789,21 @@ static int ag_prepare(ep_ctx* c, const ep_batch_samples* sm, int precision, cons
     return EP_OK;
 }
 
+// The stream of an autograd call.  NULL is the context's stream, which does not
+// wait for the legacy default stream by itself: a caller that works there (as
+// torch does unless told otherwise) may still be computing the table or the
+// upstream gradient.
+static cudaError_t ag_stream(ep_ctx* c, void* stream, cudaStream_t* s) {
+    *s = stream ? (cudaStream_t)stream : c->stream;
+    return stream ? cudaSuccess : follow(c, c->stream, cudaStreamLegacy);
+}
+
 extern "C" int ep_ag_forward(ep_ctx* c, const ep_batch_samples* sm, int precision, const void* table_dev, void* loss_dev,
                              void* stream) {
     if (!c || !table_dev || !loss_dev) return c ? c->fail(EP_ERR_INVALID_ARG, "null pointer") : EP_ERR_INVALID_ARG;
     cudaSetDevice(c->device);
-    cudaStream_t s = stream ? (cudaStream_t)stream : c->stream;
+    cudaStream_t s;
+    CK(ag_stream(c, stream, &s), "caller's stream");
     int rc = ag_prepare(c, sm, precision, table_dev, s);
     if (rc) return rc;
     // the losses alone: items, sort and reduction belong to the backward
@@ -1804,14 +1814,17 @@ extern "C" int ep_ag_forward(ep_ctx* c, const ep_batch_samples* sm, int precisio
 extern "C" int ep_ag_stage(ep_ctx* c, const ep_batch_samples* sm, int precision, const void* table_dev, void* stream) {
     if (!c || !table_dev) return c ? c->fail(EP_ERR_INVALID_ARG, "null pointer") : EP_ERR_INVALID_ARG;
     cudaSetDevice(c->device);
-    return ag_prepare(c, sm, precision, table_dev, stream ? (cudaStream_t)stream : c->stream);
+    cudaStream_t s;
+    CK(ag_stream(c, stream, &s), "caller's stream");
+    return ag_prepare(c, sm, precision, table_dev, s);
 }
 
 extern "C" int ep_ag_backward(ep_ctx* c, const void* dloss_dev, void* grad_dev, void* stream) {
     if (!c || !dloss_dev || !grad_dev) return c ? c->fail(EP_ERR_INVALID_ARG, "null pointer") : EP_ERR_INVALID_ARG;
     if (c->ag_precision < 0) return c->fail(EP_ERR_STATE, "call ep_ag_forward first");
     cudaSetDevice(c->device);
-    cudaStream_t s = stream ? (cudaStream_t)stream : c->stream;
+    cudaStream_t s;
+    CK(ag_stream(c, stream, &s), "caller's stream");
     const int tt = c->ag_precision ? TT_F64 : TT_F32;
     const size_t es = c->ag_precision ? 8 : 4;
     CK(cudaMemsetAsync(grad_dev, 0, (size_t)c->n_feat * c->dims * es, s), "clear gradient");

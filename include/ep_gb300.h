@@ -295,8 +295,8 @@ int ep_get_table_static(ep_ctx* ctx, uint64_t first_row, uint64_t n_rows, float*
  * and the table of the context's last ep_ag_forward or ep_ag_stage, which
  * must still be there.  ep_ag_stage sets these without computing the losses
  * (a backward that comes after other calls on the context).  All run on
- * `stream` (a cudaStream_t, NULL = the context stream); ep_ag_stage does not
- * wait for it, so the backward after it takes the same stream. */
+ * `stream` (a cudaStream_t; NULL = the context stream, after what the legacy
+ * default stream holds); ep_ag_stage does not wait for it, so the backward after it takes the same stream. */
 int ep_ag_forward(ep_ctx* ctx, const ep_batch_samples* samples, int precision,
                   const void* table_dev, void* loss_dev, void* stream);
 int ep_ag_stage(ep_ctx* ctx, const ep_batch_samples* samples, int precision, const void* table_dev, void* stream);

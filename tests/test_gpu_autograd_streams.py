@@ -129,3 +129,41 @@ def test_first_batch_on_a_side_stream_behind_the_upload():
             out.append((lv.detach().cpu(), t.grad.cpu()))
     for lv, g in out[1:]:
         assert torch.equal(lv, out[0][0]) and torch.equal(g, out[0][1])
+
+
+@pytest.mark.parametrize("dims", [20, 64])
+@pytest.mark.parametrize("default", [True, False])
+def test_table_and_upstream_gradient_still_being_computed(dims, default):
+    # the kernels that write the table and the upstream gradient are pending on
+    # the caller's stream, the default stream or another, when the call is made
+    prob, f = _loss(dims)
+    args = _args(prob, 100, 9)
+    want_loss, want = _grad(_loss(dims)[1], prob["table"], args)
+    src = torch.tensor(prob["table"], device="cuda")
+    weight = torch.linspace(0.5, 2.0, 100, device="cuda")
+    f(src, *args)                       # scratch is allocated
+    stream = torch.cuda.default_stream() if default else torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(stream):
+        t = torch.full_like(src, 7.0).requires_grad_()
+        torch.cuda._sleep(WAIT)
+        with torch.no_grad():
+            t.copy_(src)
+        assert not stream.query()
+        lv = f(t, *args)
+        lv.sum().backward()
+        assert np.array_equal(lv.detach().cpu().numpy(), want_loss, equal_nan=True)
+        assert np.array_equal(t.grad.cpu().numpy(), want)
+        # the same upstream gradient, late and at once
+        grads = []
+        for late in (False, True):
+            t.grad = None
+            lv = f(t, *args)
+            torch.cuda.synchronize()
+            up = torch.full_like(weight, 3.0)
+            if late:
+                torch.cuda._sleep(WAIT)
+            up.copy_(weight)
+            lv.backward(up)
+            grads.append(t.grad.cpu().numpy())
+        assert np.array_equal(grads[0], grads[1]) and not np.array_equal(grads[0], want)
