@@ -986,6 +986,7 @@ static void issue_train_batch(ep_ctx* c, cudaEvent_t* ev = nullptr, bool fork = 
         cudaEventRecord(c->ev_sorted, c->side);
         ForwardParams fp = forward_params(c, st, c->table.p, false, false);
         fp.means_dead = 1;
+        fp.beside_sort = 1;
         // the direct gathers beside the staged ones, on the long fix-ups'
         // stream (behind the previous batch's fix-ups: they update the table)
         const bool direct = may_defer(c, c->train_K);

@@ -1986,12 +1986,24 @@ void launch_scan_occ(BatchState* st, uint32_t* occ, uint32_t cap, uint64_t items
 // Warps per anchor of the staged gather, by the batch's anchors.  One warp
 // each fills the chip's 152 x 32 gather slots from about 5,000 anchors on;
 // below that, the time is one anchor's chain, which more warps shorten until
-// they wait for each other.  Forward stage in us at 1 / 2 / 4 / 8 warps: 225
-// anchors (sbm10k, 64 FP32) 25.1 / 21.4 / 20.9 / 20.5; 1,024 (cl1m, 128 FP32)
-// 47.6 / 38.0 / 37.5 / 42.2; 8,192 (cl10m, 256 BF16) 110 / 118 / - / -.
+// they wait for each other, or, in a replayed batch, take the slots of the
+// emission and sort that run beside them.
+//   Alone, forward stage in us at 1 / 2 / 4 warps (128 FP32): 225 anchors (64
+//   FP32) 25.1 / 21.4 / 20.9; 1,024 48.1 / 38.4 / 37.4; 1,536 51.1 / 40.1 /
+//   44.1; 2,560 52.5 / 49.6 / 53.0; 4,096 58.5 / 58.5 / 66.5.
+//   Replayed, whole batch: 512 anchors (64 FP32) 52.9 / 51.2 / 51.2; 1,000 (256
+//   BF16) 94.6 / 87.1 / 89.5, (128 FP32) 104.5 / 98.1 / 96.8; 1,280 (100 BF16) - /
+//   94.1 / 104.8.  Then by the bytes of a row: (256 BF16) 1,536 109 / 114 / 116,
+//   2,048 127 / 137 / 143, 4,096 176 / 192 / 199; (128 FP32) 1,536 113.5 / 108.4
+//   / 111.3, 2,048 117.1 / 117.3 / 120.7, 2,560 129 / 135 / 139, 4,096 167 / 173
+//   / 180; (256 FP32) 1,400 139 / - / 134, 2,600 172 / 165 / -, 3,600 209 / 204 /
+//   -, 4,096 223 / 221 / -.
+template <typename T, int VPL>
 static uint32_t gather_split(const ForwardParams& p, uint32_t cap) {
     if (p.gather_split) return p.gather_split;
-    return cap <= 2048 ? 4 : (cap <= 4096 ? 2 : 1);
+    if (!p.beside_sort) return cap <= 1280 ? 4 : (cap <= 3072 ? 2 : 1);
+    const uint32_t two = sizeof(T) == 2 ? 1280 : (VPL <= 4 ? 2048 : 4096);
+    return cap <= 1024 ? 4 : (cap <= two ? 2 : 1);
 }
 
 template <typename T, typename A, int VPL>
@@ -2018,7 +2030,7 @@ static void fwd_launch(const ForwardParams& p, uint32_t cap, cudaStream_t s, int
     const uint32_t gw = p.gather_warps >= 1 && p.gather_warps <= (uint32_t)FWD_WARPS ? p.gather_warps : FWD_WARPS;
     const uint32_t gblocks = (cap + gw - 1) / gw;
     const size_t gsmem = sizeof(GatherTables) * gw, one = sizeof(GatherTables);
-    const uint32_t split = gather_split(p, cap);
+    const uint32_t split = gather_split<T, VPL>(p, cap);
     if (p.gather_ctas > 2 * 152)
         launch_chain(k_fwd_gather_queue<T, A, VPL, 3>, std::min(p.gather_ctas, blocks), 32 * FWD_WARPS, smem, s, p);
     else if (p.gather_ctas)

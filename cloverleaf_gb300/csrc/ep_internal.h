@@ -178,6 +178,7 @@ struct ForwardParams {
     uint8_t* deferred;        // [n_anchors]: 1 = anchor left to k_fwd_direct (set by k_sample)
     uint32_t gather_warps;    // warps per CTA of the one-warp-per-anchor gather and item emission (1-8; 0 = 8)
     uint32_t gather_split;    // warps per anchor of the staged gather (1, 2, 4; 0 = by batch size)
+    int beside_sort;          // the item emission and sort run beside the gather (launch shape only)
     uint32_t gather_ctas;     // staged gather: 0 = a warp per anchor; else this many persistent CTAs
                               // whose warps take anchors from BatchState::fwd_next
     // outputs

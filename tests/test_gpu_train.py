@@ -518,3 +518,27 @@ def test_graph_size_follows_the_run(monkeypatch):
         one.train_batches(n)
     assert one.launch_shape()["graph_batches"] == 1
     assert np.array_equal(one.get_table(300, 16), want)
+
+
+@pytest.mark.parametrize("form", [_native.FORM_FUSED_BF16, _native.FORM_PLAIN_FP32])
+@pytest.mark.parametrize("batch", [1024, 1025, 1281, 2049, 3073, 4097])
+def test_gather_split_by_batch_size_gives_the_same_table(monkeypatch, form, batch):
+    # batch sizes on either side of each line of the rule, replayed (the sort
+    # beside the gather) and launched
+    from tests._cases import random_problem
+    prob = random_problem(93, n=9000, n_feat=4000, dims=130, deg=(1, 12), feats=(1, 6))
+    tables = []
+    for split, graphs in ((None, 1), (None, 0), ("1", 1)):
+        if split:
+            monkeypatch.setenv("EP_GATHER_SPLIT", split)
+        cfg = _native.default_config()
+        cfg.use_graphs, cfg.form = graphs, form
+        cfg.dims, cfg.negatives, cfg.loss, cfg.gamma = 130, 5, _native.LOSS_STARSPACE, 0.5
+        cfg.batch_size, cfg.passes, cfg.valid_pct, cfg.autotune = batch, 20, 0.0, 0
+        ctx = _native.Context(cfg)
+        ctx.upload_graph(prob["rows"], prob["cols"], None)
+        ctx.upload_features(prob["fptr"], prob["fids"], 4000)
+        ctx.set_table(None)
+        assert ctx.train_batches(7)["kept_anchors"] > 0
+        tables.append(ctx.get_table(4000, 130))
+    assert all(np.array_equal(tables[0], t) for t in tables[1:])
