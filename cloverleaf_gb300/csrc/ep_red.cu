@@ -44,7 +44,8 @@ enum : uint32_t { CF_HEAD = 1u, CF_THROUGH = 2u, CF_HEAD_KEPT = 8u, CF_OWNER = 4
 constexpr int RED_THREADS = 256;
 constexpr int FIX_THREADS = 128;
 constexpr uint32_t RED_MAX_CTAS = 152 * 8;
-constexpr uint32_t RED_SPLIT_CHUNKS = 3648;   // batches of up to this many chunks take several warps per chunk
+constexpr uint32_t RED_SPLIT_CHUNKS = 152 * 24;   // batches of up to this many chunks take several warps per chunk
+constexpr uint32_t RED_SPLIT4_CHUNKS = 152 * 9;   // ... four
 
 uint32_t reduce_chunks(uint64_t cap, uint32_t chunk) { return (uint32_t)((cap + chunk - 1) / chunk); }
 
@@ -685,15 +686,18 @@ __device__ __forceinline__ bool span_is_long(const ReduceParams& p, uint32_t c, 
 // Warps per chunk.  A chunk's features are independent sums, so its warps
 // take consecutive ranges of features, each feature still summed by one warp
 // in item order.  Small batches leave the chip idle at a warp per chunk, and
-// their time is one chunk's chain: reduce stage in us at 1 / 2 / 4 warps, 29
-// chunks (100 FP32) 24.3 / 18.7 / 15.1; 531 (100 BF16, queued Adam) 55.6 /
-// 33.8 / 23.8; 1,270 (128 FP32) 43.6 / 28.8 / 27.0.  From about 3,600 chunks
-// on, two warps gain nothing (6,500 chunks: 135.2 / 135.1).
+// their time is one chunk's chain.  Whole replayed batch in us at 1 / 2 / 4
+// warps: 566 chunks (256 BF16) 149 / 93.5 / 79.1, (256 FP32) 134 / 115 / 112;
+// 1,298 (128 FP32) 116 / 103 / 97.1, (100 BF16) 122 / 98.5 / 92.0; 1,462 (256
+// BF16) 179 / 129 / 127, (256 FP32) 167 / 141 / 152; 1,767 (128 FP32) 121 / 107
+// / 109; 1,946 (256 BF16) 191 / 144 / 152; 3,322 (256 FP32) 223 / 220 / -, (256
+// BF16) 218 / 191 / -; 4,056 (256 FP32) 251 / 260 / -; 5,189 (128 FP32) 173 /
+// 174 / -.  So four up to 9 chunks an SM, two up to 24.
 __device__ __forceinline__ uint32_t chunk_split(const ReduceParams& p) {
     const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
     const uint32_t nchunks = (p.st->n_items + p.chunk - 1) / p.chunk;
     uint32_t w = p.red_split;
-    if (!w) w = nchunks <= 1824u ? 4u : (nchunks <= RED_SPLIT_CHUNKS ? 2u : 1u);
+    if (!w) w = nchunks <= RED_SPLIT4_CHUNKS ? 4u : (nchunks <= RED_SPLIT_CHUNKS ? 2u : 1u);
     while (w > 1 && nchunks * w > warps) w >>= 1;
     return w;
 }

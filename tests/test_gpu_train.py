@@ -542,3 +542,31 @@ def test_gather_split_by_batch_size_gives_the_same_table(monkeypatch, form, batc
         assert ctx.train_batches(7)["kept_anchors"] > 0
         tables.append(ctx.get_table(4000, 130))
     assert all(np.array_equal(tables[0], t) for t in tables[1:])
+
+
+@pytest.mark.parametrize("form", [_native.FORM_FUSED_BF16, _native.FORM_PLAIN_FP32])
+@pytest.mark.parametrize("chunks", [1360, 1376, 3640, 3660])
+def test_reducer_split_by_chunk_count_gives_the_same_table(monkeypatch, form, chunks):
+    # batches around 1,368 and 3,648 chunks of 128 items: one feature a node,
+    # five nodes an anchor, so a batch of b anchors emits 5 b items
+    rng = np.random.default_rng(chunks)
+    batch = chunks * 128 // 5
+    n = 3 * batch
+    rows = np.arange(n + 1, dtype=np.uint64)
+    cols = rng.integers(0, n, n).astype(np.uint32)
+    fids = rng.integers(0, 50_000, n).astype(np.uint32)
+    out = []
+    for split in (None, "1"):
+        if split:
+            monkeypatch.setenv("EP_RED_SPLIT", split)
+        cfg = _native.default_config()
+        cfg.form, cfg.dims, cfg.negatives, cfg.loss, cfg.gamma = form, 36, 3, _native.LOSS_STARSPACE, 0.5
+        cfg.batch_size, cfg.passes, cfg.valid_pct, cfg.autotune = batch, 20, 0.0, 0
+        ctx = _native.Context(cfg)
+        ctx.upload_graph(rows, cols, None)
+        ctx.upload_features(rows, fids, 50_000)
+        ctx.set_table(None)
+        st = ctx.train_batches(4)
+        assert st["kept_anchors"] > 0 and abs(st["items"] / 4 / 128 - chunks) < 2
+        out.append((ctx.get_table(50_000, 36), st["unique_rows"], st["gathered_rows"]))
+    assert np.array_equal(out[0][0], out[1][0]) and out[0][1:] == out[1][1:]
