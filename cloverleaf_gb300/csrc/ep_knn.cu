@@ -1101,6 +1101,10 @@ extern "C" int ep_knn_cosine(int device, uint64_t n_db, uint32_t dims, const flo
     // 32 MB, each searched while the next one is uploaded and normalised.
     // 8,192 x 262,144 x 256, top 10 (64 CTAs, 1.89 ms of search, after a 1.5 ms
     // upload): the call 4.25 -> 2.7 ms; 739 x 48,046 x 48, top 20: 1.31 -> 0.54.
+    // Two splits fit the SMs up to 76 tiles; the call in ms, one / two: 76 tiles
+    // x 262,144 x 256 4.11 / 2.71, 77 tiles (two waves) 4.12 / 4.43; x 100,000 x
+    // 64 1.13 / 0.95 and 1.12 / 1.35.  (Chunks without a split: 3.77 and 1.13
+    // at 77 tiles.)
     const uint64_t db_bytes = n_db * dims * 4;
     uint32_t chunks = 1, splits = 1;                   // splits per chunk
     if (q_tiles <= 76 && db_tiles >= 8) {
@@ -1118,9 +1122,11 @@ extern "C" int ep_knn_cosine(int device, uint64_t n_db, uint32_t dims, const flo
         cudaEvent_t e = nullptr;
         ~EV() { if (e) cudaEventDestroy(e); }
     };
-    std::vector<EV> ready(chunks), t_from(chunks), t_to(chunks);
-    for (uint32_t c = 0; c < chunks; ++c) {
-        KCK(cudaEventCreateWithFlags(&ready[c].e, cudaEventDisableTiming), "events");
+    // one timed stretch for each chunk's search, one for the join of the splits
+    const uint32_t timed = chunks + (split ? 1 : 0);
+    std::vector<EV> ready(chunks), t_from(timed), t_to(timed);
+    for (uint32_t c = 0; c < timed; ++c) {
+        if (c < chunks) KCK(cudaEventCreateWithFlags(&ready[c].e, cudaEventDisableTiming), "events");
         KCK(cudaEventCreate(&t_from[c].e), "events");
         KCK(cudaEventCreate(&t_to[c].e), "events");
     }
@@ -1157,8 +1163,10 @@ extern "C" int ep_knn_cosine(int device, uint64_t n_db, uint32_t dims, const flo
     }
     if (split) {
         const uint32_t lists = chunks * splits * slices;
+        cudaEventRecord(t_from[chunks].e, s);
         k_merge_topk<<<(unsigned)((n_q + 3) / 4), 128, 4 * (size_t)lists, s>>>(a.part, n_q, chunks * splits, slices, k, a.idx,
                                                                              a.sim);
+        cudaEventRecord(t_to[chunks].e, s);
         KCK(cudaGetLastError(), "knn merge");
     }
     uint32_t herr = 0;
@@ -1168,7 +1176,7 @@ extern "C" int ep_knn_cosine(int device, uint64_t n_db, uint32_t dims, const flo
     KCK(cudaMemcpyAsync(&herr, ar.at<void>(o_err), 4, cudaMemcpyDeviceToHost, s), "download");
     KCK(cudaStreamSynchronize(s), "knn");
     g_knn_ms = 0.f;
-    for (uint32_t c = 0; c < chunks; ++c) {
+    for (uint32_t c = 0; c < timed; ++c) {
         float ms = 0.f;
         if (cudaEventElapsedTime(&ms, t_from[c].e, t_to[c].e) == cudaSuccess) g_knn_ms += ms;
     }

@@ -357,8 +357,8 @@ int ep_align(int device, uint64_t n_nodes, const uint64_t* row_ptr, const uint32
 const char* ep_knn_last_error(void);
 
 /* Measurement hook (no counterpart in the reference): CUDA-event time in ms
- * of the GPU kernels of this host thread's last ep_knn_cosine (the top-k
- * kernels) or ep_align call. */
+ * of the GPU kernels of this host thread's last ep_knn_cosine (the search and
+ * the join of its splits) or ep_align call. */
 float ep_knn_last_kernel_ms(void);
 
 /* ---- host-side graph construction (src/graph.rs) --------------------- */

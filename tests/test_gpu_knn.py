@@ -234,3 +234,20 @@ def test_split_database_with_few_rows_to_find():
     for i, row in enumerate(ids):
         assert set(row[:2].tolist()) == {5, 700, 2040} - {(700, 5)[i]}
         assert (row[2:] == 0xffffffff).all() and np.isneginf(sim[i, 2:]).all()
+
+
+def test_reported_time_covers_the_join_of_the_splits():
+    # one query over 152 splits of 7 tiles at most takes a CTA as long as an
+    # unsplit database of 7 tiles, and then joins some hundred lists of 32
+    # entries (75 us beside 120 us of search)
+    rng = np.random.default_rng(12)
+    db = rng.standard_normal((262_144, 8)).astype(np.float32)
+    q = rng.standard_normal((1, 8)).astype(np.float32)
+    ms = {}
+    for rows in (7 * 256, 262_144):
+        t = []
+        for _ in range(10):
+            _native.knn_cosine(db[:rows], q, 32)
+            t.append(_native.lib().ep_knn_last_kernel_ms())
+        ms[rows] = sorted(t)[2]
+    assert ms[262_144] > 1.25 * ms[7 * 256], ms
