@@ -1176,7 +1176,11 @@ static bool tune_from_cache(ep_ctx* c) {
 }
 
 // Candidates of the two tuning stages; `need` receives the batches they take.
-static void tune_candidates(const ep_ctx* c, std::vector<TuneChoice>& s1, uint32_t& need) {
+// Shapes that the rules for small batches make one launch are tried once: a
+// reducer with several warps per chunk has no five-CTA form, a gather with
+// several per anchor no CTA size.
+static void tune_candidates(const ep_ctx* c, bool use_graph, std::vector<TuneChoice>& s1,
+                            std::vector<std::pair<uint32_t, uint32_t>>& gathers, uint32_t& need) {
     const TuneChoice cur = {c->chunk, c->fused_mode, c->gather_ctas, c->ring_pw, c->ring_cw, c->ring_slots, c->queue_ctas,
                            c->gather_warps};
     const bool fused = c->cfg.form == EP_FORM_FUSED_BF16;
@@ -1191,7 +1195,7 @@ static void tune_candidates(const ep_ctx* c, std::vector<TuneChoice>& s1, uint32
         t.mode = 2;
         t.qctas = 4;
         s1.push_back(t);
-        if (c->vpl <= 8) { t.qctas = 5; s1.push_back(t); t.qctas = 4; }
+        if (c->vpl <= 8 && !reduce_splits(c->train_items, ch)) { t.qctas = 5; s1.push_back(t); t.qctas = 4; }
         if (level >= 2) { t.mode = 1; s1.push_back(t); }
         const uint32_t rings[2][3] = {{12, 4, 32}, {10, 6, 36}};
         for (const auto& r : rings)
@@ -1200,8 +1204,11 @@ static void tune_candidates(const ep_ctx* c, std::vector<TuneChoice>& s1, uint32
                 s1.push_back(t);
             }
     }
-    // stage 2 times five gather grids
-    need = (uint32_t)((s1.size() > 1 ? s1.size() : 0) + 5) * (kTuneWarm + kTuneTimed);
+    // stage 2: the staged gather's grid, with the stage-1 choice: one warp per
+    // anchor in CTAs of 2, 4 or 8 warps, or persistent at 2 or 3 CTAs per SM
+    gathers = {{0, 2}, {0, 4}, {0, 8}, {2 * 152, 8}, {3 * 152, 8}};
+    if (gather_split_of(c->tt, (int)c->vpl, c->Bcap, use_graph) > 1) gathers.erase(gathers.begin() + 1, gathers.begin() + 3);
+    need = (uint32_t)((s1.size() > 1 ? s1.size() : 0) + gathers.size()) * (kTuneWarm + kTuneTimed);
 }
 
 static int autotune(ep_ctx* c, uint32_t& n, bool use_graph) {
@@ -1209,19 +1216,17 @@ static int autotune(ep_ctx* c, uint32_t& n, bool use_graph) {
     const TuneChoice cur = {c->chunk, c->fused_mode, c->gather_ctas, c->ring_pw, c->ring_cw, c->ring_slots, c->queue_ctas,
                            c->gather_warps};
     std::vector<TuneChoice> s1;
+    std::vector<std::pair<uint32_t, uint32_t>> gathers;
     uint32_t need = 0;
-    tune_candidates(c, s1, need);
+    tune_candidates(c, use_graph, s1, gathers, need);
     if (n < need) return EP_OK;
-    // stage 2: the staged gather's grid, with the stage-1 choice: one warp per
-    // anchor in CTAs of 2, 4 or 8 warps, or persistent at 2 or 3 CTAs per SM
-    const uint32_t gathers[5][2] = {{0, 2}, {0, 4}, {0, 8}, {2 * 152, 8}, {3 * 152, 8}};
     TuneChoice pick = cur;
     int rc = tune_stage(c, s1, &pick, use_graph);
     std::vector<TuneChoice> s2;
     for (const auto& g : gathers) {
         TuneChoice t = pick;
-        t.gather_ctas = g[0];
-        t.gwarps = g[1];
+        t.gather_ctas = g.first;
+        t.gwarps = g.second;
         s2.push_back(t);
     }
     if (!rc) rc = tune_stage(c, s2, &pick, use_graph);
@@ -1262,8 +1267,9 @@ static int prepare_graphs(ep_ctx* c, uint32_t n) {
     if (!replays(c, n) || n == 0) return EP_OK;
     if (c->cfg.autotune && !tune_from_cache(c)) {
         std::vector<TuneChoice> s1;
+        std::vector<std::pair<uint32_t, uint32_t>> gathers;
         uint32_t need = 0;
-        tune_candidates(c, s1, need);
+        tune_candidates(c, true, s1, gathers, need);
         if (n >= need) return EP_OK;   // this run starts with the tuner, which rebuilds them per candidate
     }
     plan_graphs(c, n);

@@ -1998,11 +1998,9 @@ void launch_scan_occ(BatchState* st, uint32_t* occ, uint32_t cap, uint64_t items
 //   / 111.3, 2,048 117.1 / 117.3 / 120.7, 2,560 129 / 135 / 139, 4,096 167 / 173
 //   / 180; (256 FP32) 1,400 139 / - / 134, 2,600 172 / 165 / -, 3,600 209 / 204 /
 //   -, 4,096 223 / 221 / -.
-template <typename T, int VPL>
-static uint32_t gather_split(const ForwardParams& p, uint32_t cap) {
-    if (p.gather_split) return p.gather_split;
-    if (!p.beside_sort) return cap <= 1280 ? 4 : (cap <= 3072 ? 2 : 1);
-    const uint32_t two = sizeof(T) == 2 ? 1280 : (VPL <= 4 ? 2048 : 4096);
+uint32_t gather_split_of(int tt, int vpl, uint32_t cap, bool beside_sort) {
+    if (!beside_sort) return cap <= 1280 ? 4 : (cap <= 3072 ? 2 : 1);
+    const uint32_t two = tt == TT_BF16 ? 1280 : (vpl <= 4 ? 2048 : 4096);
     return cap <= 1024 ? 4 : (cap <= two ? 2 : 1);
 }
 
@@ -2030,7 +2028,7 @@ static void fwd_launch(const ForwardParams& p, uint32_t cap, cudaStream_t s, int
     const uint32_t gw = p.gather_warps >= 1 && p.gather_warps <= (uint32_t)FWD_WARPS ? p.gather_warps : FWD_WARPS;
     const uint32_t gblocks = (cap + gw - 1) / gw;
     const size_t gsmem = sizeof(GatherTables) * gw, one = sizeof(GatherTables);
-    const uint32_t split = gather_split<T, VPL>(p, cap);
+    const uint32_t split = p.gather_split ? p.gather_split : gather_split_of(sizeof(T) == 2 ? TT_BF16 : TT_F32, VPL, cap, p.beside_sort);
     if (p.gather_ctas > 2 * 152)
         launch_chain(k_fwd_gather_queue<T, A, VPL, 3>, std::min(p.gather_ctas, blocks), 32 * FWD_WARPS, smem, s, p);
     else if (p.gather_ctas)

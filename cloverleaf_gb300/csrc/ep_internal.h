@@ -242,6 +242,8 @@ void launch_scan_occ(BatchState* st, uint32_t* occ, uint32_t cap, uint64_t items
 // its tables (independent of it), or the loss (after both)
 enum ForwardPart : int { FWD_GATHER = 0, FWD_DIRECT = 1, FWD_LOSS = 2 };
 void launch_forward(int tt, int vpl, const ForwardParams& p, uint32_t cap, cudaStream_t s, int part);
+// warps per anchor of the staged gather (ForwardParams::gather_split 0)
+uint32_t gather_split_of(int tt, int vpl, uint32_t cap, bool beside_sort);
 // the item emission alone (k_fwd_emit)
 void launch_emit(const ForwardParams& p, uint32_t cap, cudaStream_t s);
 // counted: the first pass's digit counts are in hist already (ForwardParams::
@@ -251,6 +253,8 @@ void launch_radix_sort(BatchState* st, uint32_t* keys, uint32_t* keys_alt, const
                        const float* item_c, uint2* vals, uint2* vals_alt, uint32_t* hist, uint64_t cap,
                        int key_bits, bool counted, uint32_t** sorted_keys, uint2** sorted_vals, cudaStream_t s);
 void radix_clear(uint32_t* hist, uint64_t cap, int key_bits, cudaStream_t s);
+// whether batches of typ_items take several warps per chunk (ReduceParams::red_split 0, red_ctas 0)
+bool reduce_splits(uint64_t typ_items, uint32_t chunk);
 void launch_reduce(int tt, int vpl, const ReduceParams& p, uint64_t items_cap, cudaStream_t s);
 // part: 0 both fix-up kernels in order, 1 the short spans (k_fixup), 2 the
 // long spans (k_fixup_long); the two parts are independent

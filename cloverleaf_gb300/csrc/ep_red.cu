@@ -1472,13 +1472,17 @@ static size_t stream_smem(uint32_t dpad) {
     return queue_smem<T, A>(dpad) + (size_t)(QUEUE_THREADS / 32) * (STREAM_BYTES + QN * sizeof(unsigned long long));
 }
 
+bool reduce_splits(uint64_t typ_items, uint32_t chunk) {
+    return chunk <= RW && reduce_chunks(typ_items, chunk) <= RED_SPLIT_CHUNKS;
+}
+
 template <typename T, typename A, int VPL>
 static void red_launch(const ReduceParams& p, uint64_t cap, cudaStream_t s, int which) {
     const uint32_t nch = reduce_chunks(cap, p.chunk);
     const uint32_t warps = nch ? nch : 1;
     if (which == 0) {
         // few chunks expected: several warps each, with room for four
-        const bool split = p.red_split > 1 || (!p.red_split && reduce_chunks(p.typ_items, p.chunk) <= RED_SPLIT_CHUNKS);
+        const bool split = p.red_split > 1 || (!p.red_split && reduce_splits(p.typ_items, p.chunk));
         if (split && !p.red_ctas && p.chunk <= RW && (p.out_mode == OUT_DENSE || p.out_mode == OUT_QUEUE)) {
             const uint32_t w4 = (uint32_t)std::min<uint64_t>(4ull * warps, 8ull * RED_MAX_CTAS);
             if (p.out_mode == OUT_DENSE)

@@ -570,3 +570,32 @@ def test_reducer_split_by_chunk_count_gives_the_same_table(monkeypatch, form, ch
         assert st["kept_anchors"] > 0 and abs(st["items"] / 4 / 128 - chunks) < 2
         out.append((ctx.get_table(50_000, 36), st["unique_rows"], st["gathered_rows"]))
     assert np.array_equal(out[0][0], out[1][0]) and out[0][1:] == out[1][1:]
+
+
+@pytest.mark.parametrize("form,batches", [(_native.FORM_FUSED_BF16, 60), (_native.FORM_PLAIN_FP32, 30)])
+def test_autotune_tries_no_shape_twice(form, batches):
+    # 1,000 anchors: several warps per chunk (no five-CTA reducer) and per
+    # anchor (no CTA sizes).  Fused: the queue and two rings, three gather
+    # grids; plain: three gather grids; ten batches each
+    w = datagen.workload("cl10m", scale=0.003)
+
+    def context(level):
+        cfg = _native.default_config()
+        cfg.dims, cfg.negatives, cfg.loss, cfg.gamma = 256, 10, _native.LOSS_STARSPACE, 0.5
+        cfg.batch_size, cfg.alpha, cfg.passes, cfg.valid_pct = 1000, 0.01, 1, 0.0
+        cfg.max_nodes_kind, cfg.max_nodes = _native.SAMPLE_FIXED, 25.0
+        cfg.form, cfg.autotune = form, level
+        ctx = _native.Context(cfg)
+        ctx.upload_graph(w["rows"], w["cols"], None)
+        ctx.upload_features(w["fptr"], w["fids"], w["n_feat"])
+        ctx.set_table(None)
+        return ctx
+
+    ctx = context(1)
+    ctx.train_batches(batches - 1)
+    assert not ctx.launch_shape()["tuned"]
+    ctx.train_batches(batches)
+    assert ctx.launch_shape()["tuned"]
+    ref = context(0)
+    ref.train_batches(2 * batches - 1)
+    assert np.array_equal(ctx.get_table(w["n_feat"], 256), ref.get_table(w["n_feat"], 256))
