@@ -599,3 +599,97 @@ def test_autotune_tries_no_shape_twice(form, batches):
     ref = context(0)
     ref.train_batches(2 * batches - 1)
     assert np.array_equal(ctx.get_table(w["n_feat"], 256), ref.get_table(w["n_feat"], 256))
+
+
+def _table_under(monkeypatch, env, make, batches):
+    for k, v in env.items():
+        monkeypatch.setenv(k, v)
+    ctx, n_feat, dims = make()
+    st = ctx.train_batches(batches)
+    assert st["kept_anchors"] > 0
+    for k in env:
+        monkeypatch.delenv(k)
+    return ctx.get_table(n_feat, dims)
+
+
+@pytest.mark.parametrize("warps", ["1", "2", "4"])
+@pytest.mark.parametrize("graphs", [1, 0])
+def test_gather_cta_sizes_with_a_warp_per_anchor(monkeypatch, warps, graphs):
+    # (batches of this size take several warps per anchor when left to the
+    # rule, and the gather then has no CTA size)
+    w = datagen.workload("cl10m", scale=0.005)
+    make = lambda: (_cl_ctx_cfg(w, use_graphs=graphs), w["n_feat"], w["ep"]["dims"])  # noqa: E731
+    tables = [_table_under(monkeypatch, {"EP_GATHER_SPLIT": "1", "EP_GATHER_WARPS": g}, make, 19) for g in ("8", warps)]
+    assert np.array_equal(tables[0], tables[1])
+
+
+def test_five_cta_reducer_with_a_warp_per_chunk(monkeypatch):
+    # (batches of this size take several warps per chunk when left to the
+    # rule, in a kernel of their own)
+    w = datagen.workload("cl10m", scale=0.005)
+    make = lambda: (_cl_ctx(w), w["n_feat"], w["ep"]["dims"])  # noqa: E731
+    tables = [_table_under(monkeypatch, {"EP_RED_SPLIT": s, "EP_QUEUE_CTAS": q}, make, 29)
+              for s, q in (("1", "4"), ("1", "5"), ("2", "4"))]
+    assert np.array_equal(tables[0], tables[1]) and np.array_equal(tables[0], tables[2])
+
+
+@pytest.mark.parametrize("chunk", ["128", "160", "512"])
+@pytest.mark.parametrize("dims", [129, 130, 136, 200, 250, 255, 256])
+def test_streamed_reducer_gives_the_queue_reducers_table(monkeypatch, dims, chunk):
+    # BF16 rows of 129 to 256 dims: direction rows through the shared-memory
+    # ring (a warp per chunk, four CTAs) against registers (five CTAs, or four
+    # warps per chunk where a chunk is one window); lanes past the row, hot
+    # features and chunks of a feature per item, a ragged last window
+    from tests._cases import random_problem
+    for n_feat in (5, 6000):
+        prob = random_problem(dims, n=1500, n_feat=n_feat, dims=dims, deg=(1, 9), feats=(1, 5))
+
+        def make():
+            cfg = _native.default_config()
+            cfg.form, cfg.dims, cfg.negatives = _native.FORM_FUSED_BF16, dims, 4
+            cfg.loss, cfg.gamma, cfg.batch_size, cfg.passes, cfg.valid_pct = _native.LOSS_STARSPACE, 0.5, 400, 1, 0.0
+            ctx = _native.Context(cfg)
+            ctx.upload_graph(prob["rows"], prob["cols"], None)
+            ctx.upload_features(prob["fptr"], prob["fids"], n_feat)
+            ctx.set_table(None)
+            return ctx, n_feat, dims
+
+        shapes = [("1", "4"), ("1", "5")] + ([("4", "4")] if chunk == "128" else [])
+        tables = [_table_under(monkeypatch, {"EP_REDUCE_CHUNK": chunk, "EP_RED_SPLIT": s, "EP_QUEUE_CTAS": q}, make, 7)
+                  for s, q in shapes]
+        assert all(np.array_equal(tables[0], t) for t in tables[1:])
+
+
+@pytest.mark.parametrize("form", [_native.FORM_FUSED_BF16, _native.FORM_PLAIN_FP32])
+def test_training_again_on_a_context_equals_a_new_one(form):
+    # a new table leaves the captured graphs in place: the second and third
+    # runs replay them, after a given table as after a drawn one, after another
+    # run length and after explicit batches that grow the scratch
+    from tests._cases import random_problem, sample_batch
+    prob = random_problem(92, n=3000, n_feat=2000, dims=40, deg=(1, 9), feats=(1, 5))
+    small = sample_batch(1, prob, B=50, K=6, R=4)
+    large = sample_batch(2, prob, B=900, K=9, R=4)
+
+    def context():
+        cfg = _native.default_config()
+        cfg.form, cfg.dims, cfg.negatives, cfg.loss, cfg.gamma = form, 40, 4, _native.LOSS_STARSPACE, 0.5
+        cfg.batch_size, cfg.passes, cfg.valid_pct, cfg.autotune = 100, 2, 0.1, 0
+        ctx = _native.Context(cfg)
+        ctx.upload_graph(prob["rows"], prob["cols"], None)
+        ctx.upload_features(prob["fptr"], prob["fids"], 2000)
+        return ctx
+
+    def run(ctx, table, batches):
+        ctx.set_table(table)
+        stats = ctx.train_batches(batches) if batches else ctx.train(2)[-1]
+        same = ("train_loss", "valid_loss", "lr_last", "kept_anchors", "items", "gathered_rows", "unique_rows")
+        return ctx.get_table(2000, 40), [stats[k] for k in same]
+
+    used = context()
+    for table, batches, between in ((None, 0, None), (prob["table"], 0, small), (None, 45, large), (prob["table"], 7, None),
+                                    (None, 0, small), (None, 45, None)):
+        got, want = run(used, table, batches), run(context(), table, batches)
+        assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1], equal_nan=True)
+        if between:
+            used.batch_grad(_native.Context.samples(between["anchors"], between["nbr_ptr"], between["nbr"], between["nbr_w"],
+                                                    between["neg"]), 2000, 40)
