@@ -20,13 +20,16 @@ namespace ep {
 // a resident one, 205 MB 7.5 and 1.15 ms.  (An atomic addition of zero keeps
 // the contents too, but maps the shared zero page first, whose replacement
 // makes the device drop its translations: 24 us a page of 64 KB.)  205 MB take
-// 2.2 ms on four threads; on eight they stand in each other's way, 7.3 ms.
+// 2.2 ms on four threads; more stand in each other's way, 7.3 ms on eight.
 // Where the kernel does not know the advice the pages are left to the copy.
-// Arrays below THREADED, where starting threads costs more than they save
-// (0.4 ms), are made resident by wait(), on the OpenMP threads.
+// The copy follows slab by slab; smaller slabs let it start sooner (embeddings
+// of 46 MB 1.59 ms with slabs of 32 MB, 1.51 with 8).  Arrays below THREADED,
+// where starting threads costs more than they save, are made resident by
+// wait(), on the OpenMP threads: 24 MB 0.98 ms, 1.10 with threads; 31 MB 1.17
+// and 1.31; 36 MB 1.49 and 1.31.
 class ResultPages {
 public:
-    static constexpr size_t SLAB = 32u << 20, THREADED = 48u << 20;
+    static constexpr size_t SLAB = 8u << 20, THREADED = 32u << 20;
 
     ResultPages(void* p, size_t bytes);
     ~ResultPages();

@@ -76,7 +76,7 @@ def test_embeddings_over_their_table(pinned):
 
 @pytest.mark.parametrize("dims,offset", [(128, 0), (126, 4), (128, 12)])
 def test_results_of_several_slabs(oracle, dims, offset):
-    # 32 MB to a slab: two whole ones and a ragged third, at odd addresses
+    # several slabs and a ragged last one, at odd addresses
     n = 72 * MB // (4 * dims) + 1
     rows, cols, cdf = _graph(n, 3, dims)
     emb = np.random.default_rng(dims).standard_normal((n, dims)).astype(np.float32)

@@ -8,7 +8,7 @@ import numpy as np
 import pytest
 
 MB = 1 << 20
-SLAB = 32 * MB
+SLAB = 8 * MB
 
 
 def _pages(native, addr, n):
@@ -25,7 +25,7 @@ def _pages(native, addr, n):
     dtor(at)
 
 
-@pytest.mark.parametrize("n", [0, 1, 4095, 70_001, 9 * MB + 3, 48 * MB - 1, 48 * MB, 70 * MB + 5])
+@pytest.mark.parametrize("n", [0, 1, 4095, 70_001, 9 * MB + 3, 32 * MB - 1, 32 * MB, 70 * MB + 5])
 @pytest.mark.parametrize("offset", [0, 13])
 def test_contents_are_kept(native, n, offset):
     a = np.random.default_rng(n).integers(1, 256, n + offset + 64, dtype=np.uint8)
