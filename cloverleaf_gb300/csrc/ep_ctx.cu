@@ -1178,13 +1178,15 @@ static bool tune_from_cache(ep_ctx* c) {
 // Candidates of the two tuning stages; `need` receives the batches they take.
 // Shapes that the rules for small batches make one launch are tried once: a
 // reducer with several warps per chunk has no five-CTA form, a gather with
-// several per anchor no CTA size.
+// several per anchor no CTA size.  `least`, the shortest run that is tuned,
+// counts them all the same: a run spends no larger part of itself on tuning.
 static void tune_candidates(const ep_ctx* c, bool use_graph, std::vector<TuneChoice>& s1,
-                            std::vector<std::pair<uint32_t, uint32_t>>& gathers, uint32_t& need) {
+                            std::vector<std::pair<uint32_t, uint32_t>>& gathers, uint32_t& need, uint32_t& least) {
     const TuneChoice cur = {c->chunk, c->fused_mode, c->gather_ctas, c->ring_pw, c->ring_cw, c->ring_slots, c->queue_ctas,
                            c->gather_warps};
     const bool fused = c->cfg.form == EP_FORM_FUSED_BF16;
     const int level = c->cfg.autotune;
+    size_t all = 0;      // stage 1 with the shapes left out
     // stage 1: reducer chunk (level 2) x Adam placement (FUSED form)
     const std::vector<uint32_t> chunks = level >= 2 ? std::vector<uint32_t>(kTuneChunks, kTuneChunks + 3)
                                                     : std::vector<uint32_t>{c->chunk};
@@ -1195,7 +1197,10 @@ static void tune_candidates(const ep_ctx* c, bool use_graph, std::vector<TuneCho
         t.mode = 2;
         t.qctas = 4;
         s1.push_back(t);
-        if (c->vpl <= 8 && !reduce_splits(c->train_items, ch)) { t.qctas = 5; s1.push_back(t); t.qctas = 4; }
+        if (c->vpl <= 8) {
+            if (reduce_splits(c->train_items, ch)) ++all;
+            else { t.qctas = 5; s1.push_back(t); t.qctas = 4; }
+        }
         if (level >= 2) { t.mode = 1; s1.push_back(t); }
         const uint32_t rings[2][3] = {{12, 4, 32}, {10, 6, 36}};
         for (const auto& r : rings)
@@ -1207,8 +1212,13 @@ static void tune_candidates(const ep_ctx* c, bool use_graph, std::vector<TuneCho
     // stage 2: the staged gather's grid, with the stage-1 choice: one warp per
     // anchor in CTAs of 2, 4 or 8 warps, or persistent at 2 or 3 CTAs per SM
     gathers = {{0, 2}, {0, 4}, {0, 8}, {2 * 152, 8}, {3 * 152, 8}};
+    const auto batches = [&](size_t stage1) {
+        return (uint32_t)((stage1 > 1 ? stage1 : 0) + gathers.size()) * (kTuneWarm + kTuneTimed);
+    };
+    all += s1.size();
+    least = batches(all);
     if (gather_split_of(c->tt, (int)c->vpl, c->Bcap, use_graph) > 1) gathers.erase(gathers.begin() + 1, gathers.begin() + 3);
-    need = (uint32_t)((s1.size() > 1 ? s1.size() : 0) + gathers.size()) * (kTuneWarm + kTuneTimed);
+    need = batches(s1.size());
 }
 
 static int autotune(ep_ctx* c, uint32_t& n, bool use_graph) {
@@ -1217,9 +1227,9 @@ static int autotune(ep_ctx* c, uint32_t& n, bool use_graph) {
                            c->gather_warps};
     std::vector<TuneChoice> s1;
     std::vector<std::pair<uint32_t, uint32_t>> gathers;
-    uint32_t need = 0;
-    tune_candidates(c, use_graph, s1, gathers, need);
-    if (n < need) return EP_OK;
+    uint32_t need = 0, least = 0;
+    tune_candidates(c, use_graph, s1, gathers, need, least);
+    if (n < least) return EP_OK;
     TuneChoice pick = cur;
     int rc = tune_stage(c, s1, &pick, use_graph);
     std::vector<TuneChoice> s2;
@@ -1268,9 +1278,9 @@ static int prepare_graphs(ep_ctx* c, uint32_t n) {
     if (c->cfg.autotune && !tune_from_cache(c)) {
         std::vector<TuneChoice> s1;
         std::vector<std::pair<uint32_t, uint32_t>> gathers;
-        uint32_t need = 0;
-        tune_candidates(c, true, s1, gathers, need);
-        if (n >= need) return EP_OK;   // this run starts with the tuner, which rebuilds them per candidate
+        uint32_t need = 0, least = 0;
+        tune_candidates(c, true, s1, gathers, need, least);
+        if (n >= least) return EP_OK;   // this run starts with the tuner, which rebuilds them per candidate
     }
     plan_graphs(c, n);
     const uint32_t k = c->graph_batches;

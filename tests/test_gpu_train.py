@@ -572,16 +572,17 @@ def test_reducer_split_by_chunk_count_gives_the_same_table(monkeypatch, form, ch
     assert np.array_equal(out[0][0], out[1][0]) and out[0][1:] == out[1][1:]
 
 
-@pytest.mark.parametrize("form,batches", [(_native.FORM_FUSED_BF16, 60), (_native.FORM_PLAIN_FP32, 30)])
-def test_autotune_tries_no_shape_twice(form, batches):
+@pytest.mark.parametrize("form,dims,batches", [(_native.FORM_FUSED_BF16, 256, 90), (_native.FORM_FUSED_BF16, 100, 70),
+                                                (_native.FORM_PLAIN_FP32, 256, 50)])
+def test_autotune_tries_no_shape_twice(form, dims, batches):
     # 1,000 anchors: several warps per chunk (no five-CTA reducer) and per
-    # anchor (no CTA sizes).  Fused: the queue and two rings, three gather
-    # grids; plain: three gather grids; ten batches each
+    # anchor (no CTA sizes of the one-warp gather); the shortest run that is
+    # tuned stays that of all candidates, ten batches each
     w = datagen.workload("cl10m", scale=0.003)
 
     def context(level):
         cfg = _native.default_config()
-        cfg.dims, cfg.negatives, cfg.loss, cfg.gamma = 256, 10, _native.LOSS_STARSPACE, 0.5
+        cfg.dims, cfg.negatives, cfg.loss, cfg.gamma = dims, 10, _native.LOSS_STARSPACE, 0.5
         cfg.batch_size, cfg.alpha, cfg.passes, cfg.valid_pct = 1000, 0.01, 1, 0.0
         cfg.max_nodes_kind, cfg.max_nodes = _native.SAMPLE_FIXED, 25.0
         cfg.form, cfg.autotune = form, level
@@ -595,10 +596,12 @@ def test_autotune_tries_no_shape_twice(form, batches):
     ctx.train_batches(batches - 1)
     assert not ctx.launch_shape()["tuned"]
     ctx.train_batches(batches)
-    assert ctx.launch_shape()["tuned"]
+    shape = ctx.launch_shape()
+    assert shape["tuned"] and shape["queue_ctas_per_sm"] == 4
+    assert (shape["gather_ctas"], shape["gather_warps"]) in ((0, 2), (304, 8), (456, 8))
     ref = context(0)
     ref.train_batches(2 * batches - 1)
-    assert np.array_equal(ctx.get_table(w["n_feat"], 256), ref.get_table(w["n_feat"], 256))
+    assert np.array_equal(ctx.get_table(w["n_feat"], dims), ref.get_table(w["n_feat"], dims))
 
 
 def _table_under(monkeypatch, env, make, batches):
