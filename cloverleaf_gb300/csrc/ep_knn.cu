@@ -1122,11 +1122,10 @@ extern "C" int ep_knn_cosine(int device, uint64_t n_db, uint32_t dims, const flo
         cudaEvent_t e = nullptr;
         ~EV() { if (e) cudaEventDestroy(e); }
     };
-    // one timed stretch for each chunk's search, one for the join of the splits
-    const uint32_t timed = chunks + (split ? 1 : 0);
-    std::vector<EV> ready(chunks), t_from(timed), t_to(timed);
-    for (uint32_t c = 0; c < timed; ++c) {
-        if (c < chunks) KCK(cudaEventCreateWithFlags(&ready[c].e, cudaEventDisableTiming), "events");
+    // one timed stretch for each chunk's search, the last one with the join of the splits
+    std::vector<EV> ready(chunks), t_from(chunks), t_to(chunks);
+    for (uint32_t c = 0; c < chunks; ++c) {
+        KCK(cudaEventCreateWithFlags(&ready[c].e, cudaEventDisableTiming), "events");
         KCK(cudaEventCreate(&t_from[c].e), "events");
         KCK(cudaEventCreate(&t_to[c].e), "events");
     }
@@ -1159,16 +1158,15 @@ extern "C" int ep_knn_cosine(int device, uint64_t n_db, uint32_t dims, const flo
         cudaStreamWaitEvent(s, ready[c].e, 0);
         cudaEventRecord(t_from[c].e, s);
         KCK(knn_launch_k(a, (uint32_t)tile0, (uint32_t)tile1, splits, c * splits, s), "knn launch");
-        cudaEventRecord(t_to[c].e, s);
+        if (c + 1 < chunks) cudaEventRecord(t_to[c].e, s);
     }
     if (split) {
         const uint32_t lists = chunks * splits * slices;
-        cudaEventRecord(t_from[chunks].e, s);
         k_merge_topk<<<(unsigned)((n_q + 3) / 4), 128, 4 * (size_t)lists, s>>>(a.part, n_q, chunks * splits, slices, k, a.idx,
                                                                              a.sim);
-        cudaEventRecord(t_to[chunks].e, s);
         KCK(cudaGetLastError(), "knn merge");
     }
+    cudaEventRecord(t_to[chunks - 1].e, s);
     uint32_t herr = 0;
     ResultPages pi(idx_out, host_bytes(idx_out, n_q * k * 4)), ps(sim_out, host_bytes(sim_out, n_q * k * 4));
     KCK(download((char*)idx_out, a.idx, n_q * k * 4, pi, s), "download");
@@ -1176,7 +1174,7 @@ extern "C" int ep_knn_cosine(int device, uint64_t n_db, uint32_t dims, const flo
     KCK(cudaMemcpyAsync(&herr, ar.at<void>(o_err), 4, cudaMemcpyDeviceToHost, s), "download");
     KCK(cudaStreamSynchronize(s), "knn");
     g_knn_ms = 0.f;
-    for (uint32_t c = 0; c < timed; ++c) {
+    for (uint32_t c = 0; c < chunks; ++c) {
         float ms = 0.f;
         if (cudaEventElapsedTime(&ms, t_from[c].e, t_to[c].e) == cudaSuccess) g_knn_ms += ms;
     }
