@@ -232,15 +232,6 @@ class ClockSampler:
                 "samples": len(rows)}
 
 
-def fused_mode():
-    """Adam placement of the fused form (the library default is 2: Adam in the
-    reducer through a per-warp queue; 1: a separate Adam kernel)."""
-    try:
-        return int(os.environ.get("EP_FUSED_MODE", "2"))
-    except ValueError:
-        return 2
-
-
 def load_peaks():
     try:
         with open(os.path.join(ROOT, "MEASURED_PEAKS.json")) as f:
@@ -248,6 +239,22 @@ def load_peaks():
         return float(pk["hbm_gbs"]), "measured"
     except Exception:
         return 6800.0, "fallback"
+
+
+STREAMED = "k_reduce (Adam fused, direction rows streamed through shared memory)"
+
+
+def reducer_name(shape, dims):
+    """The fused form's reduction kernel under a launch shape."""
+    if shape["fused_mode"] == 1:
+        return "k_reduce (gradient rows)"
+    if shape["fused_mode"] == 0:
+        return "k_reduce (Adam as each feature closes)"
+    if shape["fused_mode"] == 3:
+        return "k_reduce (Adam by the warps of a ring)"
+    if shape["queue_ctas_per_sm"] == 5:
+        return "k_reduce_q5 (Adam fused, cp.async queue)"
+    return STREAMED if 128 < dims <= 256 else "k_reduce (Adam fused, cp.async queue)"
 
 
 def load_traffic(unique_rows):
@@ -507,6 +514,7 @@ def main():
     log(f"[bench] fused: {st['anchors']} anchors in {st['ms']:.1f} ms device / {wall:.2f} s wall "
         f"-> {value / 1e6:.2f} M nodes/s; loss {st['train_loss']:.4f}")
     stage_ms, pst = ctx.profile_batches(min(args.profile_steps, args.steps))
+    shape = ctx.launch_shape()
     ctx.close()
     B = pst["batches"] or 1
     d, s_el = ep["dims"], 2.0
@@ -519,12 +527,12 @@ def main():
     #            reducer) U*d*(2s+16): m, v read+written (FP32), table row
     #            read+written; (Adam split off) the U*d*4 gradient rows
     #   adam     (split form only) gradient rows + Adam state U*d*(2s+20)
-    split = fused_mode() == 1
+    split = shape["fused_mode"] == 1
     stage_bytes = {"forward": G * d * s_el + 4 * G + 4 * S + 8 * A * (ep["negatives"] + 2),
                    "reduce": 12 * items + (U * d * 4 if split else U * d * (2 * s_el + 16)),
                    "adam": U * d * (2 * s_el + 20) if split else 0.0}
     kernel_of = {"forward": "k_fwd_gather+k_fwd_loss", "adam": "k_adam_dense",
-                 "reduce": "k_reduce (gradient rows)" if split else "k_reduce (Adam fused, cp.async queue)"}
+                 "reduce": reducer_name(shape, d)}
     dom = max(stage_ms, key=stage_ms.get)
     peak, peak_kind = load_peaks()
     rf_stage = max(("forward", "reduce", "adam"), key=lambda k: stage_ms[k])
@@ -534,7 +542,7 @@ def main():
     roofline = {"bound": "hbm", "kernel": kernel_of[rf_stage],
                 "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                 "peak_source": f"{peak_kind} (MEASURED_PEAKS.json hbm_gbs, burst copy)",
-                "traffic": load_traffic(U) if split is False else None, "alg_bytes_per_launch": stage_bytes[rf_stage],
+                "traffic": load_traffic(U) if kernel_of["reduce"] == STREAMED else None, "alg_bytes_per_launch": stage_bytes[rf_stage],
                 "stage_ms": stage_ms, "dominant_stage": dom,
                 "stage_gbs": {k: stage_bytes[k] / (stage_ms[k] / 1e3) / 1e9 for k in stage_bytes if stage_bytes[k]},
                 "step": {"achieved": step_bytes / (step_ms / 1e3) / 1e9, "alg_bytes_per_step": step_bytes,
