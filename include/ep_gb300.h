@@ -326,7 +326,8 @@ void ep_destroy(ep_ctx* ctx);
  * src/algos/aggregator.rs:17-120: out[v] (n_nodes x dims FP32) = the
  * weighted mean of the table rows of v's features fids[fptr[v]..fptr[v+1])
  * in f32 as the reference sums them; featureless nodes get zeros.  Host
- * buffers; dims <= 512.  Errors: ep_knn_last_error(). */
+ * buffers; dims <= 512; out may overlap the inputs (they are on the device
+ * before it is written).  Errors: ep_knn_last_error(). */
 int ep_embed_features(int device, uint64_t n_nodes, const uint64_t* fptr, const uint32_t* fids,
                       const float* fweight, uint32_t n_feat, uint32_t dims, const float* table, float* out);
 
@@ -348,7 +349,8 @@ int ep_knn_cosine(int device, uint64_t n_db, uint32_t dims, const float* db, uin
  * the edge probabilities of the CDF weights w_cdf, a = alpha, or
  * min(1, 1 / ln(deg + 1)) when alpha < 0.  f32 arithmetic in the reference's
  * order.  A node without edges gets a * emb[v] (the reference indexes the
- * empty weight list).  emb / out: n_nodes x dims (<= 512).  Host buffers. */
+ * empty weight list).  emb / out: n_nodes x dims (<= 512).  Host buffers; out
+ * may be emb or overlap the inputs. */
 int ep_align(int device, uint64_t n_nodes, const uint64_t* row_ptr, const uint32_t* cols, const float* w_cdf,
              uint32_t dims, const float* emb, float alpha, uint64_t max_neighbors, float* out);
 
