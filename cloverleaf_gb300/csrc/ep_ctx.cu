@@ -877,6 +877,7 @@ static ReduceParams reduce_params(ep_ctx* c, BatchState* st, int out_mode, void*
     rp.red_ctas = c->red_ctas;
     rp.red_split = c->red_split;
     rp.typ_items = c->typ_items;
+    rp.n_feat = c->n_feat;
     return rp;
 }
 
@@ -1198,7 +1199,7 @@ static void tune_candidates(const ep_ctx* c, bool use_graph, std::vector<TuneCho
         t.qctas = 4;
         s1.push_back(t);
         if (c->vpl <= 8) {
-            if (reduce_splits(c->train_items, ch)) ++all;
+            if (reduce_splits(c->train_items, ch, c->n_feat)) ++all;
             else { t.qctas = 5; s1.push_back(t); t.qctas = 4; }
         }
         if (level >= 2) { t.mode = 1; s1.push_back(t); }

@@ -232,6 +232,7 @@ struct ReduceParams {
     // warps per chunk (1, 2, 4; 0 = by the batch's chunk count)
     uint32_t red_split;
     uint64_t typ_items;     // items a batch is expected to emit (launch shape only)
+    uint32_t n_feat;        // features of the table (launch shape only)
 };
 
 // ---- launchers (defined in the kernel translation units) -----------------
@@ -254,7 +255,7 @@ void launch_radix_sort(BatchState* st, uint32_t* keys, uint32_t* keys_alt, const
                        int key_bits, bool counted, uint32_t** sorted_keys, uint2** sorted_vals, cudaStream_t s);
 void radix_clear(uint32_t* hist, uint64_t cap, int key_bits, cudaStream_t s);
 // whether batches of typ_items take several warps per chunk (ReduceParams::red_split 0, red_ctas 0)
-bool reduce_splits(uint64_t typ_items, uint32_t chunk);
+bool reduce_splits(uint64_t typ_items, uint32_t chunk, uint32_t n_feat);
 void launch_reduce(int tt, int vpl, const ReduceParams& p, uint64_t items_cap, cudaStream_t s);
 // part: 0 both fix-up kernels in order, 1 the short spans (k_fixup), 2 the
 // long spans (k_fixup_long); the two parts are independent

@@ -44,8 +44,8 @@ enum : uint32_t { CF_HEAD = 1u, CF_THROUGH = 2u, CF_HEAD_KEPT = 8u, CF_OWNER = 4
 constexpr int RED_THREADS = 256;
 constexpr int FIX_THREADS = 128;
 constexpr uint32_t RED_MAX_CTAS = 152 * 8;
-constexpr uint32_t RED_SPLIT_CHUNKS = 152 * 24;   // batches of up to this many chunks take several warps per chunk
-constexpr uint32_t RED_SPLIT4_CHUNKS = 152 * 9;   // ... four
+// batches of up to this many chunks take several warps per chunk; see chunk_split
+constexpr uint32_t RED_SPLIT_CHUNKS = 152 * 24, RED_SPLIT4_CHUNKS = 152 * 6;
 
 uint32_t reduce_chunks(uint64_t cap, uint32_t chunk) { return (uint32_t)((cap + chunk - 1) / chunk); }
 
@@ -686,18 +686,30 @@ __device__ __forceinline__ bool span_is_long(const ReduceParams& p, uint32_t c, 
 // Warps per chunk.  A chunk's features are independent sums, so its warps
 // take consecutive ranges of features, each feature still summed by one warp
 // in item order.  Small batches leave the chip idle at a warp per chunk, and
-// their time is one chunk's chain.  Whole replayed batch in us at 1 / 2 / 4
-// warps: 566 chunks (256 BF16) 149 / 93.5 / 79.1, (256 FP32) 134 / 115 / 112;
-// 1,298 (128 FP32) 116 / 103 / 97.1, (100 BF16) 122 / 98.5 / 92.0; 1,462 (256
-// BF16) 179 / 129 / 127, (256 FP32) 167 / 141 / 152; 1,767 (128 FP32) 121 / 107
-// / 109; 1,946 (256 BF16) 191 / 144 / 152; 3,322 (256 FP32) 223 / 220 / -, (256
-// BF16) 218 / 191 / -; 4,056 (256 FP32) 251 / 260 / -; 5,189 (128 FP32) 173 /
-// 174 / -.  So four up to 9 chunks an SM, two up to 24.
-__device__ __forceinline__ uint32_t chunk_split(const ReduceParams& p) {
+// their time is one chunk's chain.  A chunk inside one hot feature gains
+// nothing, so the features of the table count as well.  Whole replayed batch
+// in us at 1 / 2 / 4 warps:
+//   many features: 566 chunks (256 BF16) 149 / 93.5 / 79.1, (256 FP32) 134 / 115
+//   / 112; 1,298 (128 FP32) 116 / 103 / 97.1, (100 BF16) 122 / 98.5 / 92.0; 1,462
+//   (256 BF16) 179 / 129 / 127, (256 FP32) 167 / 141 / 152; 1,700 (20 BF16) 130 /
+//   97 / 89; 1,767 (128 FP32) 121 / 107 / 109; 1,946 (256 BF16) 191 / 144 / 152;
+//   3,322 (256 FP32) 223 / 220 / -, (256 BF16) 218 / 191 / -; 4,056 (256 FP32) 251
+//   / 260 / -; 5,189 (128 FP32) 173 / 174 / -;
+//   few, drawn evenly (128 BF16): 225 chunks, 50 features 40.1 / 41.9 / 41.4,
+//   1,000 49.9 / 46.6 / 43.4; 675, 300 56.2 / 55.5 / 57.0, 1,000 56.6 / 56.6 /
+//   55.0, 3,000 60.0 / 55.8 / 52.8; 1,350, 50 52.2 / 53.1 / 63.6, 1,000 63.4 / 63.5
+//   / 74.2, 3,000 65.3 / 64.8 / 71.8, 10,000 69.6 / 66.5 / 71.7.
+// So none below two features to a chunk; four up to 6 chunks an SM, and with
+// sixteen features to a chunk up to 12 (9 where a direction row is 1 KB); two up
+// to 24.
+__device__ __forceinline__ uint32_t chunk_split(const ReduceParams& p, uint32_t row_bytes) {
     const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
     const uint32_t nchunks = (p.st->n_items + p.chunk - 1) / p.chunk;
     uint32_t w = p.red_split;
-    if (!w) w = nchunks <= RED_SPLIT4_CHUNKS ? 4u : (nchunks <= RED_SPLIT_CHUNKS ? 2u : 1u);
+    if (!w) {
+        const uint32_t four = p.n_feat / 16 < nchunks ? RED_SPLIT4_CHUNKS : 152u * (row_bytes > 512u ? 9u : 12u);
+        w = p.n_feat / 2 < nchunks ? 1u : (nchunks <= four ? 4u : (nchunks <= RED_SPLIT_CHUNKS ? 2u : 1u));
+    }
     while (w > 1 && nchunks * w > warps) w >>= 1;
     return w;
 }
@@ -741,7 +753,7 @@ __global__ void __launch_bounds__(MODE == OUT_QUEUE ? QUEUE_THREADS : RED_THREAD
     k_reduce_split(ReduceParams p) {
     pdl_wait();
     pdl_trigger();
-    reduce_body<T, A, VPL, MODE, true>(p, chunk_split(p));
+    reduce_body<T, A, VPL, MODE, true>(p, chunk_split(p, VPL * 32 * (uint32_t)sizeof(typename DirOf<T, A>::type)));
 }
 
 // The per-warp queue reducer at five CTAs per SM instead of four: registers
@@ -1472,8 +1484,9 @@ static size_t stream_smem(uint32_t dpad) {
     return queue_smem<T, A>(dpad) + (size_t)(QUEUE_THREADS / 32) * (STREAM_BYTES + QN * sizeof(unsigned long long));
 }
 
-bool reduce_splits(uint64_t typ_items, uint32_t chunk) {
-    return chunk <= RW && reduce_chunks(typ_items, chunk) <= RED_SPLIT_CHUNKS;
+bool reduce_splits(uint64_t typ_items, uint32_t chunk, uint32_t n_feat) {
+    const uint32_t nch = reduce_chunks(typ_items, chunk);
+    return chunk <= RW && nch <= RED_SPLIT_CHUNKS && n_feat / 2 >= nch;
 }
 
 template <typename T, typename A, int VPL>
@@ -1482,7 +1495,7 @@ static void red_launch(const ReduceParams& p, uint64_t cap, cudaStream_t s, int 
     const uint32_t warps = nch ? nch : 1;
     if (which == 0) {
         // few chunks expected: several warps each, with room for four
-        const bool split = p.red_split > 1 || (!p.red_split && reduce_splits(p.typ_items, p.chunk));
+        const bool split = p.red_split > 1 || (!p.red_split && reduce_splits(p.typ_items, p.chunk, p.n_feat));
         if (split && !p.red_ctas && p.chunk <= RW && (p.out_mode == OUT_DENSE || p.out_mode == OUT_QUEUE)) {
             const uint32_t w4 = (uint32_t)std::min<uint64_t>(4ull * warps, 8ull * RED_MAX_CTAS);
             if (p.out_mode == OUT_DENSE)

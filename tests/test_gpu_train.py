@@ -545,16 +545,18 @@ def test_gather_split_by_batch_size_gives_the_same_table(monkeypatch, form, batc
 
 
 @pytest.mark.parametrize("form", [_native.FORM_FUSED_BF16, _native.FORM_PLAIN_FP32])
-@pytest.mark.parametrize("chunks", [1360, 1376, 3640, 3660])
-def test_reducer_split_by_chunk_count_gives_the_same_table(monkeypatch, form, chunks):
-    # batches around 1,368 and 3,648 chunks of 128 items: one feature a node,
-    # five nodes an anchor, so a batch of b anchors emits 5 b items
+@pytest.mark.parametrize("chunks,n_feat", [(1360, 50_000), (1376, 50_000), (3640, 50_000), (3660, 50_000), (905, 10_000),
+                                           (920, 10_000), (1820, 50_000), (1830, 50_000), (600, 1190), (600, 1210), (600, 7)])
+def test_reducer_split_by_chunk_count_gives_the_same_table(monkeypatch, form, chunks, n_feat):
+    # batches on either side of each line of the rule (chunks of 128 items,
+    # features per chunk): one feature a node, five nodes an anchor, so a batch
+    # of b anchors emits 5 b items
     rng = np.random.default_rng(chunks)
     batch = chunks * 128 // 5
     n = 3 * batch
     rows = np.arange(n + 1, dtype=np.uint64)
     cols = rng.integers(0, n, n).astype(np.uint32)
-    fids = rng.integers(0, 50_000, n).astype(np.uint32)
+    fids = rng.integers(0, n_feat, n).astype(np.uint32)
     out = []
     for split in (None, "1"):
         if split:
@@ -564,11 +566,11 @@ def test_reducer_split_by_chunk_count_gives_the_same_table(monkeypatch, form, ch
         cfg.batch_size, cfg.passes, cfg.valid_pct, cfg.autotune = batch, 20, 0.0, 0
         ctx = _native.Context(cfg)
         ctx.upload_graph(rows, cols, None)
-        ctx.upload_features(rows, fids, 50_000)
+        ctx.upload_features(rows, fids, n_feat)
         ctx.set_table(None)
         st = ctx.train_batches(4)
         assert st["kept_anchors"] > 0 and abs(st["items"] / 4 / 128 - chunks) < 2
-        out.append((ctx.get_table(50_000, 36), st["unique_rows"], st["gathered_rows"]))
+        out.append((ctx.get_table(n_feat, 36), st["unique_rows"], st["gathered_rows"]))
     assert np.array_equal(out[0][0], out[1][0]) and out[0][1:] == out[1][1:]
 
 
